@@ -27,6 +27,15 @@ int cuda_fail(cudaError_t e, const char* what);
     if (e_ != cudaSuccess) return ::rg::cuda_fail(e_, #call); \
   } while (0)
 
+// Lets a kernel take `bytes` of dynamic shared memory, and never less than it
+// may already take: one launch plan may cover several sizes of a kernel.
+inline cudaError_t allow_smem(const void* kernel, size_t bytes) {
+  cudaFuncAttributes fa{};
+  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+  if (e != cudaSuccess || (size_t)fa.maxDynamicSharedSizeBytes >= bytes) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 // Switches to a handle's device for the duration of a call.
 struct DeviceGuard {
   int prev = -1;
@@ -76,6 +85,10 @@ struct WgDesc {
   const double2* bmat;        // [M] B diagonal
   const double2* adiag_edge;  // [M] A diagonal on slices 1 and nx
   const double2* adiag_bulk;  // [M] A diagonal in the bulk
+  // The slice matrix scaled by B^(-1/2) on both sides (rg_sweep_sym.cu):
+  const double2* wsc;         // [M] B^(-1/2)
+  const double2* aw_edge;     // [2 M] A/B on slices 1 and nx: rounded to FP64, then the rest
+  const double2* aw_bulk;     // [2 M] the same in the bulk
   const double2* sqmu_c;      // [M] complex sqrt(mu) (tdistrib Fisher-Lee)
   const double2* sqmu_r;      // [M] sqrt(real(mu)) (v1 Fisher-Lee)
   const double* costab;       // [ny * (2M+1)] cos(pi d y_j) / ny  (Dirichlet)

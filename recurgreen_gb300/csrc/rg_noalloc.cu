@@ -32,6 +32,13 @@ constexpr size_t kNoAllocHeaderBytes = 256;         // seed, queue counters, fla
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
+// Workspace of the sweep of up to 64 modes (one CTA): the potential row and
+// the matrices its lanes keep, for the largest ny that fits the pivoted
+// kernel's shared memory (28,342 points).  Apart from the array above, so
+// that the room for the potential is not reduced by it.
+constexpr size_t kNoAllocWorkBytes = 1280u << 10;
+static __device__ __align__(256) unsigned char g_noalloc_work[kNoAllocWorkBytes];
+
 // Writes the seed and zeroes the queue counters in the header of the array:
 // int32 [0] seed, [1, 1 + kQueueCounters) counters, then the flag slot.
 __global__ void noalloc_header_kernel(int32_t seed) {
@@ -43,9 +50,10 @@ __global__ void noalloc_header_kernel(int32_t seed) {
 constexpr int kMaxDevices = 64;
 std::mutex g_noalloc_mutex;
 void* g_noalloc_ptr[kMaxDevices] = {nullptr};
+void* g_noalloc_work_ptr[kMaxDevices] = {nullptr};
 
-// Device address of g_noalloc_scratch on the current device (looked up once).
-int noalloc_scratch_address(int device, unsigned char** out) {
+// Device addresses of the two arrays on the current device (looked up once).
+int noalloc_scratch_address(int device, unsigned char** out, unsigned char** work) {
   if (device < 0 || device >= kMaxDevices)
     return rg::fail(RG_ERR_INVALID_ARG, "rg_tdistrib_seed_noalloc: device index out of range");
   std::lock_guard<std::mutex> lock(g_noalloc_mutex);
@@ -53,9 +61,14 @@ int noalloc_scratch_address(int device, unsigned char** out) {
     void* p = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (e != cudaSuccess) return rg::cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
+    void* q = nullptr;
+    e = cudaGetSymbolAddress(&q, g_noalloc_work);
+    if (e != cudaSuccess) return rg::cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_work)");
+    g_noalloc_work_ptr[device] = q;
     g_noalloc_ptr[device] = p;
   }
   *out = static_cast<unsigned char*>(g_noalloc_ptr[device]);
+  *work = static_cast<unsigned char*>(g_noalloc_work_ptr[device]);
   return RG_OK;
 }
 
@@ -99,8 +112,10 @@ extern "C" int rg_tdistrib_seed_noalloc(rg_waveguide* wg, int iseed, double* d_t
   if (e != cudaSuccess) return rg::cuda_fail(e, "cudaGetDevice");
   if (cur != v.device)
     return rg::fail(RG_ERR_INVALID_ARG, "rg_tdistrib_seed_noalloc: make the handle's device current first");
-  unsigned char* base = nullptr;
-  if ((rc = noalloc_scratch_address(cur, &base))) return rc;
+  unsigned char *base = nullptr, *work = nullptr;
+  if ((rc = noalloc_scratch_address(cur, &base, &work))) return rc;
+  if (!large && sizeof(double2) * (size_t)stride * grid > kNoAllocWorkBytes)
+    return rg::fail(RG_ERR_INVALID_ARG, "rg_tdistrib_seed_noalloc: ny too large for the fixed workspace");
   int32_t* d_seed = reinterpret_cast<int32_t*>(base);
   int* d_counter = reinterpret_cast<int*>(base) + 1;
   int32_t* d_flag = reinterpret_cast<int32_t*>(base) + 1 + rg::kQueueCounters;
@@ -125,7 +140,7 @@ extern "C" int rg_tdistrib_seed_noalloc(rg_waveguide* wg, int iseed, double* d_t
   a.pot_ystride = 1;
   a.work_counter = d_counter;
   a.flag_list = a.symmetric ? d_flag : nullptr;
-  a.work = large ? reinterpret_cast<double2*>(base + kNoAllocHeaderBytes + pot_bytes) : nullptr;
-  a.work_stride = large ? stride : 0;
+  a.work = reinterpret_cast<double2*>(large ? base + kNoAllocHeaderBytes + pot_bytes : work);
+  a.work_stride = stride;
   return rg::launch_sweep(a, s, grid);
 }

@@ -328,5 +328,257 @@ __device__ void gemm_block(int M, int ti0, int tj0, bool upper, const uint4* adi
     }
 }
 
+// ---------------------------------------------------------------------------
+// Products of T x T tiles held in shared memory by one CTA, for the sweep of
+// up to 64 modes (rg_sweep_sym.cu).
+//
+// A plane holds one digit of every entry: [T row tiles][T column tiles][32
+// lanes] of 16 bytes, a lane's four words being the A fragment (a0, a1, a2,
+// a3) of the layouts above -- which is the accumulator layout of two n8
+// tiles, so the owner warp writes its planes from registers.  The same words
+// read as a B operand are the transposed tile: (a0, a2) are the fragment of
+// columns (= stored rows) 0..7 and (a1, a3) that of 8..15, so these pairs are
+// stored together, and swapped in odd octets of lanes: the 8-byte loads of
+// one pair are then free of bank conflicts.
+// Entries are signed fixed point of 8 + 9 (n - 1) bits, cut into n balanced
+// digits in [-256, 255] (the top one up to 256).
+// ---------------------------------------------------------------------------
+
+// x 2^(53-e) rounded to nearest, with sign (|x| < 2^(e+1)).
+__device__ __forceinline__ long long sfixed53(double x, int e) {
+  const long long m = (long long)(fexp(x) > e ? fixed53(x, e + 1) << 1 : fixed53(x, e));
+  return x < 0.0 ? -m : m;
+}
+
+// x 2^(62-e) as an integer (|x| < 2^e): every bit of entries down to 2^-9 of
+// the row's power of two, rounded to nearest below.
+__device__ __forceinline__ long long sfixed62(double x, int e) {
+  const uint64_t bits = (uint64_t)__double_as_longlong(x);
+  const int eb = (int)((bits >> 52) & 0x7ff);
+  const uint64_t m = (bits & ((1ULL << 52) - 1)) | (1ULL << 52);
+  const int rs = e - (eb - 1022) - 9;  // |x| 2^(62-e) = m 2^-rs
+  long long v = (long long)(m << min(max(-rs, 0), 9));
+  if (rs > 0) v = rs > 54 ? 0 : (long long)((m + (1ULL << (rs - 1))) >> rs);
+  if (eb == 0) v = 0;
+  return x < 0.0 ? -v : v;
+}
+
+// Largest exponents of rows g and g + 8 of a warp's (half) tile, gathered per
+// column half: ex[row].
+__device__ __forceinline__ void put_row_exps(int* ex, int ti, int lane, int e0, int e1) {
+#pragma unroll
+  for (int off = 1; off <= 2; off <<= 1) {
+    e0 = max(e0, __shfl_xor_sync(0xffffffffu, e0, off));
+    e1 = max(e1, __shfl_xor_sync(0xffffffffu, e1, off));
+  }
+  if ((lane & 3) == 0) {
+    ex[ti * 16 + (lane >> 2)] = e0;
+    ex[ti * 16 + (lane >> 2) + 8] = e1;
+  }
+}
+// The row's exponent over the N warps that share it; ex is [N][mp].
+template <int N>
+__device__ __forceinline__ int row_exp(const int* ex, int mp, int row) {
+  int e = ex[row];
+#pragma unroll
+  for (int k = 1; k < N; ++k) e = max(e, ex[k * mp + row]);
+  return e;
+}
+
+// Two digits (fields of 9 bits, 10 at the top) as FP16 halves: (1024 + f) -
+// 1280 = f - 256, exact.
+__device__ __forceinline__ uint32_t field_pair(uint32_t f0, uint32_t f1) {
+  const uint32_t biased = (0x6400u | f0) | ((0x6400u | f1) << 16);
+  __half2 h;
+  memcpy(&h, &biased, 4);
+  h = __hsub2(h, __floats2half2_rn(1280.0f, 1280.0f));
+  uint32_t r;
+  memcpy(&r, &h, 4);
+  return r;
+}
+
+// A lane's words of one plane to their place (s: odd octet).
+template <int NE>
+__device__ __forceinline__ void put_words(const uint32_t* w, uint4* d, int s, int half) {
+  if (NE == 8) {
+    *d = s ? make_uint4(w[1], w[3], w[0], w[2]) : make_uint4(w[0], w[2], w[1], w[3]);
+  } else {
+    uint32_t* d32 = reinterpret_cast<uint32_t*>(d);
+    d32[2 * s + half] = w[0];
+    d32[2 * (1 - s) + half] = w[1];
+  }
+}
+
+// Writes the top n digits of a lane's 2 NE values (NE real parts, then NE
+// imaginary parts; NE = 8: the whole tile, NE = 4: its column half `half`) to
+// the planes: real parts in planes 0..n-1, imaginary parts in planes
+// np..np+n-1, `plane` uint4 apart.  The values are signed fixed point of BITS
+// bits after a right shift by sh (a left shift when negative).  The words of
+// a digit that gets no plane (n = D - 1) go to `last`, when given.
+template <int BITS, int NE>
+__device__ __forceinline__ void put_planes(const long long* x, int n, uint4* dst, int plane, int np, int half,
+                                           int sh = 0, uint32_t* last = nullptr) {
+  constexpr int D = (BITS - 8) / kDigitBits + 1;  // digits of the format
+  const int s = (threadIdx.x >> 3) & 1;           // odd octet: pairs swapped
+  long long bias = 0;
+#pragma unroll
+  for (int p = 0; p < D; ++p) bias += 256LL << (kDigitBits * p);
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    unsigned long long y[NE];
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const long long v = x[NE * part + k];
+      y[k] = (unsigned long long)((sh >= 0 ? v >> min(sh, 63) : v << min(-sh, 63)) + bias);
+    }
+#pragma unroll
+    for (int p = 0; p < D; ++p) {
+      if (p < n || last) {
+        uint32_t w[NE / 2];  // words (rows g, g + 8) of each column half
+#pragma unroll
+        for (int k = 0; k < NE / 2; ++k) {
+          const uint32_t mask = p ? 511u : 1023u;
+          w[k] = field_pair((uint32_t)(y[2 * k] >> (kDigitBits * (D - 1 - p))) & mask,
+                            (uint32_t)(y[2 * k + 1] >> (kDigitBits * (D - 1 - p))) & mask);
+        }
+        if (p < n) {
+          put_words<NE>(w, dst + (part * np + p) * plane, s, half);
+        } else {
+#pragma unroll
+          for (int k = 0; k < NE / 2; ++k) last[part * (NE / 2) + k] = w[k];
+        }
+      }
+    }
+  }
+}
+
+// hi 2^sh + lo 2^(sh - 36), truncated, as an integer (it must fit).
+__device__ __forceinline__ long long fix_shift(long long hi, long long lo, int sh) {
+  hi += lo >> 36;
+  const unsigned long long f = ((unsigned long long)lo << 28) >> 1;  // fraction below hi, 63 bits
+  const int s = min(max(sh, 0), 63);
+  const long long r = (hi << s) | (long long)(f >> (63 - s));
+  return r >> min(max(-sh, 0), 63);
+}
+
+// x 2^e rounded to nearest (ties away), in integer instructions: FP64
+// conversions and scalings cost an FP64 issue slot each.  Zero below the
+// normal range.
+__device__ __forceinline__ double fix_to_double(long long x, int e) {
+  const unsigned long long m = (unsigned long long)(x < 0 ? -x : x);
+  const int lz = __clzll((long long)m);
+  const unsigned long long n = m << (lz & 63);  // top bit at 63
+  const unsigned long long mant = (n >> 11) + ((n >> 10) & 1ULL);
+  const int be = e + 63 - lz + 1023;
+  if (m == 0 || be < 1) return 0.0;
+  if (be > 2046) return __longlong_as_double((long long)((x < 0 ? 1ULL << 63 : 0ULL) | 0x7ff0000000000000ULL));
+  return __longlong_as_double((long long)((x < 0 ? 1ULL << 63 : 0ULL) + ((unsigned long long)(be - 1) << 52) + mant));
+}
+
+// 2^e (hi 2^-34 + lo 2^-70), rounded once from 62 significant bits.
+__device__ __forceinline__ double fold_to_double(long long hi, long long lo, int e) {
+  hi += lo >> 36;
+  const unsigned long long f = ((unsigned long long)lo << 28) >> 1;
+  const int s = min(36, __clzll(hi < 0 ? ~hi : hi) - 2);  // |hi| 2^s < 2^62
+  return fix_to_double((hi << s) | (long long)(f >> (63 - s)), e - 34 - s);
+}
+
+// The sums hi, lo of one 16 x 8 half of a tile of A B^T' (B in transposed
+// planes, see above): levels 0..LMAX of NA and NB digits.  a0 and a1 point at
+// the lane's word pairs (a0, a2) and (a1, a3) of the tile row's first tile, b
+// at the pair of the wanted half of the tile column's first tile; SA, SB are
+// the bytes between real and imaginary planes, `plane` those of a plane.
+// Element w of re (im) is hi[w] (hi[4 + w]), in the accumulator layout.
+// Three levels are summed side by side, so an A digit serves three B digits
+// and each B digit is loaded once per group: 128 bytes of shared memory per
+// mma.sync, half of what one level at a time reads (which is the rate at
+// which shared memory, not the tensor pipe, is the limit).  A level of n
+// digit pairs adds at most n 2^21 per k tile: with up to four pairs a level
+// the sums of two k tiles stay within 2^24, and are folded together.
+// A seventh digit of B (NB = 7) has its real plane at b6 and its imaginary
+// plane after it.
+template <int T, int NA, int NB, int LMAX>
+__device__ __forceinline__ void half_product(const char* a0, const char* a1, int SA, const char* b, int SB, int plane,
+                                             long long* hi, long long* lo, const char* b6 = nullptr) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) hi[k] = lo[k] = 0;
+#pragma unroll
+  for (int L = 0; L <= LMAX; L += 3) {
+    const int top = L + 2 < LMAX ? L + 2 : LMAX;
+    // most digit pairs of a level of the group
+    int np = 0;
+#pragma unroll
+    for (int l = L; l <= top; ++l) {
+      int c = 0;
+#pragma unroll
+      for (int p = 0; p < NA; ++p) c += (l - p >= 0 && l - p < NB) ? 1 : 0;
+      np = c > np ? c : np;
+    }
+    const int KF = np <= 4 && T > 1 ? 2 : 1;  // k tiles per fold
+#pragma unroll 1
+    for (int tk0 = 0; tk0 < T; tk0 += KF) {
+      float acc[3][8];
+#pragma unroll
+      for (int v = 0; v < 3; ++v)
+#pragma unroll
+        for (int w = 0; w < 8; ++w) acc[v][w] = 0.0f;
+#pragma unroll 1
+      for (int tk = tk0; tk < tk0 + KF && tk < T; ++tk) {
+        const char* pa0 = a0 + tk * 512;
+        const char* pa1 = a1 + tk * 512;
+        const char* pb = b + tk * 512;
+        uint2 br[3], bi[3];
+#pragma unroll
+        for (int q = 0; q < NB; ++q)  // the digits the first A digit meets
+          if (q >= L && q <= top) {
+            const char* pq = q == 6 ? b6 + tk * 512 : pb + q * plane;
+            br[q % 3] = *reinterpret_cast<const uint2*>(pq);
+            bi[q % 3] = *reinterpret_cast<const uint2*>(pq + (q == 6 ? plane : SB));
+          }
+#pragma unroll
+        for (int p = 0; p < NA; ++p) {
+          if (p > 0 && L - p >= 0 && L - p < NB) {
+            br[(L - p) % 3] = *reinterpret_cast<const uint2*>(pb + (L - p) * plane);
+            bi[(L - p) % 3] = *reinterpret_cast<const uint2*>(pb + SB + (L - p) * plane);
+          }
+          if (top - p >= 0 && L - p < NB) {
+            const uint2 r0 = *reinterpret_cast<const uint2*>(pa0 + p * plane);
+            const uint2 r1 = *reinterpret_cast<const uint2*>(pa1 + p * plane);
+            const uint2 i0 = *reinterpret_cast<const uint2*>(pa0 + SA + p * plane);
+            const uint2 i1 = *reinterpret_cast<const uint2*>(pa1 + SA + p * plane);
+            const uint4 ar = make_uint4(r0.x, r1.x, r0.y, r1.y), ai = make_uint4(i0.x, i1.x, i0.y, i1.y);
+#pragma unroll
+            for (int v = 0; v < 3; ++v) {
+              const int q = L + v - p;
+              if (q >= 0 && q < NB && L + v <= LMAX) {
+                mma16816(acc[v], ar, br[q % 3].x, br[q % 3].y);
+                mma16816(acc[v] + 4, ar, bi[q % 3].x, bi[q % 3].y);
+              }
+            }
+#pragma unroll
+            for (int v = 0; v < 3; ++v) {
+              const int q = L + v - p;
+              if (q >= 0 && q < NB && L + v <= LMAX) {
+                mma16816(acc[v], ai, bi[q % 3].x ^ 0x80008000u, bi[q % 3].y ^ 0x80008000u);
+                mma16816(acc[v] + 4, ai, br[q % 3].x, br[q % 3].y);
+              }
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < 3; ++v)
+        if (L + v <= LMAX) {
+#pragma unroll
+          for (int w = 0; w < 8; ++w) {
+            const int x = __float2int_rn(acc[v][w]);
+            if (L + v < kHiLevels) hi[w] += (long long)x * (1LL << (kDigitBits * (kHiLevels - 1 - L - v)));
+            else lo[w] += (long long)x * (1LL << (kDigitBits * (kLmax - L - v)));
+          }
+        }
+    }
+  }
+}
+
 }  // namespace oz
 }  // namespace rg

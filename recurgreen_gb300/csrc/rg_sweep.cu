@@ -445,7 +445,7 @@ template <int MCAP, int NT, int MINB>
 int plan_t(SweepArgs& a, int sm_count, int* grid, int64_t* stride) {
   a.cluster = 1;
   const size_t smem = SweepSmem<MCAP>::bytes(a.max_ny);
-  RG_CUDA(cudaFuncSetAttribute(sweep_kernel<MCAP, NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  RG_CUDA(allow_smem((const void*)sweep_kernel<MCAP, NT, MINB>, smem));
   int per_sm = 0;
   RG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_kernel<MCAP, NT, MINB>, NT, smem));
   if (per_sm < 1) return fail(RG_ERR_INVALID_ARG, "sweep kernel does not fit on an SM (ny too large?)");

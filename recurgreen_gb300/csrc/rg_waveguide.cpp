@@ -184,6 +184,7 @@ struct rg_waveguide {
   double kl = 0, kdx = 0, dos = 0, stdu = 0;
   std::vector<double> xmesh, ymesh, kpmesh;
   std::vector<cplx> mumesh, bmat, aedge, abulk, sqmu_c, sqmu_r;
+  std::vector<cplx> wsc, aw;     // B^(-1/2); A/B on edge slices and in the bulk, [2][2][nmu] (rounded, rest)
   std::vector<double> costab;    // [ny][2*nmu+1], Dirichlet
   std::vector<cplx> expfac;      // [ny][nmu], periodic
   std::vector<uint64_t> jump;    // [ny][4]
@@ -191,6 +192,7 @@ struct rg_waveguide {
   int device = 0, sm_count = 0;
   cudaStream_t stream = nullptr;
   double2 *d_bmat = nullptr, *d_aedge = nullptr, *d_abulk = nullptr, *d_sqmu_c = nullptr, *d_sqmu_r = nullptr;
+  double2 *d_wsc = nullptr, *d_aw = nullptr;
   double* d_costab = nullptr;
   double2* d_expfac = nullptr;
   uint64_t* d_jump = nullptr;
@@ -210,7 +212,7 @@ struct rg_waveguide {
   // the next call), one stream per kernel class, and the class launches
   // captured as one CUDA graph (parallel branches), replayed while the
   // launch plans and buffers stay the same.
-  static constexpr int kMultiClasses = 4;
+  static constexpr int kMultiClasses = 5;
   void* d_multi = nullptr;
   size_t multi_bytes = 0;
   cudaStream_t multi_streams[kMultiClasses] = {};
@@ -239,6 +241,8 @@ void free_device(rg_waveguide* w) {
   cudaFree(w->d_bmat);
   cudaFree(w->d_aedge);
   cudaFree(w->d_abulk);
+  cudaFree(w->d_wsc);
+  cudaFree(w->d_aw);
   cudaFree(w->d_sqmu_c);
   cudaFree(w->d_sqmu_r);
   cudaFree(w->d_costab);
@@ -268,7 +272,7 @@ void free_device(rg_waveguide* w) {
   w->ev_sweep0 = w->ev_sweep1 = nullptr;
   w->sweep_timed = false;
   if (w->stream) cudaStreamDestroy(w->stream);
-  w->d_bmat = w->d_aedge = w->d_abulk = w->d_sqmu_c = w->d_sqmu_r = nullptr;
+  w->d_bmat = w->d_aedge = w->d_abulk = w->d_sqmu_c = w->d_sqmu_r = w->d_wsc = w->d_aw = nullptr;
   w->d_costab = nullptr;
   w->d_expfac = nullptr;
   w->d_jump = nullptr;
@@ -277,6 +281,25 @@ void free_device(rg_waveguide* w) {
   w->d_scratch = nullptr;
   w->scratch_bytes = 0;
   w->stream = nullptr;
+}
+
+// a / b = q + rest, both complex FP64: the rest is what a product of q and b
+// (exact, by fused multiply-adds) leaves of a, divided by b.
+void divide_exactly(cplx a, cplx b, cplx* q, cplx* rest) {
+  *q = a / b;
+  // a - q b, term by term: each product as p + (its rounding error)
+  auto residual = [](double x, double q0, double b0, double q1, double b1) {  // x - q0 b0 - q1 b1
+    const double p0 = q0 * b0, p1 = q1 * b1;
+    const double e0 = std::fma(q0, b0, -p0), e1 = std::fma(q1, b1, -p1);
+    const double s = x - p0, z = s - x;                       // two-sum of x and -p0
+    const double es = (x - (s - z)) + (-p0 - z);
+    const double s2 = s - p1, z2 = s2 - s;                    // and of that and -p1
+    const double es2 = (s - (s2 - z2)) + (-p1 - z2);
+    return s2 + ((es + es2) - (e0 + e1));
+  };
+  const cplx r(residual(a.real(), q->real(), b.real(), -q->imag(), b.imag()),
+               residual(a.imag(), q->real(), b.imag(), q->imag(), b.real()));
+  *rest = r / b;
 }
 
 // Host tables of init_waveguide, src/waveguide.f90:81-255.
@@ -346,6 +369,8 @@ int build_tables(rg_waveguide* w, const rg_params& p) {
   w->abulk.resize(M);
   w->sqmu_c.resize(M);
   w->sqmu_r.resize(M);
+  w->wsc.resize(M);
+  w->aw.resize(4 * (size_t)M);
   double dos = 0.0;
   for (int n = 0; n < M; ++n) {
     const double kp = w->kpmesh[n];
@@ -360,6 +385,9 @@ int build_tables(rg_waveguide* w, const rg_params& p) {
     const cplx cot = mu / std::tan(mu * w->kdx);
     w->aedge[n] = iu * mu - cot;
     w->abulk[n] = -2.0 * cot;
+    w->wsc[n] = 1.0 / std::sqrt(w->bmat[n]);
+    divide_exactly(w->aedge[n], w->bmat[n], &w->aw[n], &w->aw[M + n]);
+    divide_exactly(w->abulk[n], w->bmat[n], &w->aw[2 * M + n], &w->aw[3 * M + n]);
     w->sqmu_c[n] = std::sqrt(mu);                              // src/waveguide.f90:443
     w->sqmu_r[n] = cplx(std::sqrt(std::real(mu)), 0.0);       // src/waveguide.f90:510
   }
@@ -400,6 +428,8 @@ int upload_tables(rg_waveguide* w) {
   if ((rc = upload(&w->d_bmat, w->bmat.data(), cb))) return rc;
   if ((rc = upload(&w->d_aedge, w->aedge.data(), cb))) return rc;
   if ((rc = upload(&w->d_abulk, w->abulk.data(), cb))) return rc;
+  if ((rc = upload(&w->d_wsc, w->wsc.data(), cb))) return rc;
+  if ((rc = upload(&w->d_aw, w->aw.data(), 4 * cb))) return rc;
   if ((rc = upload(&w->d_sqmu_c, w->sqmu_c.data(), cb))) return rc;
   if ((rc = upload(&w->d_sqmu_r, w->sqmu_r.data(), cb))) return rc;
   if ((rc = upload(&w->d_costab, w->costab.data(), sizeof(double) * w->costab.size()))) return rc;
@@ -422,6 +452,9 @@ int upload_tables(rg_waveguide* w) {
   d.bmat = w->d_bmat;
   d.adiag_edge = w->d_aedge;
   d.adiag_bulk = w->d_abulk;
+  d.wsc = w->d_wsc;
+  d.aw_edge = w->d_aw;
+  d.aw_bulk = w->d_aw + 2 * w->nmu;
   d.sqmu_c = w->d_sqmu_c;
   d.sqmu_r = w->d_sqmu_r;
   d.costab = w->d_costab;
@@ -1197,7 +1230,7 @@ int rg_tdistrib_multi(rg_waveguide* const* wgs, const int32_t* seeds, int n, con
     }
     item_wg[k] = (int32_t)u;
   }
-  auto klass = [](int M) { return M <= 16 ? 0 : M <= 32 ? 1 : M <= rg::kMaxModesSmem ? 2 : 3; };
+  auto klass = [](int M) { return M <= 16 ? 0 : M <= 32 ? 1 : M <= 48 ? 2 : M <= rg::kMaxModesSmem ? 3 : 4; };
   // Order: by class (largest first), then by decreasing cost M^3 * nx inside a class.
   std::vector<int> order(n);
   for (int k = 0; k < n; ++k) order[k] = k;

@@ -1,0 +1,62 @@
+"""The tensor-core sweep of up to 64 modes (rg_sweep_sym.cu) at the edges of its 16-mode tiles: one mode short of a
+tile, a full one and one more, for every tile count; odd and tiny transverse grids; the shortest guides; the
+deposition matrix, whose source slice lies inside the guide.  Bars as in test_gpu_parity.py: t and r within 1e-10 of
+the oracle (relative Frobenius), T within 1e-9; no realization may need the pivoted kernel."""
+import numpy as np
+import pytest
+
+import oracle as O
+import recurgreen_gb300 as rg
+
+pytestmark = pytest.mark.gpu
+
+
+def guide(m, ny, nx, **kw):
+    return dict(boundtype="dirichlet", nxdiso=nx, nxfree=kw.pop("nxfree", 1), wol=(m + 0.5) / 2, exfac=1.0, aratio=1.0,
+                dscat=3.0, ny=ny, **kw)
+
+
+def rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("dabso", [0.0, 0.4])
+@pytest.mark.parametrize("m", [1, 2, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64])
+def test_tile_edges(m, dabso):
+    kw = guide(m, 2 * m + 1, 6, dabso=dabso)
+    o, g = O.Waveguide(**kw), rg.Waveguide(**kw)
+    u = o.potential(4)
+    ro, to = o.refl_trans_v1_upot(u)
+    r, t = g.refl_trans_v1_upot(u, want_r=True)
+    assert rel(t, to) <= 1e-10 and rel(r, ro) <= 1e-10
+    T = g.tdistrib_batch(np.array([9, 4, 7], np.int32)).reshape(3, -1)
+    assert g.last_batch_info()["kernel"] == "symmetric" and g.last_batch_info()["rerun"] == 0
+    assert np.max(np.abs(T[1] - o.tdistrib_upot(u))) <= 1e-9
+
+
+@pytest.mark.parametrize("m,ny,nx", [(3, 1, 4), (9, 2, 2), (20, 5, 3), (50, 301, 2), (64, 64, 3)])
+def test_small_grids_and_short_guides(m, ny, nx):
+    kw = guide(m, ny, nx, nxfree=0)
+    o, g = O.Waveguide(**kw), rg.Waveguide(**kw)
+    u = o.potential(2)
+    assert rel(g.refl_trans_v1_upot(u), o.refl_trans_v1_upot(u)[1]) <= 1e-10
+
+
+@pytest.mark.parametrize("m", [8, 24, 40, 64])
+def test_source_inside_the_guide(m):
+    kw = guide(m, m, 7)
+    o, g = O.Waveguide(**kw), rg.Waveguide(**kw)
+    for fpos, ipos in ((9, 1), (3, 5), (7, 4)):
+        assert rel(g.compute_deposition(3, fpos, ipos), o.deposition_upot(o.potential(3), fpos, ipos)) <= 1e-10
+
+
+def test_classes_that_share_a_pivoted_kernel():
+    """Guides of 33 to 48 and of 49 to 64 modes are different launches of one multi call, but share the pivoted
+    kernel, whose shared memory follows the widest grid of either."""
+    gs = [rg.Waveguide(**guide(60, 240, 5)), rg.Waveguide(**guide(40, 40, 5))]
+    res, st = rg.tdistrib_multi([(gs[k % 2], 1 + k) for k in range(4)], return_status=True)
+    assert np.all(st == 0) and all(np.any(T > 0) for T in res)
+    for k, T in enumerate(res):
+        one = np.zeros((1 + k) * gs[k % 2].neigv)
+        gs[k % 2].compute_tdistrib(1 + k, one)
+        np.testing.assert_array_equal(T, one[k * gs[k % 2].neigv:])
