@@ -92,97 +92,193 @@ __device__ __forceinline__ double scaled_normal(double stdu, Xoshiro& st) {
   return stdu * (sqrt(-2.0 * log(u1)) * cos(twopi * u2));
 }
 
-// Eigenvalues of t^H t for the nrow x ncol matrix t held in shared memory at
-// W[i * LDW + j], by one-sided (Hestenes) Jacobi on the vectors of the smaller
-// dimension: columns of t if nrow >= ncol, else rows (the singular values of
-// t^T equal those of t).  The largest neigv of T_k = |v_k|^2 go to out in
-// descending order.  Every thread of the NT-thread block calls this; cc
-// (min(nrow, ncol) doubles) and *rot are shared scratch.  Returns false when
-// 60 sweeps did not converge (the same value in every thread).
+// ---------------------------------------------------------------------------
+// Singular values: Householder bidiagonalisation, then bisection.
+// ---------------------------------------------------------------------------
+
+// 1/x to about one ulp for normal x: the hardware's approximation and two
+// Newton steps (a division instruction sequence is twice as long).
+__device__ __forceinline__ double fast_rcp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+// Reflection of a complex vector x (first element a, squared norm xn2 of the
+// others): (I - tau v v^H) x = beta e_1 with v = (1, x[1:] * scale), beta real.
+struct Reflector {
+  double beta;
+  double2 tau, scale;
+};
+__device__ __forceinline__ Reflector reflector(double2 a, double xn2) {
+  Reflector r;
+  if (xn2 == 0.0 && a.y == 0.0) {
+    r.beta = a.x;
+    r.tau = r.scale = make_double2(0.0, 0.0);
+    return r;
+  }
+  r.beta = -copysign(sqrt(fma(a.x, a.x, fma(a.y, a.y, xn2))), a.x);
+  const double rb = 1.0 / r.beta;
+  r.tau = make_double2((r.beta - a.x) * rb, a.y * rb);
+  const double dx = a.x - r.beta;  // no cancellation: beta has the sign opposite to a.x
+  const double den = 1.0 / fma(dx, dx, a.y * a.y);
+  r.scale = make_double2(dx * den, -a.y * den);
+  return r;
+}
+
+// Eigenvalues below mu of B^T B, for the upper bidiagonal B with squared
+// diagonal dd[n] and superdiagonal ee[n - 1]: the negative pivots of its
+// factorisation shifted by mu, in the differential form that never forms B^T B.
+__device__ __forceinline__ int bidiag_count(const double* dd, const double* ee, int n, double mu, double tiny) {
+  double s = -mu;
+  int c = 0;
+  for (int i = 0; i < n; ++i) {
+    double q = dd[i] + s;
+    if (fabs(q) < tiny) q = -tiny;
+    c += q < 0.0 ? 1 : 0;
+    s = fma(ee[i], s * fast_rcp(q), -mu);
+  }
+  return c;
+}
+
+// The largest neig squared singular values of the bidiagonal d[n], e[n - 1]
+// (shared memory; squared in place), descending, to out.  Bisection on sigma
+// down to 2^-54 of its bound, so every value has the absolute accuracy of the
+// reduction; a warp's lanes share out its values, S lanes cutting an interval
+// into S + 1 parts.  Called by NT threads of one CTA, or by CTA `rank` of
+// `parts` (then S = 1: the bits of a value do not depend on the sharing).
 template <int NT>
-__device__ bool tt_eigenvalues(double2* W, int LDW, int nrow, int ncol, int neigv, double* cc, int* rot,
-                               double* out) {
+__device__ void bidiag_values(double* d, double* e, int n, int neig, double* out, int rank = 0, int parts = 0) {
   constexpr int NW = NT / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool bycol = nrow >= ncol;
-  const int nv = bycol ? ncol : nrow;
-  const int L = bycol ? nrow : ncol;
-  const int es = bycol ? LDW : 1;  // element stride inside a vector
-  const int vs = bycol ? 1 : LDW;  // stride between vectors
-  const int NP = (nv + 1) & ~1;
-  const double tol = 2.220446049250313e-16 * L;
-  int sweep = 0;
-  for (; sweep < 60; ++sweep) {
-    if (threadIdx.x == 0) *rot = 0;
-    __syncthreads();
-    for (int rr = 0; rr < NP - 1; ++rr) {
-      // round-robin pairing: position 0 fixed, the others rotate
-      for (int pk = warp; pk < NP / 2; pk += NW) {
-        const int pos1 = pk, pos2 = NP - 1 - pk;
-        const int vp = pos1 == 0 ? 0 : ((pos1 - 1 + rr) % (NP - 1)) + 1;
-        const int vq = ((pos2 - 1 + rr) % (NP - 1)) + 1;
-        if (vp >= nv || vq >= nv) continue;
-        double2* xp = W + vp * vs;
-        double2* xq = W + vq * vs;
-        double al = 0.0, be = 0.0, gr = 0.0, gi = 0.0;
-        for (int i = lane; i < L; i += 32) {
-          const double2 u = xp[i * es], w = xq[i * es];
-          al = fma(u.x, u.x, fma(u.y, u.y, al));
-          be = fma(w.x, w.x, fma(w.y, w.y, be));
-          gr = fma(u.x, w.x, fma(u.y, w.y, gr));   // re(conj(u) w)
-          gi = fma(u.x, w.y, fma(-u.y, w.x, gi));  // im(conj(u) w)
-        }
-#pragma unroll
-        for (int off = 16; off; off >>= 1) {
-          al += __shfl_xor_sync(0xffffffffu, al, off);
-          be += __shfl_xor_sync(0xffffffffu, be, off);
-          gr += __shfl_xor_sync(0xffffffffu, gr, off);
-          gi += __shfl_xor_sync(0xffffffffu, gi, off);
-        }
-        const double ga = sqrt(gr * gr + gi * gi);
-        if (ga > tol * sqrt(al * be) && ga > 1e-300) {
-          if (lane == 0) *rot = 1;
-          const double zeta = (be - al) / (2.0 * ga);
-          const double t = fabs(zeta) > 1e100 ? 0.5 / zeta
-                                              : copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-          const double c = 1.0 / sqrt(1.0 + t * t), s = c * t;
-          const double2 ph = make_double2(gr / ga, -gi / ga);  // exp(-i phi), gamma = |gamma| exp(i phi)
-          for (int i = lane; i < L; i += 32) {
-            const double2 u = xp[i * es];
-            const double2 w = cmul(ph, xq[i * es]);
-            xp[i * es] = make_double2(c * u.x - s * w.x, c * u.y - s * w.y);
-            xq[i * es] = make_double2(s * u.x + c * w.x, s * u.y + c * w.y);
-          }
-        }
-      }
-      __syncthreads();
-    }
-    if (!*rot) break;
-    __syncthreads();
+  __syncthreads();
+  double bound = 0.0, top = 0.0;  // every thread: ||B|| <= bound, largest square
+  bool finite = true;
+  for (int i = lane; i < n; i += 32) {
+    const double di = fabs(d[i]), e0 = i > 0 ? fabs(e[i - 1]) : 0.0, e1 = i + 1 < n ? fabs(e[i]) : 0.0;
+    bound = fmax(bound, di + fmax(e0, e1));
+    top = fmax(top, fmax(di * di, e1 * e1));
+    finite = finite && di + e1 < INFINITY;
   }
-  // T_k = |v_k|^2, ranked in descending order (ties by index).
-  for (int k = warp; k < nv; k += NW) {
-    const double2* xk = W + k * vs;
-    double s = 0.0;
-    for (int i = lane; i < L; i += 32) {
-      const double2 u = xk[i * es];
-      s = fma(u.x, u.x, fma(u.y, u.y, s));
-    }
 #pragma unroll
-    for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (lane == 0) cc[k] = s;
+  for (int off = 16; off; off >>= 1) {
+    bound = fmax(bound, __shfl_xor_sync(0xffffffffu, bound, off));
+    top = fmax(top, __shfl_xor_sync(0xffffffffu, top, off));
+  }
+  finite = __all_sync(0xffffffffu, finite);
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += NT) {
+    d[i] *= d[i];
+    e[i] = i + 1 < n ? e[i] * e[i] : 0.0;
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < nv; k += NT) {
-    const double tk = cc[k];
-    int rank = 0;
-    for (int j = 0; j < nv; ++j) {
-      const double tj = cc[j];
-      rank += (tj > tk || (tj == tk && j < k)) ? 1 : 0;
-    }
-    if (rank < neigv) out[rank] = tk;
+  const int share = parts ? (neig + parts - 1) / parts : neig, j0 = rank * share, cnt = min(share, neig - j0);
+  if (!finite) {
+    for (int k = threadIdx.x; k < cnt; k += NT) out[j0 + k] = NAN;
+    return;
   }
-  return sweep < 60;
+  // warps in use: at least one per scheduler, then a warp per 32 values
+  const int wn = min(NW, max(4, (cnt + 31) / 32));
+  if (warp >= wn) return;
+  const int per = (cnt + wn - 1) / wn;           // values of a warp
+  const double tiny = fmax(1e-40 * top, 1e-300);
+  for (int v0 = 0; v0 < per; v0 += 32) {
+    const int here = min(32, per - v0), S = parts ? 1 : 32 / here;
+    const int grp = lane / S, s = lane % S;
+    const int k = warp * per + v0 + grp;          // position among this sharer's values
+    const bool on = grp < here && k < cnt;
+    const int want = n - 1 - (j0 + k);            // the value has this many below it
+    double lo = 0.0, hi = bound;
+    const double rs = 1.0 / (S + 1);
+    // 54 halvings, or as many cuts into S + 1 parts as shrink the interval alike
+    const int steps = (int)ceilf(54.0f / log2f((float)(S + 1)));
+    for (int it = 0; it < steps; ++it) {
+      const double x = fma(hi - lo, (s + 1) * rs, lo);
+      const bool above = on ? bidiag_count(d, e, n, x * x, tiny) > want : true;
+      const unsigned b = (__ballot_sync(0xffffffffu, above) >> (grp * S)) & (S == 32 ? ~0u : (1u << S) - 1u);
+      const int f = b ? __ffs(b) - 1 : S;         // the first cut above the value
+      const double w = hi - lo, base = lo;
+      if (f < S) hi = fma(w, (f + 1) * rs, base);
+      if (f > 0) lo = fma(w, f * rs, base);
+    }
+    if (on && s == 0) {
+      const double x = 0.5 * (lo + hi);
+      out[j0 + k] = x * x;
+    }
+  }
+}
+
+// Eigenvalues of t^H t for the nrow x ncol matrix t held in shared memory at
+// W[i * LDW + j]: the largest neigv, descending, to out.  Every thread of the
+// NT-thread block calls this; sc is shared scratch of 2 n + 2 max(nrow, ncol)
+// + 4 doubles, n the smaller dimension.
+//
+// Householder reflections from both sides make t real bidiagonal (8/3 n^3
+// complex multiply-adds) and bisection gives the values, as accurate as the
+// reference's zgesvd (absolutely, to the norm of t).  One-sided Jacobi took
+// nine sweeps of 4 n^3 on the same FP64 pipe: 57 M clocks for 64 x 64.
+template <int NT>
+__device__ void tt_eigenvalues(double2* W, int LDW, int nrow, int ncol, int neigv, double* sc, double* out) {
+  constexpr int NW = NT / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool tall = nrow >= ncol;
+  const int m = tall ? nrow : ncol, n = tall ? ncol : nrow;
+  const int rs = tall ? LDW : 1, cs = tall ? 1 : LDW;  // A(i, j) = W[i rs + j cs], t or its transpose
+  double* d = sc;
+  double* e = d + n;
+  double2* v = reinterpret_cast<double2*>(e + n);  // [max(m, n)] reflection vector
+  double2* tau = v + m;                            // [1]
+  // warp 0: the reflector of L elements at x (stride st), conjugated for a row
+  auto reflect = [&](const double2* x, int st, int L, double sg, double* beta) {
+    double xn2 = 0.0;
+    for (int i = 1 + lane; i < L; i += 32) {
+      const double2 u = x[i * st];
+      xn2 = fma(u.x, u.x, fma(u.y, u.y, xn2));
+    }
+#pragma unroll
+    for (int off = 16; off; off >>= 1) xn2 += __shfl_xor_sync(0xffffffffu, xn2, off);
+    const Reflector r = reflector(make_double2(x[0].x, sg * x[0].y), xn2);
+    for (int i = 1 + lane; i < L; i += 32) v[i] = cmul(make_double2(x[i * st].x, sg * x[i * st].y), r.scale);
+    if (lane == 0) {
+      v[0] = make_double2(1.0, 0.0);
+      *tau = r.tau;
+      *beta = r.beta;
+    }
+  };
+  // x <- x - f (v^H x) v for the L elements at x, by one warp (f tau of a
+  // column; for a row both are conjugated, which conjugates v)
+  auto apply = [&](double2* x, int st, int L, double2 f, double sg) {
+    double re = 0.0, im = 0.0;
+    for (int i = lane; i < L; i += 32) {
+      const double2 q = v[i], u = x[i * st];
+      re = fma(q.x, u.x, fma(sg * q.y, u.y, re));
+      im = fma(q.x, u.y, fma(-sg * q.y, u.x, im));
+    }
+    // lanes 0..15 sum re, lanes 16..31 im
+    const double other = __shfl_xor_sync(0xffffffffu, lane < 16 ? im : re, 16);
+    double h = (lane < 16 ? re : im) + other;
+#pragma unroll
+    for (int off = 8; off; off >>= 1) h += __shfl_xor_sync(0xffffffffu, h, off);
+    const double2 w = cmul(f, make_double2(__shfl_sync(0xffffffffu, h, 0), __shfl_sync(0xffffffffu, h, 16)));
+    for (int i = lane; i < L; i += 32) {
+      const double2 q = v[i], u = x[i * st];
+      x[i * st] = make_double2(fma(-w.x, q.x, fma(sg * w.y, q.y, u.x)), fma(-w.x, sg * q.y, fma(-w.y, q.x, u.y)));
+    }
+  };
+  for (int k = 0; k < n; ++k) {
+    if (warp == 0) reflect(W + k * rs + k * cs, rs, m - k, 1.0, d + k);
+    __syncthreads();
+    for (int j = k + 1 + warp; j < n; j += NW) apply(W + k * rs + j * cs, rs, m - k, *tau, 1.0);
+    __syncthreads();
+    if (k + 1 >= n) break;
+    if (warp == 0) reflect(W + k * rs + (k + 1) * cs, cs, n - k - 1, -1.0, e + k);
+    __syncthreads();
+    const double2 tc = make_double2(tau->x, -tau->y);
+    for (int i = k + 1 + warp; i < m; i += NW) apply(W + i * rs + (k + 1) * cs, cs, n - k - 1, tc, -1.0);
+    __syncthreads();
+  }
+  bidiag_values<NT>(d, e, n, min(neigv, n), out);
 }
 
 }  // namespace rg

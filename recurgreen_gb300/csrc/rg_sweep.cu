@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(SweepArgs a) {
   int* sinv = pinv + MCAP;                     // [MCAP] physical row of logical row c
   int* colmap = sinv + MCAP;                   // [MCAP] W column holding Gss column c
   int* used = colmap + MCAP;                   // [MCAP]
-  __shared__ int s_r, s_p, s_status, s_rot;
+  __shared__ int s_r, s_p, s_status;
   __shared__ double2 s_d;
   __shared__ WgDesc wd;
 
@@ -401,10 +401,10 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(SweepArgs a) {
         if (e < nrow * ncol) W[(e % nrow) * LDW + e / nrow] = tv[s];
       }
       __syncthreads();
-      // 6. Eigenvalues of t^H t, sorted descending into teig.
+      // 6. Eigenvalues of t^H t, sorted descending into teig (colbuf, rowW and
+      //    rowR are its scratch).
       const int64_t obase = a.teig_off ? a.teig_off[r] : (int64_t)r * wd.neigv;
-      if (!tt_eigenvalues<NT>(W, LDW, nrow, ncol, wd.neigv, cc, &s_rot, a.teig + obase) && tid == 0)
-        s_status = RG_ERR_NOCONV;
+      tt_eigenvalues<NT>(W, LDW, nrow, ncol, wd.neigv, (double*)colbuf, a.teig + obase);
     }
     __syncthreads();
     if (tid == 0) a.status[r] = s_status;

@@ -44,6 +44,7 @@
 // at a later slice (inject_at), not resume from a state.
 #include <cooperative_groups.h>
 
+#include "rg_bidiag.cuh"
 #include "rg_device.cuh"
 #include "rg_ozaki.cuh"
 
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
   int* piv = (int*)(cc + 2 * MX + 2);       // [M] pivot of step k
   int* used = piv + MX;                     // [M] swept
   int* used0 = used + MX;                   // [M] swept at the start of the panel
-  __shared__ int s_r, s_p, s_status, s_rot;
+  __shared__ int s_r, s_p, s_status;
   __shared__ unsigned long long s_key[NW], s_cmx[NW], s_cmax;
   __shared__ int s_idx[NW];
   __shared__ WgDesc wd;
@@ -993,7 +994,7 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
     }
 
     // 5. Fisher-Lee from R (natural order): t = 2i sqmu Gs1 sqmu, Gs1 = sign R,
-    //    into the workspace, column-major (ld = nrow).
+    //    into the workspace, column-major (t or its transpose).
     const double gsign = (wd.nx >= 2) ? -1.0 : 1.0;
     const int row0 = tmat ? 0 : wd.row0, col0 = tmat ? 0 : wd.col0;
     const int nrow = tmat ? M : wd.nrow, ncol = tmat ? M : wd.ncol;
@@ -1005,97 +1006,16 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
       const double2 g = cscale(gsign, __ldcg(Rg + (int64_t)gi * M + gj));
       const double2 v = cmul(cmul(sqmu[gi], g), sqmu[gj]);
       const double2 t = make_double2(-2.0 * v.y, 2.0 * v.x);
-      Tg[e] = t;
+      Tg[nrow >= ncol ? e : j + i * ncol] = t;  // the larger dimension along a column
       if (tout) tout[e] = t;
     }
     cluster.sync();
 
     if (!tmat) {
-      // 6. Eigenvalues of t^H t: one-sided Jacobi on the vectors of the
-      //    smaller dimension, in the workspace; the pairs of a round are
-      //    split over the cluster's warps.
-      const bool bycol = nrow >= ncol;
-      const int nv = bycol ? ncol : nrow;
-      const int L = bycol ? nrow : ncol;
-      const int es = bycol ? 1 : nrow;
-      const int vs = bycol ? nrow : 1;
-      const int NP = (nv + 1) & ~1;
-      const double tol = 2.220446049250313e-16 * L;
-      int* rot0 = cluster.map_shared_rank(&s_rot, 0);
-      int sweep = 0;
-      for (; sweep < 60; ++sweep) {
-        if (rank == 0 && tid == 0) s_rot = 0;
-        cluster.sync();
-        for (int rr = 0; rr < NP - 1; ++rr) {
-          for (int pk = rank * NW + warp; pk < NP / 2; pk += C * NW) {
-            const int pos1 = pk, pos2 = NP - 1 - pk;
-            const int vp = pos1 == 0 ? 0 : ((pos1 - 1 + rr) % (NP - 1)) + 1;
-            const int vq = ((pos2 - 1 + rr) % (NP - 1)) + 1;
-            if (vp >= nv || vq >= nv) continue;
-            double2* xp = Tg + (int64_t)vp * vs;
-            double2* xq = Tg + (int64_t)vq * vs;
-            double al = 0.0, be = 0.0, gr = 0.0, gi = 0.0;
-            for (int i = lane; i < L; i += 32) {
-              const double2 u = __ldcg(xp + (int64_t)i * es), w = __ldcg(xq + (int64_t)i * es);
-              al = fma(u.x, u.x, fma(u.y, u.y, al));
-              be = fma(w.x, w.x, fma(w.y, w.y, be));
-              gr = fma(u.x, w.x, fma(u.y, w.y, gr));
-              gi = fma(u.x, w.y, fma(-u.y, w.x, gi));
-            }
-#pragma unroll
-            for (int off = 16; off; off >>= 1) {
-              al += __shfl_xor_sync(0xffffffffu, al, off);
-              be += __shfl_xor_sync(0xffffffffu, be, off);
-              gr += __shfl_xor_sync(0xffffffffu, gr, off);
-              gi += __shfl_xor_sync(0xffffffffu, gi, off);
-            }
-            const double ga = sqrt(gr * gr + gi * gi);
-            if (ga > tol * sqrt(al * be) && ga > 1e-300) {
-              if (lane == 0) atomicOr(rot0, 1);
-              const double zeta = (be - al) / (2.0 * ga);
-              const double t = fabs(zeta) > 1e100 ? 0.5 / zeta
-                                                  : copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-              const double c = 1.0 / sqrt(1.0 + t * t), s = c * t;
-              const double2 ph = make_double2(gr / ga, -gi / ga);
-              for (int i = lane; i < L; i += 32) {
-                const double2 u = __ldcg(xp + (int64_t)i * es);
-                const double2 w = cmul(ph, __ldcg(xq + (int64_t)i * es));
-                xp[(int64_t)i * es] = make_double2(c * u.x - s * w.x, c * u.y - s * w.y);
-                xq[(int64_t)i * es] = make_double2(s * u.x + c * w.x, s * u.y + c * w.y);
-              }
-            }
-          }
-          cluster.sync();
-        }
-        const int any = *rot0;
-        cluster.sync();  // every CTA has read the flag before rank 0 clears it
-        if (!any) break;
-      }
-      if (sweep == 60 && tid == 0 && s_status == RG_OK) s_status = RG_ERR_NOCONV;
-      if (rank == 0) {
-        for (int k = warp; k < nv; k += NW) {
-          const double2* xk = Tg + (int64_t)k * vs;
-          double s = 0.0;
-          for (int i = lane; i < L; i += 32) {
-            const double2 u = __ldcg(xk + (int64_t)i * es);
-            s = fma(u.x, u.x, fma(u.y, u.y, s));
-          }
-#pragma unroll
-          for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-          if (lane == 0) cc[k] = s;
-        }
-        __syncthreads();
-        const int64_t obase = a.teig_off ? a.teig_off[r] : (int64_t)r * wd.neigv;
-        for (int k = tid; k < nv; k += NT) {
-          const double tk = cc[k];
-          int rank_k = 0;
-          for (int j = 0; j < nv; ++j) {
-            const double tj = cc[j];
-            rank_k += (tj > tk || (tj == tk && j < k)) ? 1 : 0;
-          }
-          if (rank_k < wd.neigv) a.teig[obase + rank_k] = tk;
-        }
-      }
+      // 6. Eigenvalues of t^H t, on the whole cluster; W and R are free now.
+      const int m = max(nrow, ncol), n = min(nrow, ncol);
+      const int64_t obase = a.teig_off ? a.teig_off[r] : (int64_t)r * wd.neigv;
+      cluster_tt_eigenvalues<NT>(C, rank, Tg, m, n, min(wd.neigv, n), W, sm, a.teig + obase);
     }
     __syncthreads();
     if (rank == 0 && tid == 0) a.status[r] = s_status;

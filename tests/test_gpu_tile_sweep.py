@@ -60,3 +60,18 @@ def test_classes_that_share_a_pivoted_kernel():
         one = np.zeros((1 + k) * gs[k % 2].neigv)
         gs[k % 2].compute_tdistrib(1 + k, one)
         np.testing.assert_array_equal(T, one[k * gs[k % 2].neigv:])
+
+
+@pytest.mark.parametrize("m,napera,naperb", [(1, 1.0, 1.0), (2, 1.0, 0.6), (13, 0.5, 1.0), (33, 1.0, 0.7), (64, 0.9, 0.8),
+                                             (65, 1.0, 1.0), (72, 0.6, 1.0), (100, 1.0, 0.5), (130, 0.03, 1.0)])
+def test_eigenvalues_are_the_squared_singular_values_of_t(m, napera, naperb):
+    """Tall, wide and square filter windows: every singular value within 64 eps ||t|| of LAPACK's for the same t (both
+    reductions are backward stable), whatever the number of CTAs a realization gets."""
+    kw = guide(m, m + 3, 4, dabso=0.2, napera=napera, naperb=naperb)
+    g = rg.Waveguide(**kw)
+    T, t = g.tdistrib_upot(O.Waveguide(**kw).potential(6), want_t=True)
+    s = np.linalg.svd(t, compute_uv=False)
+    assert np.all(np.diff(T) <= 0)
+    assert np.max(np.abs(np.sqrt(T) - s[: T.size])) <= 64 * np.finfo(float).eps * s[0]
+    many = g.tdistrib_batch(np.arange(1, 301, dtype=np.int32)).reshape(300, -1)
+    np.testing.assert_array_equal(many[5], g.tdistrib_batch(np.array([6], np.int32)))
