@@ -148,11 +148,12 @@ struct SweepArgs {
   // of carrying B Gs1 through the Gauss-Jordan sweep (up to 512 modes).
   // Set from RG_TENSOR_R (default on).
   int tensor_r;
-  // With tensor_r, the levels (0..2) of the 2 x 2 block inverse of X in the
-  // blocked symmetric kernel: each level halves an even size of at least 128
-  // modes into two half-size inverses and four half-size tensor-core
-  // products; the blocks left are inverted by FP64 Gauss-Jordan sweeps.
-  // Set from RG_SPLIT_INVERSE (default 2).
+  // With tensor_r, the levels of the 2 x 2 block inverse of X in the blocked
+  // symmetric kernel: each halves a size into two half-size inverses and four
+  // half-size tensor-core products; the blocks left are inverted by FP64
+  // Gauss-Jordan sweeps.  3: as many as the kernel's rule takes; 0..2: at most
+  // that many, of even sizes of at least 128.  Set from RG_SPLIT_INVERSE
+  // (default 3).
   int split_inverse;
 };
 

@@ -57,8 +57,12 @@ constexpr int kSymNT = 256;
 constexpr int kSymNB = 8;
 constexpr int kSymMaxCluster = 8;
 constexpr int kSymMaxRowSplit = 8;
-// The 2 x 2 block inverse for even mode counts from this size up.
-constexpr int kSplitMinModes = 128;
+// The 2 x 2 block inverse: blocks are halved down to at most kLeafModes modes.
+// A Gauss-Jordan block of n modes costs 4 n^3 FP64 flops and n serial steps,
+// so a level takes three quarters of the FP64 work of the one below it and
+// adds four products of half the size.
+constexpr int kLeafModes = 64;
+constexpr int kMaxLevels = 4;  // 512 -> 32
 // Gauss-Jordan blocks of at most this many modes are eliminated in shared
 // memory (gj_small): [n][n+1] matrix, two [n] vectors, [n] flags and the
 // n(n+1)/2 triangle index, within the product staging area.
@@ -104,60 +108,83 @@ __host__ __device__ inline int64_t large_sym_base_stride(int M, int ny) {
   const int64_t urow = ((int64_t)ny + 1) / 2;
   return ((3 * mm + 2 * (int64_t)ny + urow + (int64_t)kSymMaxCluster * kSymNB * M) + 15) & ~(int64_t)15;
 }
-// Then the 2 x 2 block inverse's buffers: three h x h (h = M / 2) for the
-// first level, three (h/2) x (h/2) for the second.
+// Then the 2 x 2 block inverse's buffers: for each level three h x h, h the
+// larger half of that level's blocks (level 0: half of M).
 __host__ __device__ inline int64_t large_sym_schur_offset(int M, int ny) {
   const int64_t ex = ((int64_t)kSymMaxCluster * 2 * 16 * oz::tiles(M) * 4 + 15) / 16;
   return (large_sym_base_stride(M, ny) + 2 * oz::operand_uint4(M) + ex + 15) & ~(int64_t)15;
 }
+__host__ __device__ inline int64_t level_offset(int M, int level) {
+  int64_t o = 0;
+  for (int q = 0; q < level; ++q) {
+    M = (M + 1) / 2;
+    o += 3 * (int64_t)M * M;
+  }
+  return o;
+}
 inline int64_t large_sym_stride(int M, int ny, bool tensor) {
   if (!tensor) return large_sym_base_stride(M, ny);
-  return (large_sym_schur_offset(M, ny) + 3 * (int64_t)(M / 2) * (M / 2) + 3 * (int64_t)(M / 4) * (M / 4) + 15) &
-         ~(int64_t)15;
+  return (large_sym_schur_offset(M, ny) + level_offset(M, kMaxLevels) + 15) & ~(int64_t)15;
 }
 
-// Levels of the 2 x 2 block inverse for M modes, at most `want`: a level
-// halves an even size of at least kSplitMinModes.
+// Levels of the 2 x 2 block inverse for M modes: down to blocks of kLeafModes,
+// or, when fewer are asked for (RG_SPLIT_INVERSE=0..2), at most `want` halvings
+// of even sizes of at least 128.
 __host__ __device__ inline int split_depth(int want, int M) {
   int d = 0;
-  while (d < want && d < 2 && M >= kSplitMinModes && (M % 2) == 0) {
-    ++d;
-    M >>= 1;
+  if (want < 3) {
+    for (; d < want && M >= 128 && M % 2 == 0; ++d) M >>= 1;
+  } else {
+    for (; d < kMaxLevels && M > kLeafModes; ++d) M = (M + 1) / 2;
   }
   return d;
 }
 
-// The steps of the symmetric inverse for 0, 1 and 2 block levels: code =
-// op * 4 + frame (frame 0: X itself; 1: frame 0's block A, inverted in place
-// in its buffer; 2: frame 0's Schur complement S, likewise).
-enum : int { kInvGJ, kInvCopyA, kInvGJA, kInvT, kInvS, kInvGJS, kInvY12, kInvY11, kInvY22 };
-#define RG_INV(op, f) (unsigned char)((op) * 4 + (f))
-__constant__ unsigned char kInvSteps[3][22] = {
-    {RG_INV(kInvGJ, 0)},
-    {RG_INV(kInvCopyA, 0), RG_INV(kInvGJA, 0), RG_INV(kInvT, 0), RG_INV(kInvS, 0), RG_INV(kInvGJS, 0),
-     RG_INV(kInvY12, 0), RG_INV(kInvY11, 0), RG_INV(kInvY22, 0)},
-    {RG_INV(kInvCopyA, 0),
-     RG_INV(kInvCopyA, 1), RG_INV(kInvGJA, 1), RG_INV(kInvT, 1), RG_INV(kInvS, 1), RG_INV(kInvGJS, 1),
-     RG_INV(kInvY12, 1), RG_INV(kInvY11, 1), RG_INV(kInvY22, 1),
-     RG_INV(kInvT, 0), RG_INV(kInvS, 0),
-     RG_INV(kInvCopyA, 2), RG_INV(kInvGJA, 2), RG_INV(kInvT, 2), RG_INV(kInvS, 2), RG_INV(kInvGJS, 2),
-     RG_INV(kInvY12, 2), RG_INV(kInvY11, 2), RG_INV(kInvY22, 2),
-     RG_INV(kInvY12, 0), RG_INV(kInvY11, 0), RG_INV(kInvY22, 0)}};
-#undef RG_INV
-__constant__ int kInvStepCount[3] = {1, 8, 22};
+// The steps of the symmetric inverse for 0 to kMaxLevels block levels.  Node 1
+// is X itself; node k splits into [[A, B], [B^T, D]] with the larger half
+// first: node 2k is its block A, node 2k + 1 its Schur complement S.
+enum : int { kInvGJ, kInvCopyA, kInvT, kInvS, kInvY12, kInvY11, kInvY22 };
+struct InvSteps {
+  int count = 0;
+  unsigned short code[7 * 15 + 1] = {};  // op * 32 + node
+  constexpr void add(int op, int node) { code[count++] = (unsigned short)(op * 32 + node); }
+  constexpr void block(int node, int levels) {
+    if (levels == 0) {
+      add(kInvGJ, node);
+      return;
+    }
+    add(kInvCopyA, node);
+    block(2 * node, levels - 1);
+    add(kInvT, node);
+    add(kInvS, node);
+    block(2 * node + 1, levels - 1);
+    add(kInvY12, node);
+    add(kInvY11, node);
+    add(kInvY22, node);
+  }
+};
+constexpr InvSteps inv_steps(int levels) {
+  InvSteps s;
+  s.block(1, levels);
+  return s;
+}
+__constant__ InvSteps kInvSteps[kMaxLevels + 1] = {inv_steps(0), inv_steps(1), inv_steps(2), inv_steps(3),
+                                                   inv_steps(4)};
 
 __device__ __forceinline__ double2 cneg(double2 a) { return make_double2(-a.x, -a.y); }
 
 // An operand of a cluster product: entry (r, c) is p[r ld + c + off], or,
 // with trans, p[c ld + r + off], or, with sym, the symmetric matrix stored
 // as the upper triangle at p (row stride ld).
+// Entries outside nr x nc are zero.
 struct Opnd {
   const double2* p;
   int64_t ld, off;
-  int sym, trans;
+  int sym, trans, nr, nc;
 };
 
 __device__ __forceinline__ double2 opnd_at(const Opnd& o, int r, int c) {
+  if (r >= o.nr || c >= o.nc) return make_double2(0.0, 0.0);
   if (o.sym) return __ldcg(o.p + (r <= c ? (int64_t)r * o.ld + c : (int64_t)c * o.ld + r));
   return o.trans ? __ldcg(o.p + (int64_t)c * o.ld + r + o.off) : __ldcg(o.p + (int64_t)r * o.ld + c + o.off);
 }
@@ -166,13 +193,14 @@ __device__ __forceinline__ double2 opnd_at(const Opnd& o, int r, int c) {
 //   dst[i ld + j + off] = sign C_ij + aux(i, j)   (only i <= j when upper),
 // aux(i, j) = 0, or aux[i aux_ld + j + aux_off], or, with aux_sym, the
 // symmetric matrix stored as the upper triangle at aux (row stride aux_ld).
+// Only the nr x nc entries of the product proper are written.
 struct TileOut {
   double2* dst;
   int64_t ld, off;
   double sign;
   const double2* aux;
   int64_t aux_ld, aux_off;
-  int aux_sym, upper;
+  int aux_sym, upper, nr, nc;
 };
 
 // One CTA's 2 x 4 block of 16 x 16 output tiles of a cluster product (warp
@@ -184,7 +212,7 @@ struct TileOut {
 __device__ __noinline__ void block_product(int Mb, int ti0, int tj0, const uint4* adig, const uint4* bdig,
                                            const int* ea, const int* eb, uint4* stage, const TileOut* o) {
   oz::gemm_block(Mb, ti0, tj0, o->upper != 0, adig, bdig, ea, eb, stage, [&](int i, int j, double re, double im) {
-    if (o->upper && i > j) return;
+    if (i >= o->nr || j >= o->nc || (o->upper && i > j)) return;
     const double sg = o->sign;
     double2 v = make_double2(sg * re, sg * im);
     if (o->aux) {
@@ -369,16 +397,9 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
     uint4* adig = reinterpret_cast<uint4*>(ws + large_sym_base_stride(M, ny));  // product digit planes
     uint4* bdig = adig + oz::operand_uint4(M);
     int* expart = reinterpret_cast<int*>(bdig + oz::operand_uint4(M));  // [C][2][16 T] partial exponents
-    // the 2 x 2 block inverse's levels (0: one Gauss-Jordan elimination) and
-    // buffers: A^-1, T = A^-1 B, S^-1 (h x h each, h = M / 2), then the same
-    // for the half-size blocks (M / 4 each)
+    // the 2 x 2 block inverse's levels (0: one Gauss-Jordan elimination) and buffers
     const int split_levels = split_depth(gemm_on ? a.split_inverse : 0, M);
-    double2* Wa = ws + large_sym_schur_offset(M, ny);
-    double2* Tb = Wa + (int64_t)(M / 2) * (M / 2);
-    double2* Ws = Tb + (int64_t)(M / 2) * (M / 2);
-    double2* Wa2 = Ws + (int64_t)(M / 2) * (M / 2);
-    double2* Tb2 = Wa2 + (int64_t)(M / 4) * (M / 4);
-    double2* Ws2 = Tb2 + (int64_t)(M / 4) * (M / 4);
+    double2* schur = ws + large_sym_schur_offset(M, ny);
     if (tid == 0) s_status = wd.periodic ? kStatusNeedPivot : RG_OK;  // periodic X is Hermitian, not symmetric
     const double one = a.inject_at > 0 ? 0.0 : 1.0;  // the source at slice 0, or zero until inject_at
     for (int64_t e = ctid; e < mm; e += CNT) Rg[e] = make_double2((e / M) == (e % M) ? one : 0.0, 0.0);
@@ -875,55 +896,65 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
         return __ldcg(Wb + (i <= j ? (int64_t)i * Mb + j : (int64_t)j * Mb + i));
       };
 
-      // X^-1 by its 2 x 2 block form, X = [[A, B], [B^T, D]] with h x h
-      // blocks, two half-size inverses and four half-size products on the
-      // tensor cores:
+      // X^-1 by its 2 x 2 block form, X = [[A, B], [B^T, D]]: two inverses of
+      // half the size and four products on the tensor cores,
       //   T = A^-1 B,  S = D - B^T T,  Y12 = -T S^-1,  Y11 = A^-1 - Y12 T^T,
       //   Y22 = S^-1,
-      // with, at two levels, the half-size inverses of A and S in the same
-      // form.  The steps (kInvSteps) act on frames: frame 0 splits X (at W,
-      // row stride M) with the buffers Wa, Tb, Ws; frames 1 and 2 split A^-1's
-      // block Wa and S's block Ws (row stride h) with Wa2, Tb2, Ws2.  Every
-      // Gauss-Jordan block goes through the one call below.  A small pivot in
-      // a block flags the realization as the full elimination does.
+      // with A and S inverted in the same form, in place in their buffers,
+      // down to the leaves (kInvSteps).  Every Gauss-Jordan block goes through
+      // the one call below.  A small pivot in a block flags the realization
+      // as the full elimination does.
       {
-        const int nsteps = kInvStepCount[split_levels];
-        for (int st = 0; st < nsteps; ++st) {
-          const int code = kInvSteps[split_levels][st];
-          const int op = code >> 2, f = code & 3;
-          double2* P = f == 0 ? W : (f == 1 ? Wa : Ws);
-          const int nP = f == 0 ? M : M >> 1;  // also P's row stride
-          double2* Ha = f == 0 ? Wa : Wa2;
-          double2* Hb = f == 0 ? Tb : Tb2;
-          double2* Hs = f == 0 ? Ws : Ws2;
-          const int h = nP >> 1;
-          const int64_t hh = (int64_t)h * h;
-          if (op == kInvGJ || op == kInvGJA || op == kInvGJS) {
-            double2* Q = op == kInvGJ ? W : (op == kInvGJA ? Ha : Hs);
-            const int nq = op == kInvGJ ? M : h;
-            if (nq <= kSmallGJ) gj_small(Q, nq);
-            else gj(Q, nq);
+        const InvSteps& steps = kInvSteps[split_levels];
+        for (int st = 0; st < steps.count; ++st) {
+          const int op = steps.code[st] >> 5, node = steps.code[st] & 31;
+          // size and place of the node, and of its level's buffers
+          const int depth = 31 - __clz(node);
+          int nP = M, h = M;  // h: the larger half of the level's largest block
+          for (int q = depth - 1; q >= 0; --q) nP = ((node >> q) & 1) ? nP >> 1 : (nP + 1) >> 1;
+          for (int q = 0; q <= depth; ++q) h = (h + 1) >> 1;
+          double2* up = schur + (depth ? level_offset(M, depth - 1) : 0);
+          const int hup = depth ? (M + (1 << depth) - 1) >> depth : 0;  // that half one level up
+          double2* P = depth == 0 ? W : (node & 1) ? up + 2 * (int64_t)hup * hup : up;  // row stride nP
+          double2* Ha = schur + level_offset(M, depth);
+          double2* Hb = Ha + (int64_t)h * h;
+          double2* Hs = Hb + (int64_t)h * h;
+          const int h1 = (nP + 1) >> 1, h2 = nP >> 1;  // A is h1 x h1, S is h2 x h2
+          if (op == kInvGJ) {
+            if (nP <= kSmallGJ) gj_small(P, nP);
+            else gj(P, nP);
           } else if (op == kInvCopyA) {  // A into Ha (upper triangle)
-            for (int64_t e = ctid; e < hh; e += CNT) {
-              const int i = (int)(e / h), j = (int)(e % h);
+            for (int e = ctid; e < h1 * h1; e += CNT) {
+              const int i = e / h1, j = e % h1;
               if (i <= j) Ha[e] = __ldcg(P + (int64_t)i * nP + j);
             }
             cluster.sync();
-          } else if (op == kInvT) {
-            cluster_zgemm(zc, h, Opnd{Ha, h, 0, 1, 0}, Opnd{P, nP, h, 0, 0}, TileOut{Hb, h, 0, 1.0, nullptr, 0, 0, 0, 0});
-          } else if (op == kInvS) {
-            cluster_zgemm(zc, h, Opnd{P, nP, h, 0, 1}, Opnd{Hb, h, 0, 0, 0},
-                          TileOut{Hs, h, 0, -1.0, P, nP, (int64_t)h * nP + h, 0, 1});
-          } else if (op == kInvY12) {
-            cluster_zgemm(zc, h, Opnd{Hb, h, 0, 0, 0}, Opnd{Hs, h, 0, 1, 0}, TileOut{P, nP, h, -1.0, nullptr, 0, 0, 0, 0});
-          } else if (op == kInvY11) {
-            cluster_zgemm(zc, h, Opnd{P, nP, h, 0, 0}, Opnd{Hb, h, 0, 0, 1}, TileOut{P, nP, 0, -1.0, Ha, h, 0, 1, 1});
-          } else {  // kInvY22: Y22 = S^-1
-            for (int64_t e = ctid; e < hh; e += CNT) {
-              const int i = (int)(e / h), j = (int)(e % h);
-              if (i <= j) P[(int64_t)(h + i) * nP + h + j] = __ldcg(Hs + e);
+          } else if (op == kInvY22) {  // Y22 = S^-1
+            for (int e = ctid; e < h2 * h2; e += CNT) {
+              const int i = e / h2, j = e % h2;
+              if (i <= j) P[(int64_t)(h1 + i) * nP + h1 + j] = __ldcg(Hs + e);
             }
             cluster.sync();
+          } else {
+            Opnd A, B;
+            TileOut o{P, nP, h1, -1.0, nullptr, 0, 0, 0, 0, h1, h2};
+            if (op == kInvT) {
+              A = Opnd{Ha, h1, 0, 1, 0, h1, h1};
+              B = Opnd{P, nP, h1, 0, 0, h1, h2};
+              o.dst = Hb, o.ld = h1, o.off = 0, o.sign = 1.0;
+            } else if (op == kInvS) {
+              A = Opnd{P, nP, h1, 0, 1, h2, h1};
+              B = Opnd{Hb, h1, 0, 0, 0, h1, h2};
+              o = TileOut{Hs, h2, 0, -1.0, P, nP, (int64_t)h1 * nP + h1, 0, 1, h2, h2};
+            } else if (op == kInvY12) {
+              A = Opnd{Hb, h1, 0, 0, 0, h1, h2};
+              B = Opnd{Hs, h2, 0, 1, 0, h2, h2};
+            } else {  // kInvY11
+              A = Opnd{P, nP, h1, 0, 0, h1, h2};
+              B = Opnd{Hb, h1, 0, 0, 1, h2, h1};
+              o = TileOut{P, nP, 0, -1.0, Ha, h1, 0, 1, 1, h1, h1};
+            }
+            cluster_zgemm(zc, h1, A, B, o);
           }
         }
       }
@@ -943,7 +974,8 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
           cluster.sync();  // the new right-hand side is complete before the next slice
         } else {
           // the result overwrites B Gs1 in place (its digits are already taken)
-          cluster_zgemm(zc, M, Opnd{W, M, 0, 1, 0}, Opnd{Rg, M, 0, 0, 0}, TileOut{Rg, M, 0, 1.0, nullptr, 0, 0, 0, 0});
+          cluster_zgemm(zc, M, Opnd{W, M, 0, 1, 0, M, M}, Opnd{Rg, M, 0, 0, 0, M, M},
+                        TileOut{Rg, M, 0, 1.0, nullptr, 0, 0, 0, 0, M, M});
         }
       }
       if (a.state_dump && *status0 != kStatusNeedPivot) {

@@ -507,13 +507,14 @@ bool tensor_r_enabled() {
 }
 
 // With the tensor-core product, the levels of the 2 x 2 block inverse of the
-// slice matrix (each halves an even mode count of at least 128): 2 unless
-// RG_SPLIT_INVERSE is 0 or 1.
+// slice matrix: the kernel's rule (3), or, with RG_SPLIT_INVERSE 0, 1 or 2, at
+// most that many, each of an even mode count of at least 128.
 int split_inverse_levels() {
   const char* e = std::getenv("RG_SPLIT_INVERSE");
   if (e && std::strcmp(e, "0") == 0) return 0;
   if (e && std::strcmp(e, "1") == 0) return 1;
-  return 2;
+  if (e && std::strcmp(e, "2") == 0) return 2;
+  return 3;
 }
 
 // Launch arguments for items of this one waveguide (the caller sets nreal,
