@@ -49,7 +49,7 @@ def _stale(target: str, deps: list[str]) -> bool:
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     headers = [os.path.join(CSRC, "rg_internal.h"), os.path.join(CSRC, "rg_device.cuh"),
-               os.path.join(CSRC, "rg_ozaki.cuh"), os.path.join(CSRC, "rg_bidiag.cuh"),
+               os.path.join(CSRC, "rg_ozaki.cuh"), os.path.join(CSRC, "rg_bidiag.cuh"), os.path.join(CSRC, "rg_crt.cuh"),
                os.path.join(ROOT, "include", "recurgreen.h")]
     jobs = []
     objs = []

@@ -1,7 +1,6 @@
 // Batched complex products with FP64 accuracy on the FP16 tensor cores, for
 // the adjoint's per-slice products (rg_zgemm_batched) and for tests
-// (rg_ozaki_zgemm): the device functions of rg_ozaki.cuh, which the blocked
-// symmetric sweep also uses for its propagator product, behind three
+// (rg_ozaki_zgemm): the device functions of rg_ozaki.cuh behind three
 // stream-ordered kernels per call -- exponents, digit planes, product.
 #include <algorithm>
 

@@ -26,14 +26,13 @@
 // factorisation (whose column fetches read W anywhere) from its update, and
 // another ends the update.
 //
-// With tensor_r the sweep inverts X alone (4 M^3 +
-// O(M^2) FP64 flops) and then forms the new right-hand side B Gs1 <- X^-1
-// (B Gs1) as one complex product on the FP16 tensor cores with FP64
-// accuracy (rg_ozaki.cuh: 8 M^3 of the slice's flops leave the FP64 pipe):
-// the row exponents of X^-1 and column exponents of B Gs1 are reduced over
-// the cluster, the cluster writes both operands' digit planes to its
-// workspace, and each CTA computes 16 x 128 column groups of the product,
-// row tile by row tile, with its 8 warps.
+// With tensor_r the sweep inverts X alone, by recursive 2 x 2 blocks
+// (kInvSteps), and then forms the new right-hand side B Gs1 <- X^-1 (B Gs1).
+// The products of both run on the FP16 tensor cores with FP64 accuracy in
+// modular arithmetic (rg_crt.cuh, cluster_zgemm): the row exponents of A and
+// column exponents of B are reduced over the cluster, the cluster writes both
+// operands' residue planes to its workspace, and each CTA computes 64 x 64
+// blocks of the product with its 8 warps.
 //
 // A diagonal pivot below sym_tau times the largest unswept entry of its
 // column flags the realization (kStatusNeedPivot, appended to flag_list);
@@ -45,8 +44,7 @@
 #include <cooperative_groups.h>
 
 #include "rg_bidiag.cuh"
-#include "rg_device.cuh"
-#include "rg_ozaki.cuh"
+#include "rg_crt.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -71,8 +69,8 @@ constexpr int kSmallGJ = 64;
 // The pivot column (panel phase) and the chunk's z values (update phase)
 // share one region: they are never live at the same time.
 //
-// With tensor_r the products' two digit stages (72 KB) and, between
-// products, the shared-memory Gauss-Jordan blocks overlay the start of this
+// With tensor_r the products' stages (64 KB) and, between products, the
+// shared-memory Gauss-Jordan blocks overlay the start of this
 // area (dead during either), and two arrays of 16-padded exponents follow.
 constexpr size_t kSmallGJBytes = sizeof(double2) * (kSmallGJ * (kSmallGJ + 1) + 2 * kSmallGJ) +
                                  sizeof(int) * (kSmallGJ + kSmallGJ * (kSmallGJ + 1) / 2);
@@ -85,9 +83,9 @@ struct LargeSymSmem {
     return sizeof(double2) * ((size_t)M * kSymNB + kSymNB * kSymNB + (size_t)M + kSymNB + shared_region(M)) +
            sizeof(double) * (2 * (size_t)M + 2) + sizeof(int) * 3 * (size_t)M;
   }
-  // the products' staged digits, or a shared-memory Gauss-Jordan block
+  // the products' staged residues, or a shared-memory Gauss-Jordan block
   static constexpr size_t kStage =
-      sizeof(uint4) * oz::kBlkStageUint4 > kSmallGJBytes ? sizeof(uint4) * oz::kBlkStageUint4 : kSmallGJBytes;
+      sizeof(uint4) * crt::kStageUint4 > kSmallGJBytes ? sizeof(uint4) * crt::kStageUint4 : kSmallGJBytes;
   __host__ __device__ static size_t exps_offset(int M) {
     const size_t b = sizeof(double2) * ((size_t)M * kSymNB + kSymNB * kSymNB + (size_t)M + kSymNB + shared_region(M)) +
                      sizeof(double) * (2 * (size_t)M + 2) + sizeof(int) * 3 * (size_t)M;
@@ -101,7 +99,7 @@ struct LargeSymSmem {
 // Workspace of one cluster, in double2 units: W, R, t (M x M each), the
 // generator states (ny x 4 uint64), the paired potential row (ny doubles)
 // and each CTA's raw pivot columns (kSymMaxCluster x NB x M).
-// With tensor_r the digit planes of both product operands and the cluster's
+// With tensor_r the residue planes of both product operands and the cluster's
 // exponent exchange area ([kSymMaxCluster][2][16 T] ints) follow.
 __host__ __device__ inline int64_t large_sym_base_stride(int M, int ny) {
   const int64_t mm = (int64_t)M * M;
@@ -112,7 +110,7 @@ __host__ __device__ inline int64_t large_sym_base_stride(int M, int ny) {
 // larger half of that level's blocks (level 0: half of M).
 __host__ __device__ inline int64_t large_sym_schur_offset(int M, int ny) {
   const int64_t ex = ((int64_t)kSymMaxCluster * 2 * 16 * oz::tiles(M) * 4 + 15) / 16;
-  return (large_sym_base_stride(M, ny) + 2 * oz::operand_uint4(M) + ex + 15) & ~(int64_t)15;
+  return (large_sym_base_stride(M, ny) + 2 * crt::operand_uint4(M) + ex + 15) & ~(int64_t)15;
 }
 __host__ __device__ inline int64_t level_offset(int M, int level) {
   int64_t o = 0;
@@ -122,9 +120,13 @@ __host__ __device__ inline int64_t level_offset(int M, int level) {
   }
   return o;
 }
-inline int64_t large_sym_stride(int M, int ny, bool tensor) {
-  if (!tensor) return large_sym_base_stride(M, ny);
+// Then the scratch of each CTA's product block.
+__host__ __device__ inline int64_t large_sym_block_offset(int M, int ny) {
   return (large_sym_schur_offset(M, ny) + level_offset(M, kMaxLevels) + 15) & ~(int64_t)15;
+}
+inline int64_t large_sym_stride(int M, int ny, bool tensor, int cluster) {
+  if (!tensor) return large_sym_base_stride(M, ny);
+  return large_sym_block_offset(M, ny) + cluster * crt::kBlockUint4;
 }
 
 // Levels of the 2 x 2 block inverse for M modes: down to blocks of kLeafModes,
@@ -189,6 +191,43 @@ __device__ __forceinline__ double2 opnd_at(const Opnd& o, int r, int c) {
   return o.trans ? __ldcg(o.p + (int64_t)c * o.ld + r + o.off) : __ldcg(o.p + (int64_t)r * o.ld + c + o.off);
 }
 
+// Largest exponents of an operand's rows (by_row) or columns into ex (shared
+// memory), by warps w0, w0 + nw, ...: a warp takes storage rows and runs along
+// them, so loads are coalesced whatever the orientation; the maximum along a
+// storage row is reduced over the warp, those along storage columns stay in
+// registers to the end.  (An entry of a stored triangle counts for its row and
+// its column.)
+__device__ __forceinline__ void operand_exps(const Opnd& o, bool by_row, int* ex, int w0, int nw) {
+  const int lane = threadIdx.x & 31;
+  const int R = o.trans ? o.nc : o.nr, N = o.trans ? o.nr : o.nc;  // storage rows and columns
+  const bool rows = o.sym || by_row != (o.trans != 0), cols = o.sym || by_row == (o.trans != 0);
+  for (int b0 = 0; b0 < N; b0 += 128) {
+    int cm[4] = {oz::kNoExp, oz::kNoExp, oz::kNoExp, oz::kNoExp};
+#pragma unroll 2
+    for (int r = w0; r < R; r += nw) {
+      int rm = oz::kNoExp;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int b = b0 + lane + 32 * q;
+        if (b < N && !(o.sym && b < r)) {
+          const int e = oz::fexp2(__ldcg(o.p + (int64_t)r * o.ld + b + o.off));
+          cm[q] = max(cm[q], e);
+          rm = max(rm, e);
+        }
+      }
+      if (rows) {
+        rm = __reduce_max_sync(0xffffffffu, rm);
+        if (lane == 0) atomicMax(ex + r, rm);
+      }
+    }
+    if (cols) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (b0 + lane + 32 * q < N) atomicMax(ex + b0 + lane + 32 * q, cm[q]);
+    }
+  }
+}
+
 // Where one output tile of a cluster product goes:
 //   dst[i ld + j + off] = sign C_ij + aux(i, j)   (only i <= j when upper),
 // aux(i, j) = 0, or aux[i aux_ld + j + aux_off], or, with aux_sym, the
@@ -203,15 +242,13 @@ struct TileOut {
   int aux_sym, upper, nr, nc;
 };
 
-// One CTA's 2 x 4 block of 16 x 16 output tiles of a cluster product (warp
-// w: row tile ti0 + w/4, column tile tj0 + w%4; both operands' digits staged
-// in shared memory per chunk).  The output description o lives in shared
-// memory, so none of its fields holds a register through the tensor-core
-// loop.  Not inlined: one copy of the loop, with its own register
+// One CTA's 64 x 64 block of a cluster product.  The output description o
+// lives in shared memory, so none of its fields holds a register through the
+// tensor-core loop.  Not inlined: one copy of the loop, with its own register
 // allocation, serves all of a slice's products.
 __device__ __noinline__ void block_product(int Mb, int ti0, int tj0, const uint4* adig, const uint4* bdig,
-                                           const int* ea, const int* eb, uint4* stage, const TileOut* o) {
-  oz::gemm_block(Mb, ti0, tj0, o->upper != 0, adig, bdig, ea, eb, stage, [&](int i, int j, double re, double im) {
+                                           const int* ea, const int* eb, uint4* stage, uint4* res, const TileOut* o) {
+  crt::gemm_block(Mb, ti0, tj0, adig, bdig, ea, eb, stage, res, [&](int i, int j, double re, double im) {
     if (i >= o->nr || j >= o->nc || (o->upper && i > j)) return;
     const double sg = o->sign;
     double2 v = make_double2(sg * re, sg * im);
@@ -226,8 +263,8 @@ __device__ __noinline__ void block_product(int Mb, int ti0, int tj0, const uint4
 }
 
 // Where a cluster product keeps its state: the CTA's exponent arrays in
-// shared memory, the cluster's partial exponents and both operands' digit
-// planes in the workspace, and the CTA's staging area.
+// shared memory, the cluster's partial exponents and both operands' residue
+// planes in the workspace, the CTA's staging area and its block's residues.
 struct ZgemmCtx {
   int* ea_s;
   int* eb_s;
@@ -235,16 +272,16 @@ struct ZgemmCtx {
   uint4* adig;
   uint4* bdig;
   uint4* stage;
+  uint4* res;
 };
 
 // A cluster-wide complex product C = A B of two Mb x Mb operands on the
-// tensor cores (rg_ozaki.cuh): exponents reduced over the cluster, digit
-// planes in the workspace, then CTA tasks (blocks of 2 x 4 output tiles,
-// both operands' digits staged in shared memory; with out.upper, blocks
-// wholly below the diagonal are skipped).  The operands are read only in
-// the first two phases, so out may overwrite them.  Called by every thread
-// of the cluster; ends with a cluster barrier.  Not inlined: the slice's
-// five products share one copy.
+// tensor cores (rg_crt.cuh): exponents reduced over the cluster, residue
+// planes in the workspace, then CTA tasks (64 x 64 blocks of the output; with
+// out.upper, blocks wholly below the diagonal are skipped).  The operands are
+// read only in the first two phases, so out may overwrite them.  Called by
+// every thread of the cluster; ends with a cluster barrier.  Not inlined: the
+// products of a slice share one copy.
 __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const Opnd A, const Opnd B,
                                            const TileOut out) {
   cg::cluster_group cluster = cg::this_cluster();
@@ -258,11 +295,8 @@ __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const
     c.eb_s[i] = oz::kNoExp;
   }
   __syncthreads();
-  for (int64_t e = ctid; e < (int64_t)Mb * Mb; e += CNT) {
-    const int i = (int)(e / Mb), j = (int)(e % Mb);
-    atomicMax(c.ea_s + i, oz::fexp2(getA(i, j)));
-    atomicMax(c.eb_s + j, oz::fexp2(getB(i, j)));
-  }
+  operand_exps(A, true, c.ea_s, ctid >> 5, CNT >> 5);
+  operand_exps(B, false, c.eb_s, ctid >> 5, CNT >> 5);
   __syncthreads();
   int* mine = c.expart + rank * 32 * T;
   for (int i = tid; i < 16 * T; i += kSymNT) {
@@ -280,19 +314,18 @@ __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const
     c.eb_s[i] = y;
   }
   __syncthreads();
-  oz::split_a(Mb, getA, c.ea_s, c.adig, ctid, CNT);
-  oz::split_b(Mb, getB, c.eb_s, c.bdig, ctid, CNT);
+  crt::split_a(Mb, getA, c.ea_s, c.adig, ctid, CNT);
+  crt::split_b(Mb, getB, c.eb_s, c.bdig, ctid, CNT);
   __shared__ TileOut s_out;
   if (tid == 0) s_out = out;
-  cluster.sync();  // every digit is written before any CTA reads them (and s_out is set)
-  const int nbr = (T + oz::kBlkRows - 1) / oz::kBlkRows, nbc = (T + oz::kBlkCols - 1) / oz::kBlkCols;
+  cluster.sync();  // every residue is written before any CTA reads them (and s_out is set)
+  const int nb = (T + crt::kBlkTiles - 1) / crt::kBlkTiles;
   int k = 0;
-  for (int bi = 0; bi < nbr; ++bi)
-    for (int bj = 0; bj < nbc; ++bj) {
-      const int ti0 = bi * oz::kBlkRows, tj0 = bj * oz::kBlkCols;
-      if (out.upper && ti0 > tj0 + oz::kBlkCols - 1) continue;
-      if (k++ % C == rank) block_product(Mb, ti0, tj0, c.adig, c.bdig, c.ea_s, c.eb_s, c.stage, &s_out);
-    }
+  for (int bi = 0; bi < nb; ++bi)
+    for (int bj = out.upper ? bi : 0; bj < nb; ++bj)
+      if (k++ % C == rank)
+        block_product(Mb, bi * crt::kBlkTiles, bj * crt::kBlkTiles, c.adig, c.bdig, c.ea_s, c.eb_s, c.stage, c.res,
+                      &s_out);
   cluster.sync();
 }
 
@@ -394,9 +427,9 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
     uint64_t* gen = (uint64_t*)(ws + 3 * mm);     // [ny][4]
     double* urow_g = (double*)(gen + 4 * ny);     // [ny] paired potential row
     double2* PR = (double2*)(urow_g + ((ny + 1) & ~1)) + (int64_t)rank * NB * M;  // [NB][M] this CTA's raw pivot columns
-    uint4* adig = reinterpret_cast<uint4*>(ws + large_sym_base_stride(M, ny));  // product digit planes
-    uint4* bdig = adig + oz::operand_uint4(M);
-    int* expart = reinterpret_cast<int*>(bdig + oz::operand_uint4(M));  // [C][2][16 T] partial exponents
+    uint4* adig = reinterpret_cast<uint4*>(ws + large_sym_base_stride(M, ny));  // product residue planes
+    uint4* bdig = adig + crt::operand_uint4(M);
+    int* expart = reinterpret_cast<int*>(bdig + crt::operand_uint4(M));  // [C][2][16 T] partial exponents
     // the 2 x 2 block inverse's levels (0: one Gauss-Jordan elimination) and buffers
     const int split_levels = split_depth(gemm_on ? a.split_inverse : 0, M);
     double2* schur = ws + large_sym_schur_offset(M, ny);
@@ -492,19 +525,20 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
       //    R = B Gs1 (elements split over the cluster).
       const double2* adiag = (n == 0 || n == wd.nx - 1) ? wd.adiag_edge : wd.adiag_bulk;
       const double rsign = (n == 1) ? 1.0 : -1.0;
-      for (int64_t e = ctid; e < mm; e += CNT) {
-        const int i = (int)(e / M), j = (int)(e % M);
-        if (i <= j) {
-          double2 x = (i == j) ? adiag[i] : make_double2(0.0, 0.0);
-          if (dis) x = csub(x, make_double2(cc[j - i] - cc[i + j + 2], 0.0));
-          if (n > 0) x = csub(x, cmul(cmul(wd.bmat[i], __ldcg(W + e)), wd.bmat[j]));
-          W[e] = x;
+      for (int i = ctid >> 5; i < M; i += CNT >> 5)
+        for (int j = lane; j < M; j += 32) {
+          const int64_t e = (int64_t)i * M + j;
+          if (i <= j) {
+            double2 x = (i == j) ? adiag[i] : make_double2(0.0, 0.0);
+            if (dis) x = csub(x, make_double2(cc[j - i] - cc[i + j + 2], 0.0));
+            if (n > 0) x = csub(x, cmul(cmul(wd.bmat[i], __ldcg(W + e)), wd.bmat[j]));
+            W[e] = x;
+          }
+          // At the source slice the right-hand side is -I (Gs1 = -R after slice 0).
+          if (n > 0)
+            Rg[e] = (n == a.inject_at) ? make_double2(i == j ? -1.0 : 0.0, 0.0)
+                                       : cmul(wd.bmat[i], cscale(rsign, __ldcg(Rg + e)));
         }
-        // At the source slice the right-hand side is -I (Gs1 = -R after slice 0).
-        if (n > 0)
-          Rg[e] = (n == a.inject_at) ? make_double2(i == j ? -1.0 : 0.0, 0.0)
-                                     : cmul(wd.bmat[i], cscale(rsign, __ldcg(Rg + e)));
-      }
       cluster.sync();
       // 3. Blocked symmetric Gauss-Jordan of the M x M symmetric matrix whose
       //    upper triangle is stored at W (row stride M): W becomes its inverse
@@ -837,7 +871,7 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
             double2 d = make_double2(0.0, 0.0);
             if (!singular) {
               const double2 z = Sw[pk * ld + pk];
-              const double rden = 1.0 / fma(z.x, z.x, z.y * z.y);
+              const double rden = fast_rcp(fma(z.x, z.x, z.y * z.y));
               d = make_double2(z.x * rden, -z.y * rden);
             }
             unsigned long long offmax = 0ULL;
@@ -891,7 +925,8 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
           }
         cluster.sync();
       };
-      const ZgemmCtx zc{ea_s, eb_s, expart, adig, bdig, stage};
+      const ZgemmCtx zc{ea_s, eb_s, expart, adig, bdig, stage,
+                        reinterpret_cast<uint4*>(ws + large_sym_block_offset(M, ny)) + rank * crt::kBlockUint4};
       auto wsym = [&](const double2* Wb, int Mb, int i, int j) {  // symmetric matrix from its upper triangle
         return __ldcg(Wb + (i <= j ? (int64_t)i * Mb + j : (int64_t)j * Mb + i));
       };
@@ -924,16 +959,12 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
             if (nP <= kSmallGJ) gj_small(P, nP);
             else gj(P, nP);
           } else if (op == kInvCopyA) {  // A into Ha (upper triangle)
-            for (int e = ctid; e < h1 * h1; e += CNT) {
-              const int i = e / h1, j = e % h1;
-              if (i <= j) Ha[e] = __ldcg(P + (int64_t)i * nP + j);
-            }
+            for (int i = ctid >> 5; i < h1; i += CNT >> 5)
+              for (int j = i + lane; j < h1; j += 32) Ha[i * h1 + j] = __ldcg(P + (int64_t)i * nP + j);
             cluster.sync();
           } else if (op == kInvY22) {  // Y22 = S^-1
-            for (int e = ctid; e < h2 * h2; e += CNT) {
-              const int i = e / h2, j = e % h2;
-              if (i <= j) P[(int64_t)(h1 + i) * nP + h1 + j] = __ldcg(Hs + e);
-            }
+            for (int i = ctid >> 5; i < h2; i += CNT >> 5)
+              for (int j = i + lane; j < h2; j += 32) P[(int64_t)(h1 + i) * nP + h1 + j] = __ldcg(Hs + i * h2 + j);
             cluster.sync();
           } else {
             Opnd A, B;
@@ -967,13 +998,11 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
           // X^-1 (+-I) at the source slice: the full symmetric inverse itself
           // (+I at slice 0, -I at a later source slice)
           const double sg = n == 0 ? 1.0 : -1.0;
-          for (int64_t e = ctid; e < mm; e += CNT) {
-            const int i = (int)(e / M), j = (int)(e % M);
-            Rg[e] = cscale(sg, wsym(W, M, i, j));
-          }
+          for (int i = ctid >> 5; i < M; i += CNT >> 5)
+            for (int j = lane; j < M; j += 32) Rg[(int64_t)i * M + j] = cscale(sg, wsym(W, M, i, j));
           cluster.sync();  // the new right-hand side is complete before the next slice
         } else {
-          // the result overwrites B Gs1 in place (its digits are already taken)
+          // the result overwrites B Gs1 in place (its residues are already taken)
           cluster_zgemm(zc, M, Opnd{W, M, 0, 1, 0, M, M}, Opnd{Rg, M, 0, 0, 0, M, M},
                         TileOut{Rg, M, 0, 1.0, nullptr, 0, 0, 0, 0, M, M});
         }
@@ -984,11 +1013,12 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
         // (S_n, Z_n).
         double2* d1 = a.state_dump + ((int64_t)r * wd.nx + n) * 2 * mm;
         const double gs = (n == 0) ? 1.0 : -1.0;
-        for (int64_t e = ctid; e < mm; e += CNT) {
-          const int i = (int)(e / M), j = (int)(e % M);
-          d1[e] = __ldcg(W + (i <= j ? (int64_t)i * M + j : (int64_t)j * M + i));
-          d1[mm + e] = cscale(gs, __ldcg(Rg + e));
-        }
+        for (int i = ctid >> 5; i < M; i += CNT >> 5)
+          for (int j = lane; j < M; j += 32) {
+            const int64_t e = (int64_t)i * M + j;
+            d1[e] = __ldcg(W + (i <= j ? e : (int64_t)j * M + i));
+            d1[mm + e] = cscale(gs, __ldcg(Rg + e));
+          }
         cluster.sync();  // W and R are read before the next slice rewrites them
       }
     }
@@ -1100,7 +1130,7 @@ int sweep_large_sym_plan(SweepArgs& a, int sm_count, int* grid, int64_t* work_st
   if (nclusters < 1) nclusters = 1;
   a.cluster = C;
   *grid = nclusters * C;
-  *work_stride = large_sym_stride(a.max_M, a.max_ny, tensor);
+  *work_stride = large_sym_stride(a.max_M, a.max_ny, tensor, C);
   return RG_OK;
 }
 
