@@ -50,6 +50,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     os.makedirs(OBJ, exist_ok=True)
     headers = [os.path.join(CSRC, "rg_internal.h"), os.path.join(CSRC, "rg_device.cuh"),
                os.path.join(CSRC, "rg_ozaki.cuh"), os.path.join(CSRC, "rg_bidiag.cuh"), os.path.join(CSRC, "rg_crt.cuh"),
+               os.path.join(CSRC, "rg_tile_inverse.cuh"),
                os.path.join(ROOT, "include", "recurgreen.h")]
     jobs = []
     objs = []

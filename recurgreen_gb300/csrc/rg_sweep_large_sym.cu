@@ -45,6 +45,7 @@
 
 #include "rg_bidiag.cuh"
 #include "rg_crt.cuh"
+#include "rg_tile_inverse.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -56,10 +57,13 @@ constexpr int kSymNB = 8;
 constexpr int kSymMaxCluster = 8;
 constexpr int kSymMaxRowSplit = 8;
 // The 2 x 2 block inverse: blocks are halved down to at most kLeafModes modes.
-// A Gauss-Jordan block of n modes costs 4 n^3 FP64 flops and n serial steps,
-// so a level takes three quarters of the FP64 work of the one below it and
-// adds four products of half the size.
-constexpr int kLeafModes = 64;
+// A Gauss-Jordan block of n modes takes n serial steps of 4,700 clocks
+// (gj_small); two blocks of at most 32 on the tensor cores 58,000 each
+// (leaf_inverse), and the four products that join them 35,000 each
+// (tiny_zgemm).  Leaves of up to 32 against leaves of up to 64: t and r at 100
+// modes (25 or 50) 94 and 108 ms; 304 realizations of 256 modes 218 and 233;
+// one of 256 111 and 145; gradients at 128 84 and 96.
+constexpr int kLeafModes = 32;
 constexpr int kMaxLevels = 4;  // 512 -> 32
 // Gauss-Jordan blocks of at most this many modes are eliminated in shared
 // memory (gj_small): [n][n+1] matrix, two [n] vectors, [n] flags and the
@@ -327,6 +331,130 @@ __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const
         block_product(Mb, bi * crt::kBlkTiles, bj * crt::kBlkTiles, c.adig, c.bdig, c.ea_s, c.eb_s, c.stage, c.res,
                       &s_out);
   cluster.sync();
+}
+
+// A product of at most 32 x 32 by every CTA of the cluster on its own, in
+// shared memory from operands to result (rank 0 writes it): digits of
+// rg_ozaki.cuh in the tile layout of the sweep of up to 64 modes, one warp per
+// column half of the 2 x 2 tiles.  Serial latencies bound it: 35,000 clocks,
+// where the general path's passes through the workspace and its cluster
+// barriers took over 100,000 whatever the size.  Reads the operands before a cluster barrier, writes after it, and
+// ends with another.
+constexpr int kTinyModes = 32;
+__device__ __noinline__ void tiny_zgemm(uint4* stage, const Opnd A, const Opnd B, const TileOut o) {
+  cg::cluster_group cluster = cg::this_cluster();
+  constexpr int T = 2, PL = T * T * 32, MP = 16 * T, NE = 4;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t4 = lane & 3, tile = warp >> 1, half = warp & 1, ti = tile >> 1, tj = tile & 1;
+  uint4* pa = stage;
+  uint4* pb = stage + 12 * PL;
+  int* exa = reinterpret_cast<int*>(stage + 24 * PL);  // [4][MP] row exponents by column half, of A
+  int* exb = exa + 4 * MP;                             // and of B^T
+  const int r0 = ti * 16 + g, c0 = tj * 16 + 2 * t4 + 8 * half;
+  double2 a[NE], b[NE];
+  int e[4] = {oz::kNoExp, oz::kNoExp, oz::kNoExp, oz::kNoExp};
+#pragma unroll
+  for (int k = 0; k < NE; ++k) {
+    const int r = r0 + 8 * (k >> 1), c = c0 + (k & 1);
+    a[k] = opnd_at(A, r, c);
+    b[k] = opnd_at(B, c, r);
+    e[k >> 1] = max(e[k >> 1], oz::fexp2(a[k]));
+    e[2 + (k >> 1)] = max(e[2 + (k >> 1)], oz::fexp2(b[k]));
+  }
+  __syncthreads();  // the staging area's previous contents have been used
+  oz::put_row_exps(exa + (2 * tj + half) * MP, ti, lane, e[0], e[1]);
+  oz::put_row_exps(exb + (2 * tj + half) * MP, ti, lane, e[2], e[3]);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    e[q] = oz::row_exp<4>(exa, MP, r0 + 8 * q);
+    e[2 + q] = oz::row_exp<4>(exb, MP, r0 + 8 * q);
+  }
+  {
+    long long x[2 * NE];
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      x[k] = oz::sfixed53(a[k].x, e[k >> 1]);
+      x[NE + k] = oz::sfixed53(a[k].y, e[k >> 1]);
+    }
+    oz::put_planes<53, NE>(x, 6, pa + tile * 32 + lane, PL, 6, half);
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      x[k] = oz::sfixed53(b[k].x, e[2 + (k >> 1)]);
+      x[NE + k] = oz::sfixed53(b[k].y, e[2 + (k >> 1)]);
+    }
+    oz::put_planes<53, NE>(x, 6, pb + tile * 32 + lane, PL, 6, half);
+  }
+  if (cluster.num_blocks() > 1) cluster.sync();
+  else __syncthreads();
+  if (cluster.block_rank() == 0) {
+    const int odd = (lane >> 3) & 1;
+    const char* ca = reinterpret_cast<const char*>(pa) + ti * T * 512 + lane * 16;
+    const char* cb = reinterpret_cast<const char*>(pb) + tj * T * 512 + lane * 16;
+    long long hi[8], lo[8];
+    oz::half_product<T, 6, 6, oz::kLmax>(ca + 8 * odd, ca + 8 * (1 - odd), 6 * 16 * PL, cb + 8 * (odd ^ half), 6 * 16 * PL,
+                                         16 * PL, hi, lo);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const int i = r0 + 8 * (w >> 1), j = c0 + (w & 1);
+      if (i < o.nr && j < o.nc && !(o.upper && i > j)) {
+        const int ex = e[w >> 1] + oz::row_exp<4>(exb, MP, j);
+        double2 v = make_double2(o.sign * oz::fold_to_double(hi[w], lo[w], ex),
+                                 o.sign * oz::fold_to_double(hi[4 + w], lo[4 + w], ex));
+        if (o.aux) {
+          const double2 x = o.aux_sym ? __ldcg(o.aux + (i <= j ? (int64_t)i * o.aux_ld + j : (int64_t)j * o.aux_ld + i))
+                                      : __ldcg(o.aux + (int64_t)i * o.aux_ld + j + o.aux_off);
+          v.x += x.x;
+          v.y += x.y;
+        }
+        o.dst[(int64_t)i * o.ld + j + o.off] = v;
+      }
+    }
+  }
+  if (cluster.num_blocks() > 1) cluster.sync();
+  else __syncthreads();
+}
+
+// The leaf blocks of the inverse, at most 32 modes: the symmetric n x n matrix
+// whose upper triangle is stored at P (row stride n) becomes its inverse.
+// Every CTA of the cluster inverts its own copy in shared memory, rank 0
+// writes it.  Ends with a cluster barrier.  False, with P as it was, where
+// tile_inverse gives up on its pivots in natural order.  (An FP64 Gauss-Jordan
+// elimination takes 150,000 clocks for 32 modes, 4,700 a step.)
+__device__ __noinline__ bool leaf_inverse(double2* P, const int n, const float tau, uint4* stage) {
+  cg::cluster_group cluster = cg::this_cluster();
+  constexpr int T = 2, NE = 4, PL = T * T * 32, MP = 16 * T, NCW = 4;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = warp >> 1;
+  const int r0 = (tile >> 1) * 16 + (lane >> 2), c0 = (tile & 1) * 16 + 2 * (lane & 3) + 8 * (warp & 1);
+  TileSmem ts;
+  ts.regA = stage;
+  ts.regB = stage + 12 * PL;
+  ts.rsum = reinterpret_cast<unsigned long long*>(stage + 24 * PL);
+  ts.red = reinterpret_cast<unsigned*>(ts.rsum + 2);
+  ts.exX = reinterpret_cast<int*>(ts.red + 32);
+  ts.exY = ts.exX + NCW * MP;
+  __shared__ int s_flag;
+  double2 x[NE], gd[NE];
+#pragma unroll
+  for (int k = 0; k < NE; ++k) {
+    const int i = r0 + erow(k), j = c0 + ecol(k);
+    x[k] = i < n && j < n ? __ldcg(P + (i <= j ? i * n + j : j * n + i)) : make_double2(0.0, 0.0);
+  }
+  if (tid == 0) s_flag = RG_OK;
+  __syncthreads();  // the staging area's previous contents have been used
+  int ey0, ey1;
+  const bool ok = tile_inverse<T, NE>(x, n, tau, ts, &s_flag, [] { __syncthreads(); }, [] {}, gd, ey0, ey1);
+  if (cluster.num_blocks() > 1) cluster.sync();  // every CTA has read P
+  if (ok && cluster.block_rank() == 0) {
+#pragma unroll
+    for (int k = 0; k < NE; ++k) {
+      const int i = r0 + erow(k), j = c0 + ecol(k);
+      if (i <= j && j < n) P[i * n + j] = gd[k];
+    }
+  }
+  if (cluster.num_blocks() > 1) cluster.sync();
+  else __syncthreads();
+  return ok;
 }
 
 __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a) {
@@ -956,8 +1084,11 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
           double2* Hs = Hb + (int64_t)h * h;
           const int h1 = (nP + 1) >> 1, h2 = nP >> 1;  // A is h1 x h1, S is h2 x h2
           if (op == kInvGJ) {
-            if (nP <= kSmallGJ) gj_small(P, nP);
-            else gj(P, nP);
+            const float tau = (float)fmin(kNaturalTau * a.sym_tau, 3e38);
+            if (nP > kTinyModes || !leaf_inverse(P, nP, tau, stage)) {
+              if (nP <= kSmallGJ) gj_small(P, nP);
+              else gj(P, nP);
+            }
           } else if (op == kInvCopyA) {  // A into Ha (upper triangle)
             for (int i = ctid >> 5; i < h1; i += CNT >> 5)
               for (int j = i + lane; j < h1; j += 32) Ha[i * h1 + j] = __ldcg(P + (int64_t)i * nP + j);
@@ -985,7 +1116,8 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
               B = Opnd{Hb, h1, 0, 0, 1, h2, h1};
               o = TileOut{P, nP, 0, -1.0, Ha, h1, 0, 1, 1, h1, h1};
             }
-            cluster_zgemm(zc, h1, A, B, o);
+            if (h1 <= kTinyModes) tiny_zgemm(stage, A, B, o);
+            else cluster_zgemm(zc, h1, A, B, o);
           }
         }
       }
