@@ -123,7 +123,7 @@ struct SweepArgs {
   double2* state_dump;        // [nreal][n_end-n_begin][2][M][M] (Gss, Gs1) after every slice, optional
   double2* state_out;         // [nreal][2][M][M] state after slice n_end-1, optional
   int force_large;            // 1: the pivoted blocked kernel even for max_M <= 64 (segment mode with states)
-  // Symmetric sweep (Dirichlet items): the symmetric kernel (shared-memory
+  // Symmetric sweep (Dirichlet items, periodic ones up to 64 modes): the symmetric kernel (shared-memory
   // or blocked, by max_M) runs every item and appends those it cannot pivot
   // stably to flag_list; the pivoted kernel of the same class re-runs them.
   int symmetric;              // 1: symmetric kernel first (needs flag_list)

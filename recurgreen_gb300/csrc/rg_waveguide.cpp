@@ -490,6 +490,10 @@ bool symmetric_enabled() {
   return !(e && std::strcmp(e, "0") == 0);
 }
 
+// The guides it takes: Dirichlet ones, and periodic ones of up to 64 modes,
+// whose kernel works in real modes (rg_sweep_sym.cu).
+bool symmetric_form(int nmu, bool periodic) { return !periodic || nmu <= rg::kMaxModesSmem; }
+
 double symmetric_tau() {
   const char* e = std::getenv("RG_SYM_TAU");
   if (!e || !*e) return rg::kSymTau;
@@ -526,7 +530,7 @@ rg::SweepArgs make_args(const rg_waveguide* w, int mode) {
   a.work_counter = w->d_counter;
   a.max_M = w->nmu;
   a.max_ny = w->ny;
-  a.symmetric = (w->p.boundtype == RG_BOUND_DIRICHLET && symmetric_enabled()) ? 1 : 0;
+  a.symmetric = (symmetric_form(w->nmu, w->p.boundtype == RG_BOUND_PERIODIC) && symmetric_enabled()) ? 1 : 0;
   a.sym_tau = symmetric_tau();
   a.tensor_r = tensor_r_enabled() ? 1 : 0;
   a.split_inverse = split_inverse_levels();
@@ -565,8 +569,8 @@ int place_workspace(rg_waveguide* w, rg::SweepArgs& a, size_t off, int* grid) {
 //     updates a row, not the row's operations);
 //   * up to 64 modes, the persistent CTAs per SM of the shared-memory
 //     kernels (each realization is one CTA's, whatever the grid).
-// The kernel itself (symmetric for Dirichlet guides, pivoted shared-memory
-// for periodic ones up to 64 modes, blocked above) and the panel width of the
+// The kernel itself (symmetric but for periodic guides above 64 modes, which
+// take the blocked one) and the panel width of the
 // blocked elimination (8; another width regroups the rank updates and
 // changes the rounding) are fixed, so a realization gives the same bits in a
 // batch of any size and in a single call.
@@ -910,7 +914,7 @@ int green_view(const rg_waveguide* w, GreenView* out) {
   out->kpmesh = w->kpmesh.data();
   out->sqmu_r = w->sqmu_r.data();
   const SweepArgs a = make_args(w, kModeEig);
-  out->symmetric = a.symmetric;
+  out->symmetric = a.symmetric && !out->periodic;  // states are kept in the modes of the guide
   out->sym_tau = a.sym_tau;
   out->tensor_r = a.tensor_r;
   out->split_inverse = a.split_inverse;
@@ -1310,11 +1314,12 @@ int rg_tdistrib_multi(rg_waveguide* const* wgs, const int32_t* seeds, int n, con
     a.work_counter = d_cnt + cls.size() * rg::kQueueCounters;
     a.max_M = maxM;
     a.max_ny = maxny;
-    // The symmetric kernel when the class has Dirichlet items (it hands
-    // periodic ones straight to the pivoted kernel).
-    bool any_dirichlet = false;
-    for (int k = k0; k < k1; ++k) any_dirichlet = any_dirichlet || !descs[o_wg[k]].periodic;
-    a.symmetric = (any_dirichlet && symmetric_enabled()) ? 1 : 0;
+    // The symmetric kernel when the class has items that it takes (the
+    // blocked one hands periodic items straight to the pivoted kernel).
+    bool any_symmetric = false;
+    for (int k = k0; k < k1; ++k)
+      any_symmetric = any_symmetric || symmetric_form(descs[o_wg[k]].M, descs[o_wg[k]].periodic != 0);
+    a.symmetric = (any_symmetric && symmetric_enabled()) ? 1 : 0;
     a.sym_tau = symmetric_tau();
     a.tensor_r = tensor_r_enabled() ? 1 : 0;
     a.split_inverse = split_inverse_levels();

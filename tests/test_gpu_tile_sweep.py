@@ -75,3 +75,25 @@ def test_eigenvalues_are_the_squared_singular_values_of_t(m, napera, naperb):
     assert np.max(np.abs(np.sqrt(T) - s[: T.size])) <= 64 * np.finfo(float).eps * s[0]
     many = g.tdistrib_batch(np.arange(1, 301, dtype=np.int32)).reshape(300, -1)
     np.testing.assert_array_equal(many[5], g.tdistrib_batch(np.array([6], np.int32)))
+
+
+@pytest.mark.parametrize("dabso,exfac", [(0.0, 1.0), (0.4, 1.3)])
+@pytest.mark.parametrize("m,ny,nxfree", [(1, 1, 0), (1, 6, 1), (3, 3, 1), (15, 15, 0), (17, 40, 2), (31, 33, 1), (33, 16, 0),
+                                         (47, 47, 1), (49, 101, 0), (63, 64, 1)])
+def test_periodic_guides_in_real_modes(m, ny, nxfree, dabso, exfac):
+    """t, r and filtered T of periodic guides, which this kernel sweeps in the modes cos and sin, at tile edges, with
+    closed channels, and on odd, even and tiny grids; a batch gives the single call's bits.  (Closed channels decay by
+    exp(10) over one of these long slices: there the kernel may pass realizations on.)"""
+    kw = dict(boundtype="periodic", nxdiso=6, nxfree=nxfree, wol=(m // 2 + 0.45) / exfac, exfac=exfac, aratio=1.0,
+              dscat=3.0, dabso=dabso, ny=ny, napera=0.8, naperb=0.6)
+    o, g = O.Waveguide(**kw), rg.Waveguide(**kw)
+    assert g.nmu == m
+    u = o.potential(4)
+    ro, to = o.refl_trans_v1_upot(u)
+    r, t = g.refl_trans_v1_upot(u, want_r=True)
+    assert rel(t, to) <= 1e-10 and rel(r, ro) <= 1e-10
+    T = g.tdistrib_batch(np.arange(1, 401, dtype=np.int32)).reshape(400, -1)
+    info = g.last_batch_info()
+    assert info["kernel"] == "symmetric" and (info["rerun"] == 0 or exfac > 1.0)
+    assert np.max(np.abs(T[3] - o.tdistrib_upot(u))) <= 1e-9
+    np.testing.assert_array_equal(T[3], g.tdistrib_batch(np.array([4], np.int32)))
