@@ -15,22 +15,26 @@
 //    product modulo p into two real ones: u_C = u_A u_B, v_C = v_A v_B.  24
 //    real products of M^3 in all, where 26 digit pairs with four real products
 //    each take 104;
+//  * the residues of an integer are its six 9-bit limbs times constants modulo
+//    p, one mma for 16 planes and 8 entries (split);
 //  * residues are balanced, |r| <= 511, exact in FP16; sums over 64 k stay
 //    below 64 511^2 + 511 < 2^24, so they are exact in FP32, and are reduced
 //    modulo p after every 64 k;
-//  * a_m = (C' (P/p_m)^-1) mod p_m for both parts comes from u and v by one
-//    constant each, and C' = sum_m a_m P/p_m - k P with k = the nearest
-//    integer to sum_m a_m / p_m (|C'| < P/8, so an FP32 sum decides it).  The
-//    sum is formed in 96-bit integers in units of 2^23 (error below 2^36, 2^-70
-//    of 2^106), then rounded to FP64 once.
+//  * C'/P = sum_m (u_m + v_m) k_m / p_m modulo 1 with constants k_m (for the
+//    imaginary part u_m - v_m), |C'| < P/8: the fractions k_m / p_m, to 88
+//    bits in balanced base-2^11 digits, are again an mma's other operand, whose
+//    eight sums (below 2^24, exact) make up C'/P modulo 1 in integers.  The
+//    rounding of the fractions is below 2^44 in C' (the operands' own rounding
+//    is near 2^56); the result is rounded to FP64 once.
 //
 // The result depends on neither tiling nor order.  What it replaces in the
 // blocked sweep is the digit loop (oz::gemm_block): 7.5k clocks per 32 x 64
 // block and 16 k with two CTAs on an SM, bound by instructions around the mma
 // (1,400 a warp for 208), the folds of the level sums above all.
 //
-// Layouts: fragment order as in rg_ozaki.cuh.  An operand's planes: uint4 [12
-// moduli][u, v][T row (A) or column (B) tiles][T k tiles][32 lanes].
+// Layout: an operand's planes are uint4 [12 moduli][u, v][T tiles along rows
+// (A) or columns (B)][T k tiles][32 lanes], in the order of the A fragments of
+// A or of B^T: the planes of one serve as the other's.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -42,7 +46,7 @@ namespace rg {
 namespace crt {
 
 constexpr int kMod = 12;
-constexpr int kUnit = 23;  // C' is summed in units of 2^kUnit
+constexpr int kFracBits = 88;  // of C'/P: eight balanced digits of 11 bits
 
 __host__ __device__ inline int64_t operand_uint4(int M) {
   const int64_t T = oz::tiles(M);
@@ -52,16 +56,22 @@ __host__ __device__ inline int64_t operand_uint4(int M) {
 constexpr int64_t kBlockUint4 = 2LL * kMod * 16 * 32;
 
 struct Tables {
-  float p[kMod], inv[kMod];     // modulus and its reciprocal
-  float c[kMod][3];             // 2^14, 2^28, 2^42 mod p
-  float s[kMod][4];             // s 2^(14 j) mod p
-  float k1[kMod], k2[kMod];     // a_re = (u + v) k1, a_im = (u - v) k2 mod p
-  uint32_t g[kMod][3];          // P / p / 2^kUnit, rounded, 32-bit words from the lowest
-  uint32_t q[3];                // P / 2^kUnit, rounded
-  uint32_t off[3];              // sum over m of 1024 g, modulo 2^96
+  float p[kMod], inv[kMod];  // modulus and its reciprocal
+  // Fragments by lane (g, t), pairs of FP16 integers.  Limbs to residues (A
+  // operand, rows = planes 2 m + v; column of the limbs: lane t has limbs 0, 1,
+  // 2 of the 27-bit half t & 1 of the part t >> 1): planes g and g + 8 of limbs
+  // 0, 1; of limb 2; plane g + 16 of limbs 0, 1; of limb 2.
+  uint32_t split[32][6];
+  // Residues to digits of C'/P (B operand, column g = digit g): moduli 2 t, 2 t
+  // + 1 and 2 t + 8, 2 t + 9 for the real part, then for the imaginary part.
+  uint32_t join[32][4];
+  long long top;  // P in kTopBits bits
+  int shift;      // and P = top 2^shift
 };
+constexpr int kTopBits = 63;
 
 typedef unsigned __int128 u128;
+typedef __int128 i128;
 
 constexpr int kModuli[kMod] = {1021, 1013, 1009, 997, 985, 977, 953, 949, 941, 937, 929, 901};
 
@@ -82,36 +92,59 @@ constexpr int root_of_minus_one(int p) {
   return 0;
 }
 
+constexpr uint32_t half_of(int x) {  // FP16 bits of an integer, |x| <= 2048
+  if (x == 0) return 0;
+  uint32_t a = (uint32_t)(x < 0 ? -x : x), e = 25;
+  while (a < 1024) a <<= 1, --e;
+  if (a >= 2048) a >>= 1, ++e;  // (2048 itself)
+  return (x < 0 ? 0x8000u : 0u) | (e << 10) | (a & 1023u);
+}
+constexpr uint32_t half_pair(int a, int b) { return half_of(a) | half_of(b) << 16; }
+
 constexpr Tables make_tables() {
   Tables t{};
   u128 P = 1;
   for (int m = 0; m < kMod; ++m) P *= (u128)kModuli[m];
-  u128 off = 0;
+  int digits[2][kMod][8] = {};
   for (int m = 0; m < kMod; ++m) {
     const int p = kModuli[m];
-    const u128 Pm = P / (u128)p;
-    const int inv = inverse((int)(Pm % (u128)p), p), s = root_of_minus_one(p);
+    const int inv = inverse((int)(P / (u128)p % (u128)p), p), s = root_of_minus_one(p);
     t.p[m] = (float)p;
     t.inv[m] = 1.0f / (float)p;
-    for (int j = 0; j < 4; ++j) {
-      const int c = balanced(1LL << (14 * j), p);
-      if (j > 0) t.c[m][j - 1] = (float)c;
-      t.s[m][j] = (float)balanced((long long)c * s, p);
+    for (int c = 0; c < 2; ++c) {  // C'_re: (u + v)/2, C'_im: (u - v)/(2 s)
+      const int k = balanced((long long)inv * inverse(c ? 2 * s : 2, p), p);
+      i128 f = (i128)k * ((i128)1 << kFracBits) * 2;
+      f = (f + (f < 0 ? -p : p)) / (2 * p);
+      for (int d = 0; d < 8; ++d) {
+        const int r = d < 7 ? (int)(((f + 1024) & 2047) - 1024) : (int)f;
+        digits[c][m][d] = r;
+        f = (f - r) / 2048;
+      }
     }
-    t.k1[m] = (float)balanced((long long)inv * inverse(2, p), p);
-    t.k2[m] = (float)balanced((long long)inv * inverse(2 * s, p), p);
-    const u128 gm = (Pm + ((u128)1 << (kUnit - 1))) >> kUnit;
-    for (int w = 0; w < 3; ++w) t.g[m][w] = (uint32_t)(gm >> (32 * w));
-    off += gm * 1024;
   }
-  const u128 q = (P + ((u128)1 << (kUnit - 1))) >> kUnit;
-  for (int w = 0; w < 3; ++w) {
-    t.q[w] = (uint32_t)(q >> (32 * w));
-    t.off[w] = (uint32_t)(off >> (32 * w));
+  for (int lane = 0; lane < 32; ++lane) {
+    const int g = lane >> 2, q = lane & 3;
+    for (int w = 0; w < 3; ++w) {
+      const int plane = g + 8 * w, p = kModuli[plane >> 1], s = root_of_minus_one(p);
+      int c[3] = {};
+      for (int j = 0; j < 3; ++j) {
+        long long x = (1LL << (9 * j + 27 * (q & 1))) % p;
+        if (q >> 1) x = x * ((plane & 1) ? p - s : s) % p;
+        c[j] = balanced(x, p);
+      }
+      t.split[lane][w < 2 ? w : 4] = half_pair(c[0], c[1]);
+      t.split[lane][w < 2 ? w + 2 : 5] = half_pair(c[2], 0);
+    }
+    for (int c = 0; c < 2; ++c) {
+      t.join[lane][2 * c] = half_pair(digits[c][2 * q][g], digits[c][2 * q + 1][g]);
+      t.join[lane][2 * c + 1] = q < 2 ? half_pair(digits[c][2 * q + 8][g], digits[c][2 * q + 9][g]) : 0;
+    }
   }
+  while ((P >> (t.shift + kTopBits)) != 0) ++t.shift;
+  t.top = (long long)(P >> t.shift);
   return t;
 }
-static __constant__ Tables kT = make_tables();
+static __device__ const Tables kT = make_tables();
 
 constexpr float kMagic = 12582912.0f;  // 1.5 2^23: x + kMagic rounds x to an integer in the low bits
 
@@ -135,15 +168,6 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
   memcpy(&o, &r, 8);
   return o;
 }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  unsigned long long x, y, r;
-  memcpy(&x, &a, 8);
-  memcpy(&y, &b, 8);
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
-  float2 o;
-  memcpy(&o, &r, 8);
-  return o;
-}
 __device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 reduce2(float2 x, float2 mp, float2 inv) {  // mp = -p
   const float2 q = add2(fma2(x, inv, both(kMagic)), both(-kMagic));
@@ -153,16 +177,6 @@ __device__ __forceinline__ float2 reduce2(float2 x, float2 mp, float2 inv) {  //
 __device__ __forceinline__ float reduce(float x, float p, float inv) {
   const float q = fmaf(x, inv, kMagic) - kMagic;
   return fmaf(-q, p, x);
-}
-
-// Balanced base-2^14 limbs of a signed integer below 2^53 + 1, as floats.
-__device__ __forceinline__ void limbs(long long x, float f[4]) {
-  const long long bias = 8192LL * (1 + (1LL << 14) + (1LL << 28));
-  const unsigned long long y = (unsigned long long)(x + bias + (8192LL << 42));
-#pragma unroll
-  for (int j = 0; j < 3; ++j)
-    f[j] = __uint_as_float(0x4B000000u | ((uint32_t)(y >> (14 * j)) & 16383u)) - (8388608.0f + 8192.0f);
-  f[3] = __uint_as_float(0x4B000000u | (uint32_t)(y >> 42)) - (8388608.0f + 8192.0f);
 }
 
 __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
@@ -178,81 +192,86 @@ __device__ __forceinline__ long long fixed(double x, int e) {
   return x < 0.0 ? -m : m;
 }
 
-// The 24 planes' uint4 of one lane of one tile from its 8 complex entries in
-// fragment order and their exponents; dst points at [modulus 0][u][this
-// tile][lane], `plane` uint4 between planes.
-__device__ __forceinline__ void write_residues(const double2 v[8], const int e[8], uint4* dst, int64_t plane) {
-  float2 xr[4][4], xi[4][4];  // [word][limb]
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    float r0[4], r1[4], i0[4], i1[4];
-    limbs(fixed(v[2 * k].x, e[2 * k]), r0);
-    limbs(fixed(v[2 * k + 1].x, e[2 * k + 1]), r1);
-    limbs(fixed(v[2 * k].y, e[2 * k]), i0);
-    limbs(fixed(v[2 * k + 1].y, e[2 * k + 1]), i1);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      xr[k][j] = make_float2(r0[j], r1[j]);
-      xi[k][j] = make_float2(i0[j], i1[j]);
-    }
-  }
-#pragma unroll 1
-  for (int m = 0; m < kMod; ++m) {
-    const float2 mp = both(-kT.p[m]), inv = both(kT.inv[m]);
-    const float2 c1 = both(kT.c[m][0]), c2 = both(kT.c[m][1]), c3 = both(kT.c[m][2]);
-    const float2 s0 = both(kT.s[m][0]), s1 = both(kT.s[m][1]), s2 = both(kT.s[m][2]), s3 = both(kT.s[m][3]);
-    uint32_t u[4], w[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float2 x = fma2(xr[k][3], c3, fma2(xr[k][2], c2, fma2(xr[k][1], c1, xr[k][0])));
-      const float2 y = reduce2(fma2(xi[k][3], s3, fma2(xi[k][2], s2, fma2(xi[k][1], s1, mul2(xi[k][0], s0)))), mp, inv);
-      const float2 a = reduce2(add2(x, y), mp, inv), b = reduce2(fma2(y, both(-1.0f), x), mp, inv);
-      u[k] = pack_half2(a.x, a.y);
-      w[k] = pack_half2(b.x, b.y);
-    }
-    __stcg(dst + (2 * m) * plane, make_uint4(u[0], u[1], u[2], u[3]));
-    __stcg(dst + (2 * m + 1) * plane, make_uint4(w[0], w[1], w[2], w[3]));
-  }
+__device__ __forceinline__ uint32_t sub_half2(uint32_t a, uint32_t b) {
+  __half2 x, y;
+  memcpy(&x, &a, 4);
+  memcpy(&y, &b, 4);
+  x = __hsub2(x, y);
+  memcpy(&a, &x, 4);
+  return a;
+}
+__device__ __forceinline__ uint32_t add_half2(uint32_t a, uint32_t b) {
+  __half2 x, y;
+  memcpy(&x, &a, 4);
+  memcpy(&y, &b, 4);
+  x = __hadd2(x, y);
+  memcpy(&a, &x, 4);
+  return a;
 }
 
-// Residue planes of A: entries A(i, k) = getA(i, k) (zero outside M x M),
-// exponents ea[i].  Task = (row tile, k tile, lane), from task0 by `step`.
-template <class GetA>
-__device__ void split_a(int M, GetA getA, const int* ea, uint4* dig, int task0, int step) {
-  const int T = oz::tiles(M);
+// Residue planes of an operand with rows i = rows of A or columns of B:
+// entries get(i, k) (zero outside M x M), exponents ex[i].  A warp per 16 x 16
+// tile, tiles warp0, warp0 + nwarps, ...; stg: kSplitUint4 of shared memory for
+// each warp of the CTA.  The entries' integers pass through shared memory, so
+// that loads and conversions are made once, and a quad of lanes then has the
+// 27-bit halves of both parts of an entry, three limbs a lane.  Residues by
+// FP32 multiply-adds instead, 18 and 2 roundings for two entries and a modulus,
+// made this phase as long as the product itself at 256 modes.
+constexpr int kSplitUint4 = 32 * 10;  // a lane's 8 entries, and 32 bytes against bank conflicts
+template <class Get>
+__device__ __forceinline__ void split(int M, Get get, const int* ex, uint4* dig, uint4* stg, int warp0, int nwarps) {
+  const int T = oz::tiles(M), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int64_t plane = (int64_t)T * T * 32;
-  for (int task = task0; task < T * T * 32; task += step) {
-    const int lane = task & 31, tk = (task >> 5) % T, ti = (task >> 5) / T;
-    const int r0 = ti * 16 + (lane >> 2), k0 = tk * 16 + 2 * (lane & 3);
-    double2 v[8];
-    int e[8];
+  uint4* st = stg + (threadIdx.x >> 5) * kSplitUint4;
+  const uint32_t* sw = reinterpret_cast<const uint32_t*>(st) + (g >> 1) * 40 + (g & 1) * 4 + t;
+  uint32_t wt[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) wt[k] = kT.split[lane][k];
+  float2 mp[3], inv[3];
+#pragma unroll
+  for (int w = 0; w < 3; ++w) {
+    mp[w] = both(-kT.p[(g >> 1) + 4 * w]);
+    inv[w] = both(kT.inv[(g >> 1) + 4 * w]);
+  }
+  for (int tile = warp0; tile < T * T; tile += nwarps) {
+    const int tk = tile % T, ti = tile / T;
+    const int r0 = ti * 16 + g, k0 = tk * 16 + 2 * t;
+    __syncwarp();  // the last tile's integers have been used
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int r = r0 + 8 * ((k >> 1) & 1), c = k0 + (k & 1) + 8 * (k >> 2);
-      v[k] = r < M && c < M ? getA(r, c) : make_double2(0.0, 0.0);
-      e[k] = r < M ? ea[r] : 0;
+      const double2 v = r < M && c < M ? get(r, c) : make_double2(0.0, 0.0);
+      const int e = r < M ? ex[r] : 0;
+      const long long x = fixed(v.x, e), y = fixed(v.y, e);
+      st[lane * 10 + k] = make_uint4((uint32_t)x & 0x7ffffffu, (uint32_t)(x >> 27), (uint32_t)y & 0x7ffffffu,
+                                     (uint32_t)(y >> 27));
     }
-    write_residues(v, e, dig + ((int64_t)ti * T + tk) * 32 + lane, plane);
-  }
-}
-
-// Residue planes of B: entries B(k, j) = getB(k, j), exponents eb[j].
-template <class GetB>
-__device__ void split_b(int M, GetB getB, const int* eb, uint4* dig, int task0, int step) {
-  const int T = oz::tiles(M);
-  const int64_t plane = (int64_t)T * T * 32;
-  for (int task = task0; task < T * T * 32; task += step) {
-    const int lane = task & 31, tk = (task >> 5) % T, tj = (task >> 5) / T;
-    const int c0 = tj * 16 + (lane >> 2), k0 = tk * 16 + 2 * (lane & 3);
-    double2 v[8];
-    int e[8];
+    __syncwarp();
+    uint4* dst = dig + (int64_t)tile * 32 + g * plane + t;
+#pragma unroll 2
+    for (int grp = 0; grp < 8; ++grp) {  // entries of lanes 4 grp .. 4 grp + 3
+      uint32_t out[3][4];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int c = c0 + 8 * (k >> 2), r = k0 + (k & 1) + 8 * ((k >> 1) & 1);
-      v[k] = r < M && c < M ? getB(r, c) : make_double2(0.0, 0.0);
-      e[k] = c < M ? eb[c] : 0;
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t x = sw[grp * 160 + q * 8];
+        // limbs as FP16: 1024 + l has l in its low bits; the last is signed
+        const uint32_t l01 = (x & 511u) | ((x & 0x3fe00u) << 7) | 0x64006400u;
+        const uint32_t l2 = (uint32_t)(((int)x >> 18) + 512) | 0x64006400u;
+        const uint32_t b0 = sub_half2(l01, 0x64006400u), b1 = sub_half2(l2, 0x64006600u);
+        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        oz::mma16816(c, make_uint4(wt[0], wt[1], wt[2], wt[3]), b0, b1);
+        oz::mma16816(d, make_uint4(wt[4], 0u, wt[5], 0u), b0, b1);
+        const float2 u0 = reduce2(make_float2(c[0], c[1]), mp[0], inv[0]);
+        const float2 u1 = reduce2(make_float2(c[2], c[3]), mp[1], inv[1]);
+        const float2 u2 = reduce2(make_float2(d[0], d[1]), mp[2], inv[2]);
+        out[0][q] = pack_half2(u0.x, u0.y);
+        out[1][q] = pack_half2(u1.x, u1.y);
+        out[2][q] = pack_half2(u2.x, u2.y);
+      }
+#pragma unroll
+      for (int w = 0; w < 3; ++w)
+        __stcg(dst + 8 * w * plane + 4 * grp, make_uint4(out[w][0], out[w][1], out[w][2], out[w][3]));
     }
-    write_residues(v, e, dig + ((int64_t)tj * T + tk) * 32 + lane, plane);
   }
 }
 
@@ -268,8 +287,8 @@ constexpr int kOneUint4 = 2 * 2 * kBlkTiles * kStageK * 32;  // [A, B][u, v][til
 constexpr int kStages = 4;
 constexpr int kStageUint4 = kStages * kOneUint4;
 
-// Stores C_ij by out(i, j, re, im) for i, j < M in the block at tiles (ti0,
-// tj0); res: the CTA's scratch (kBlockUint4).
+// Stores C_ij by out(i, j, 0, re) and out(i, j, 1, im) for i, j < M in the
+// block at tiles (ti0, tj0); res: the CTA's scratch (kBlockUint4).
 template <class Out>
 __device__ void gemm_block(int M, int ti0, int tj0, const uint4* adig, const uint4* bdig, const int* ea, const int* eb,
                            uint4* stg, uint4* res, Out out) {
@@ -342,8 +361,8 @@ __device__ void gemm_block(int M, int ti0, int tj0, const uint4* adig, const uin
         for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
-            oz::mma16816(acc[i][j], af[i], bf[j].x, bf[j].y);
-            oz::mma16816(acc[i][j] + 4, af[i], bf[j].z, bf[j].w);
+            oz::mma16816(acc[i][j], af[i], bf[j].x, bf[j].z);
+            oz::mma16816(acc[i][j] + 4, af[i], bf[j].y, bf[j].w);
           }
       }
     }
@@ -374,88 +393,64 @@ __device__ void gemm_block(int M, int ti0, int tj0, const uint4* adig, const uin
     }
   }
   __syncthreads();  // the residues are written
-  // Chinese remainders, four entries of one n8 tile at a time.
+  // Chinese remainders.  A lane takes the words of lane 8 h + g of a tile, for
+  // moduli 2 t, 2 t + 1 and 2 t + 8, 2 t + 9: row g of an mma is a word's first
+  // entry, row g + 8 its second.  Its sums, two digits of four numbers (two
+  // entries, re and im), go through shared memory, and lane t of a quad ends
+  // up with all digits of number t.
   const int g = lane >> 2, t4 = lane & 3;
+  long long* part = reinterpret_cast<long long*>(stg) + (warp * 8 + g) * 18;  // [4 numbers][4], two against conflicts
+  uint32_t jc[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) jc[k] = kT.join[lane][k];
 #pragma unroll 1
-  for (int task = warp; task < 32; task += 8) {
-    const int n = task & 1, j = (task >> 1) & 1, i = (task >> 2) & 1, qd = task >> 3;
+  for (int task = warp; task < 64; task += 8) {
+    const int h = task & 3, i = (task >> 3) & 1, j = (task >> 2) & 1, qd = task >> 4;
     const int ti = ti0 + 2 * (qd >> 1) + i, tj = tj0 + 2 * (qd & 1) + j;
     if (ti >= T || tj >= T) continue;
-    const uint2* src = reinterpret_cast<const uint2*>(res + (qd * 4 + 2 * i + j) * 32 + lane) + n;
-    unsigned long long s0[8], s1[8], s2[8];  // re of the four entries, then im
-    float2 kf[4];
+    const uint4* src = res + (qd * 4 + 2 * i + j) * 32 + 8 * h + g;
+    uint4 re[4], im[4];  // sums and differences of u and v for the four moduli
 #pragma unroll
-    for (int w = 0; w < 8; ++w) s0[w] = s1[w] = s2[w] = 0ULL;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) kf[w] = make_float2(0.0f, 0.0f);
-    // the residues of four moduli are loaded while those of the last four are used
-    uint2 U[4], V[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      U[q] = __ldcg(src + (2 * q) * 1024);
-      V[q] = __ldcg(src + (2 * q + 1) * 1024);
-    }
-#pragma unroll 1
-    for (int m0 = 0; m0 < kMod; m0 += 4) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int mm = m0 + q;
-        const uint2 Uq = U[q], Vq = V[q];
-        if (mm + 4 < kMod) {
-          U[q] = __ldcg(src + (2 * (mm + 4)) * 1024);
-          V[q] = __ldcg(src + (2 * (mm + 4) + 1) * 1024);
-        }
-        const float2 mp = both(-kT.p[mm]), inv = both(kT.inv[mm]);
-        const uint32_t g0 = kT.g[mm][0], g1 = kT.g[mm][1], g2 = kT.g[mm][2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          __half2 uh, vh;
-          const uint32_t uw = h ? Uq.y : Uq.x, vw = h ? Vq.y : Vq.x;
-          memcpy(&uh, &uw, 4);
-          memcpy(&vh, &vw, 4);
-          const float2 u = __half22float2(uh), v = __half22float2(vh);
-          const float2 x[2] = {mul2(add2(u, v), both(kT.k1[mm])), mul2(fma2(v, both(-1.0f), u), both(kT.k2[mm]))};
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const float2 r = reduce2(x[c], mp, inv);
-            kf[2 * c + h] = fma2(r, inv, kf[2 * c + h]);
-            const float2 am = add2(r, both(kMagic + 1024.0f));  // r + 1024 in the low bits
-            const uint32_t a0 = __float_as_uint(am.x) & 4095u, a1 = __float_as_uint(am.y) & 4095u;
-            const int w = 4 * c + 2 * h;
-            s0[w] += (unsigned long long)a0 * g0;
-            s1[w] += (unsigned long long)a0 * g1;
-            s2[w] += (unsigned long long)a0 * g2;
-            s0[w + 1] += (unsigned long long)a1 * g0;
-            s1[w + 1] += (unsigned long long)a1 * g1;
-            s2[w + 1] += (unsigned long long)a1 * g2;
-          }
-        }
+    for (int k = 0; k < 4; ++k) {
+      re[k] = im[k] = make_uint4(0u, 0u, 0u, 0u);
+      const int mm = 2 * t4 + (k & 1) + 8 * (k >> 1);
+      if (mm < kMod) {
+        const uint4 u = __ldcg(src + (2 * mm) * 512), v = __ldcg(src + (2 * mm + 1) * 512);
+        re[k] = make_uint4(add_half2(u.x, v.x), add_half2(u.y, v.y), add_half2(u.z, v.z), add_half2(u.w, v.w));
+        im[k] = make_uint4(sub_half2(u.x, v.x), sub_half2(u.y, v.y), sub_half2(u.z, v.z), sub_half2(u.w, v.w));
       }
     }
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      const int row = ti * 16 + g + ((w & 2) ? 8 : 0), col = tj * 16 + n * 8 + 2 * t4 + (w & 1);
-      if (row < M && col < M) {
-        const int e = ea[row] + eb[col] - 106 + kUnit;
-        double r[2];
+      auto word = [&](const uint4& x) { return w == 0 ? x.x : w == 1 ? x.y : w == 2 ? x.z : x.w; };
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int x = 4 * c + w;
-          // s - off - k q modulo 2^96, as hi64 : lo32
-          const long long k = (long long)__float2int_rn((x & 1) ? kf[x >> 1].y : kf[x >> 1].x);
-          const unsigned long long t0 = s0[x] - (unsigned long long)kT.off[0];
-          const unsigned long long kq0 = (unsigned long long)(k * (long long)kT.q[0]);
-          const unsigned long long kq1 = (unsigned long long)(k * (long long)kT.q[1]);
-          const unsigned long long kq2 = (unsigned long long)(k * (long long)kT.q[2]);
-          const unsigned long long l0 = t0 - kq0;  // signed, |l0| < 2^49
-          const unsigned long long l1 = s1[x] - kT.off[1] - kq1 + (unsigned long long)((long long)l0 >> 32);
-          const unsigned long long l2 = s2[x] - kT.off[2] - kq2 + (unsigned long long)((long long)l1 >> 32);
-          const long long top = (long long)((l2 << 32) | (l1 & 0xffffffffULL));  // bits 32..95
-          const uint32_t low = (uint32_t)l0;
-          const int sh = min(32, __clzll(top < 0 ? ~top : top) - 2);
-          r[c] = oz::fix_to_double((top << sh) + (long long)((unsigned long long)low >> (32 - sh)), e + 32 - sh);
-        }
-        out(row, col, r[0], r[1]);
+      for (int c = 0; c < 2; ++c) {
+        const uint4* x = c ? im : re;
+        const uint32_t x0 = word(x[0]), x1 = word(x[1]), x2 = word(x[2]), x3 = word(x[3]);
+        float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        oz::mma16816(d, make_uint4(__byte_perm(x0, x1, 0x5410), __byte_perm(x0, x1, 0x7632),
+                                   __byte_perm(x2, x3, 0x5410), __byte_perm(x2, x3, 0x7632)),
+                     jc[2 * c], jc[2 * c + 1]);
+        part[c * 4 + t4] = (long long)__float2int_rn(d[0]) + (long long)__float2int_rn(d[1]) * 2048;
+        part[(2 + c) * 4 + t4] = (long long)__float2int_rn(d[2]) + (long long)__float2int_rn(d[3]) * 2048;
+      }
+      __syncwarp();
+      const longlong2 p01 = *reinterpret_cast<const longlong2*>(part + t4 * 4);
+      const longlong2 p23 = *reinterpret_cast<const longlong2*>(part + t4 * 4 + 2);
+      __syncwarp();
+      const int row = ti * 16 + 2 * h + (g >> 2) + 8 * (w & 1);
+      const int col = tj * 16 + 8 * (w >> 1) + 2 * (g & 3) + (t4 >> 1);
+      if (row < M && col < M) {
+        // C'/P 2^88 = lo + 2^44 hi modulo 2^88: its top 64 bits, and 24 more
+        const long long lo = p01.x + p01.y * (1LL << 22);
+        const unsigned long long hi =
+            (unsigned long long)p23.x + ((unsigned long long)p23.y << 22) + (unsigned long long)(lo >> 44);
+        const long long top = (long long)((hi << 20) | (unsigned)((lo >> 24) & 0xfffff));
+        const unsigned rest = (unsigned)lo & 0xffffffu;
+        const int sh = min(24, __clzll(top < 0 ? ~top : top) - 1);
+        const long long f = (long long)((unsigned long long)top << sh) + (long long)(rest >> (24 - sh));
+        out(row, col, t4 & 1,
+            oz::fix_to_double(__mul64hi(f, kT.top), ea[row] + eb[col] - 106 + kT.shift - sh));
       }
     }
   }

@@ -252,17 +252,15 @@ struct TileOut {
 // allocation, serves all of a slice's products.
 __device__ __noinline__ void block_product(int Mb, int ti0, int tj0, const uint4* adig, const uint4* bdig,
                                            const int* ea, const int* eb, uint4* stage, uint4* res, const TileOut* o) {
-  crt::gemm_block(Mb, ti0, tj0, adig, bdig, ea, eb, stage, res, [&](int i, int j, double re, double im) {
+  crt::gemm_block(Mb, ti0, tj0, adig, bdig, ea, eb, stage, res, [&](int i, int j, int c, double v) {
     if (i >= o->nr || j >= o->nc || (o->upper && i > j)) return;
-    const double sg = o->sign;
-    double2 v = make_double2(sg * re, sg * im);
+    if (o->sign < 0.0) v = -v;
     if (o->aux) {
-      const double2 x = o->aux_sym ? __ldcg(o->aux + (i <= j ? (int64_t)i * o->aux_ld + j : (int64_t)j * o->aux_ld + i))
-                                   : __ldcg(o->aux + (int64_t)i * o->aux_ld + j + o->aux_off);
-      v.x += x.x;
-      v.y += x.y;
+      const int64_t x = o->aux_sym ? (i <= j ? (int64_t)i * o->aux_ld + j : (int64_t)j * o->aux_ld + i)
+                                   : (int64_t)i * o->aux_ld + j + o->aux_off;
+      v += __ldcg(reinterpret_cast<const double*>(o->aux + x) + c);
     }
-    o->dst[(int64_t)i * o->ld + j + o->off] = v;
+    reinterpret_cast<double*>(o->dst + (int64_t)i * o->ld + j + o->off)[c] = v;
   });
 }
 
@@ -291,8 +289,6 @@ __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int tid = threadIdx.x, ctid = rank * kSymNT + tid, CNT = C * kSymNT;
-  auto getA = [&](int i, int k) { return opnd_at(A, i, k); };
-  auto getB = [&](int k, int j) { return opnd_at(B, k, j); };
   const int T = oz::tiles(Mb);
   for (int i = tid; i < 16 * T; i += kSymNT) {
     c.ea_s[i] = oz::kNoExp;
@@ -318,8 +314,8 @@ __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const
     c.eb_s[i] = y;
   }
   __syncthreads();
-  crt::split_a(Mb, getA, c.ea_s, c.adig, ctid, CNT);
-  crt::split_b(Mb, getB, c.eb_s, c.bdig, ctid, CNT);
+  crt::split(Mb, [&](int i, int k) { return opnd_at(A, i, k); }, c.ea_s, c.adig, c.stage, ctid >> 5, CNT >> 5);
+  crt::split(Mb, [&](int j, int k) { return opnd_at(B, k, j); }, c.eb_s, c.bdig, c.stage, ctid >> 5, CNT >> 5);
   __shared__ TileOut s_out;
   if (tid == 0) s_out = out;
   cluster.sync();  // every residue is written before any CTA reads them (and s_out is set)
