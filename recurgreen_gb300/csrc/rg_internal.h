@@ -127,6 +127,7 @@ struct SweepArgs {
   // or blocked, by max_M) runs every item and appends those it cannot pivot
   // stably to flag_list; the pivoted kernel of the same class re-runs them.
   int symmetric;              // 1: symmetric kernel first (needs flag_list)
+  int prop_warps;             // set by sweep_sym_plan: the propagator has warps of its own
   int32_t* flag_list;         // [nreal] flagged item indices
   double sym_tau;             // smallest accepted |diagonal pivot| / max |unswept entry of its row|
   // Queue indirection of the pivoted kernel (set by launch_sweep for the re-run):

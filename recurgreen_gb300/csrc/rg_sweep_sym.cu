@@ -30,7 +30,7 @@
 // within 0.95 to 1.3 (7 to 64 modes, 40 to 300 slices; geometric mean 1.08).
 // Measured, with the eigenvalues: 304 guides of 64 modes and 600 slices 607 ms
 // before, 184 now; 500 of 37 modes and 150 slices 110 ms before, 41 now; one
-// guide of 10 modes and 200 slices 8.2 ms before, 4.4 now.
+// guide of 10 modes and 200 slices 8.2 ms before, 3.4 now.
 //
 // Layout: T = ceil(M/16) tiles a side, one warp per tile or two, as in
 // rg_tile_inverse.cuh.  (Q is kept transposed so that it is only ever an A
@@ -54,9 +54,10 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
 
-// Named barriers: the main warps, the producer warps, and the two buffers of
-// projection coefficients (filled / free again).
-constexpr int kBarMain = 1, kBarProd = 2, kBarFull = 3, kBarFree = 5;
+// Named barriers: the main warps, the producer warps, the two buffers of
+// projection coefficients (filled / free again), the propagator's warps, and
+// the two buffers of G' for them.
+constexpr int kBarMain = 1, kBarProd = 2, kBarFull = 3, kBarFree = 5, kBarProp = 7, kBarGFull = 8, kBarGFree = 10;
 
 // Element (i, j) of modal^T diag(U) modal in the real modes of the guide from
 // its projection coefficients co.  Dirichlet: co[d] = cos coefficient d.
@@ -95,7 +96,12 @@ __device__ __forceinline__ double2 from_real_modes(const double2* F, int ld, int
   return cscale(0.70710678118654752440, make_double2(c.x - f * s.y, c.y + f * s.x));
 }
 
-template <int T>
+// PROP: Q has warps of its own, as many as the main ones, one slice behind
+// them.  Q_n does not feed the recursion of G', so a slice's chain is then the
+// inverse alone.  They cost registers and shared memory, so the CTAs per SM
+// fall from 4 to 2 (up to 16 modes) and from 2 to 1 (up to 32): taken while
+// every realization has its CTA at once (prop_warps).
+template <int T, bool PROP>
 struct SymCfg {
   static constexpr int MP = 16 * T;                // padded modes
   static constexpr int NE = T == 4 ? 8 : 4;        // complex entries per lane: a whole tile, or its column half
@@ -104,13 +110,15 @@ struct SymCfg {
   static constexpr int NMAIN = 32 * T * T * NHALF;
   // Producer threads.  Registers are handed out to four warps at a time.
   static constexpr int PROD = T == 4 ? 128 : 64;
-  static constexpr int NT = NMAIN + PROD;
-  static constexpr int MINB = T == 1 ? 4 : T == 2 ? 2 : 1;  // CTAs per SM
+  static constexpr int NPROP = PROP ? NMAIN : 0;
+  static constexpr int NT = NMAIN + PROD + NPROP;
+  static constexpr int MINB = T == 1 ? (PROP ? 2 : 4) : T == 2 && !PROP ? 2 : 1;  // CTAs per SM
   static constexpr int PL = T * T * 32;            // uint4 of one digit plane
   static constexpr int LDW = MP + 1;
   static constexpr size_t bytes() {
     return sizeof(uint4) * 24 * PL + sizeof(double) * (2 * (2 * MP + 2) + PROD) + sizeof(unsigned long long) * 2 +
-           sizeof(unsigned) * 32 + sizeof(int) * 3 * NCW * MP;
+           sizeof(unsigned) * 32 + sizeof(int) * 3 * NCW * MP +
+           (PROP ? sizeof(uint4) * 24 * PL + sizeof(double2) * 2 * NMAIN * NE + sizeof(int) * 2 * MP : 0);
   }
 };
 
@@ -120,9 +128,9 @@ inline int64_t sym_stride(int T, int max_ny) {
   return (2 * (int64_t)max_ny + (max_ny + 1) / 2 + 3 * (int64_t)T * T * 256 + 15) & ~(int64_t)15;
 }
 
-template <int T>
-__global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kernel(SweepArgs a) {
-  using Cf = SymCfg<T>;
+template <int T, bool PROP>
+__global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sweep_sym_kernel(SweepArgs a) {
+  using Cf = SymCfg<T, PROP>;
   constexpr int MP = Cf::MP, NMAIN = Cf::NMAIN, NT = Cf::NT, PL = Cf::PL, LDW = Cf::LDW, kProd = Cf::PROD;
   constexpr int NE = Cf::NE, NV = 2 * NE, NHALF = Cf::NHALF, NCW = Cf::NCW;
   extern __shared__ uint4 smem[];
@@ -135,12 +143,17 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
   int* exX = (int*)(red + 32);                 // [NCW][MP] row exponents by warp column: X',
   int* exY = exX + NCW * MP;                   // Y0,
   int* exQ = exY + NCW * MP;                   // Q
+  // of the propagator's warps: [24] planes (G', Q), [2][NMAIN NE] G', [2][MP] its row exponents
+  uint4* regC = (uint4*)(((size_t)(exQ + NCW * MP) + 15) & ~(size_t)15);
+  double2* gbuf = (double2*)(regC + 24 * PL);
+  int* eybuf = (int*)(gbuf + 2 * NMAIN * NE);
   __shared__ int s_r;
-  __shared__ volatile int s_status, s_abort[2];
+  __shared__ volatile int s_status, s_abort[2], s_gabort[2];
   __shared__ WgDesc wd;
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool main_thread = tid < NMAIN;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool main_thread = tid < NMAIN, prop_thread = PROP && tid >= NMAIN + kProd;
+  const int warp = (prop_thread ? tid - NMAIN - kProd : tid) >> 5;  // of a propagator warp: the main one it follows
   const int g = lane >> 2, t4 = lane & 3;
   const int tile = warp / NHALF, half = NHALF == 2 ? warp & 1 : 0;
   const int ti = tile / T, tj = tile % T;
@@ -148,7 +161,7 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
   double2* ws = a.work + (int64_t)blockIdx.x * a.work_stride;
   uint64_t* gen = (uint64_t*)ws;               // [max_ny][4]
   double* urow = (double*)(ws + 2 * (int64_t)a.max_ny);  // [max_ny] potential row
-  double2* Qs = ws + 2 * (int64_t)a.max_ny + (a.max_ny + 1) / 2 + (main_thread ? warp * 32 * NE + lane : 0);
+  double2* Qs = ws + 2 * (int64_t)a.max_ny + (a.max_ny + 1) / 2 + (main_thread || prop_thread ? warp * 32 * NE + lane : 0);
   double2* Gs = Qs + T * T * 256;              // entry k of this lane at [32 k]
   double2* Ww = Gs + T * T * 256;
   // This lane's place in the planes: its tile, and the word pairs of its tile
@@ -190,6 +203,82 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
 
     if (pass_on) {
       // handed to the pivoted kernel below
+    } else if (prop_thread) {
+      // Q, one slice behind the main warps, in this lane's registers.
+      double2 q[NE];
+      const char* bC = (const char*)regC;
+      const char* bD = (const char*)(regC + 12 * PL);
+      auto pbar = [&]() { bar_sync(kBarProp, NMAIN); };
+      for (int n = 0; n < nx && !refl; ++n) {
+        const int b = n & 1;
+        bar_sync(kBarGFull + b, 2 * NMAIN);
+        const bool skip = s_gabort[b] != 0;
+        double2 gd[NE];
+        int ec[NE];  // by column of an element
+        const int ey0 = eybuf[b * MP + r0], ey1 = eybuf[b * MP + r0 + 8];
+#pragma unroll
+        for (int k = 0; k < NE; ++k) {
+          gd[k] = gbuf[(b * (NMAIN / 32) + warp) * 32 * NE + 32 * k + lane];
+          ec[k] = eybuf[b * MP + c0 + ecol(k)];
+        }
+        if (n <= nx - 3) bar_arrive(kBarGFree + b, 2 * NMAIN);
+        if (skip) continue;
+        if (n > a.inject_at) {
+          int eq0 = oz::kNoExp, eq1 = oz::kNoExp;
+#pragma unroll
+          for (int k = 0; k < NE; ++k) {
+            if (erow(k)) eq1 = max(eq1, oz::fexp2(q[k]));
+            else eq0 = max(eq0, oz::fexp2(q[k]));
+          }
+          pbar();  // the last slice's planes and exponents have been read
+          oz::put_row_exps(exQ + (tj * NHALF + half) * MP, ti, lane, eq0, eq1);
+          long long acc[NV];
+#pragma unroll
+          for (int k = 0; k < NE; ++k) {
+            acc[k] = oz::sfixed53(gd[k].x, erow(k) ? ey1 : ey0);
+            acc[NE + k] = oz::sfixed53(gd[k].y, erow(k) ? ey1 : ey0);
+          }
+          oz::put_planes<53, NE>(acc, 6, regC + own, PL, 6, half);
+          pbar();
+          eq0 = oz::row_exp<NCW>(exQ, MP, r0);
+          eq1 = oz::row_exp<NCW>(exQ, MP, r0 + 8);
+#pragma unroll
+          for (int k = 0; k < NE; ++k) {
+            const int e = erow(k) ? eq1 : eq0;
+            acc[k] = oz::sfixed53(q[k].x, e);
+            acc[NE + k] = oz::sfixed53(q[k].y, e);
+          }
+          oz::put_planes<53, NE>(acc, 6, regC + 12 * PL + own, PL, 6, half);
+          pbar();
+#pragma unroll
+          for (int h = 0; h < NE / 4; ++h) {
+            long long hi[8], lo[8];
+            oz::half_product<T, 6, 6, oz::kLmax>(bD + offA0, bD + offA1, 6 * kPlane, bC + offB + 8 * (odd ^ (half | h)),
+                                                 6 * kPlane, kPlane, hi, lo);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+              const int k = 4 * h + w, e = (erow(k) ? eq1 : eq0) + ec[k];
+              q[k] = make_double2(-oz::fold_to_double(hi[w], lo[w], e), -oz::fold_to_double(hi[4 + w], lo[4 + w], e));
+            }
+          }
+        } else {
+          // the source slice: Q = G'; zero before it
+#pragma unroll
+          for (int k = 0; k < NE; ++k) q[k] = n == a.inject_at ? gd[k] : make_double2(0.0, 0.0);
+        }
+        if (a.state_dump) {
+          double2* d1 = a.state_dump + ((int64_t)r * nx + n) * 2 * M * M + (int64_t)M * M;
+#pragma unroll
+          for (int k = 0; k < NE; ++k) {
+            const int i = r0 + erow(k), j = c0 + ecol(k);
+            if (i < M && j < M) d1[(int64_t)j * M + i] = cmul(cmul(wd.wsc[i], wd.wsc[j]), q[k]);
+          }
+        }
+      }
+      if (!refl) {
+#pragma unroll
+        for (int k = 0; k < NE; ++k) Qs[32 * k] = q[k];
+      }
     } else if (!main_thread) {
       // Producers: the potential row of slice n and its projection
       // cc[d] = sum_j tab[j][d] U_j, one slice ahead.  The transverse grid
@@ -211,7 +300,7 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
       const double* tab = per ? (const double*)wd.expfac : wd.costab;  // [ny][nd]
       for (int n = 0; n < nx; ++n) {
         const int b = n & 1;
-        if (n >= 2) bar_sync(kBarFree + b, NT);
+        if (n >= 2) bar_sync(kBarFree + b, NMAIN + kProd);
         const int id = (refl ? nx - 1 - n : n) - wd.nxfree;
         if (id >= 0 && id < wd.nxdiso && !s_abort[b]) {
           for (int j = pt; j < ny; j += kProd) {
@@ -281,7 +370,7 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
           }
           bar_sync(kBarProd, kProd);  // urow is read before the next slice draws into it
         }
-        bar_arrive(kBarFull + b, NT);
+        bar_arrive(kBarFull + b, NMAIN + kProd);
       }
     } else {
       // Scaling products w_i w_j of this lane's elements.
@@ -298,7 +387,7 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
       bool aborted = false;
       for (int n = 0; n < nx; ++n) {
         const int b = n & 1;
-        bar_sync(kBarFull + b, NT);
+        bar_sync(kBarFull + b, NMAIN + kProd);
         double2 x[NE];
         if (!aborted) {
           // 1. X' = A/B - w V w - G' (zero outside M x M).
@@ -334,12 +423,20 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
         }
         if (n <= nx - 3) {
           if (tid == 0) s_abort[b] = aborted ? 1 : 0;
-          bar_arrive(kBarFree + b, NT);
+          bar_arrive(kBarFree + b, NMAIN + kProd);
         }
-        if (aborted) continue;
+        const bool hand_on = PROP && !refl;
+        if (aborted) {
+          if (hand_on) {
+            if (n >= 2) bar_sync(kBarGFree + b, 2 * NMAIN);
+            if (tid == 0) s_gabort[b] = 1;
+            bar_arrive(kBarGFull + b, 2 * NMAIN);
+          }
+          continue;
+        }
 
         // 2. G' = X'^-1 (rg_tile_inverse.cuh).
-        const bool prod = !refl && n > a.inject_at;
+        const bool prod = !PROP && !refl && n > a.inject_at;
         double2 q[NE], gd[NE];
         int ey0, ey1;
         auto q_exps = [&]() {  // Q, and its row exponents for the others
@@ -355,7 +452,23 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
         };
         if (!tile_inverse<T, NE>(x, M, tau, ts, &s_status, mbar, q_exps, gd, ey0, ey1)) {
           aborted = true;
+          if (hand_on) {
+            if (n >= 2) bar_sync(kBarGFree + b, 2 * NMAIN);
+            if (tid == 0) s_gabort[b] = 1;
+            bar_arrive(kBarGFull + b, 2 * NMAIN);
+          }
           continue;
+        }
+        if (hand_on) {
+          if (n >= 2) bar_sync(kBarGFree + b, 2 * NMAIN);
+#pragma unroll
+          for (int k = 0; k < NE; ++k) gbuf[(b * (NMAIN / 32) + warp) * 32 * NE + 32 * k + lane] = gd[k];
+          if (tj == 0 && half == 0 && t4 == 0) {
+            eybuf[b * MP + r0] = ey0;
+            eybuf[b * MP + r0 + 8] = ey1;
+          }
+          if (tid == 0) s_gabort[b] = 0;
+          bar_arrive(kBarGFull + b, 2 * NMAIN);
         }
 
         // 3. Q <- -Q G' on the tensor cores.
@@ -394,7 +507,7 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
               Qs[32 * k] = make_double2(-oz::fold_to_double(hi[w], lo[w], e), -oz::fold_to_double(hi[4 + w], lo[4 + w], e));
             }
           }
-        } else if (!refl) {
+        } else if (!PROP && !refl) {
           // the source slice: Q = G'; zero before it
 #pragma unroll
           for (int k = 0; k < NE; ++k) Qs[32 * k] = n == a.inject_at ? Gs[32 * k] : make_double2(0.0, 0.0);
@@ -408,7 +521,7 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
             const int i = r0 + erow(k), j = c0 + ecol(k);
             if (i < M && j < M) {
               d1[(int64_t)i * M + j] = cmul(Ww[32 * k], Gs[32 * k]);
-              d1[(int64_t)M * M + (int64_t)j * M + i] = cmul(Ww[32 * k], Qs[32 * k]);
+              if (!PROP) d1[(int64_t)M * M + (int64_t)j * M + i] = cmul(Ww[32 * k], Qs[32 * k]);
             }
           }
         }
@@ -493,12 +606,22 @@ __global__ void __launch_bounds__(SymCfg<T>::NT, SymCfg<T>::MINB) sweep_sym_kern
   }
 }
 
+// Whether Q gets warps of its own: while all realizations run at once with
+// them.  10 modes and 200 slices, batches of 1, 152, 200 and 304: 3.4, 3.9, 4.0
+// and 4.0 ms with, 4.9, 4.9, 5.0 and 5.0 without; 400 would need two waves for
+// 5.2 ms.  32 modes and 150 slices, 1 and 152: 5.1 and 5.2 against 6.6 ms.
 template <int T>
+bool prop_warps(const SweepArgs& a, int sm_count) {
+  return T == 1 ? a.nreal <= 2 * sm_count : T == 2 && a.nreal <= sm_count;
+}
+
+template <int T, bool PROP>
 int plan_sym_t(SweepArgs& a, int sm_count, int* grid, int64_t* stride) {
-  const size_t smem = SymCfg<T>::bytes();
-  RG_CUDA(allow_smem((const void*)sweep_sym_kernel<T>, smem));
+  const size_t smem = SymCfg<T, PROP>::bytes();
+  const auto kernel = sweep_sym_kernel<T, PROP>;
+  RG_CUDA(allow_smem((const void*)kernel, smem));
   int per_sm = 0;
-  RG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_sym_kernel<T>, SymCfg<T>::NT, smem));
+  RG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, SymCfg<T, PROP>::NT, smem));
   if (per_sm < 1) return fail(RG_ERR_INVALID_ARG, "symmetric sweep kernel does not fit on an SM");
   if (a.force_per_sm > 0 && a.force_per_sm < per_sm) per_sm = a.force_per_sm;
   int g = per_sm * sm_count;
@@ -506,12 +629,13 @@ int plan_sym_t(SweepArgs& a, int sm_count, int* grid, int64_t* stride) {
   *grid = g < 1 ? 1 : g;
   *stride = sym_stride(T, a.max_ny);
   a.cluster = 1;
+  a.prop_warps = PROP;
   return RG_OK;
 }
 
-template <int T>
+template <int T, bool PROP>
 int launch_sym_t(const SweepArgs& a, cudaStream_t stream, int grid) {
-  sweep_sym_kernel<T><<<grid, SymCfg<T>::NT, SymCfg<T>::bytes(), stream>>>(a);
+  sweep_sym_kernel<T, PROP><<<grid, SymCfg<T, PROP>::NT, SymCfg<T, PROP>::bytes(), stream>>>(a);
   RG_CUDA(cudaGetLastError());
   return RG_OK;
 }
@@ -519,19 +643,23 @@ int launch_sym_t(const SweepArgs& a, cudaStream_t stream, int grid) {
 }  // namespace
 
 int sweep_sym_plan(SweepArgs& a, int sm_count, int* grid, int64_t* work_stride) {
-  if (a.max_M <= 16) return plan_sym_t<1>(a, sm_count, grid, work_stride);
-  if (a.max_M <= 32) return plan_sym_t<2>(a, sm_count, grid, work_stride);
-  if (a.max_M <= 48) return plan_sym_t<3>(a, sm_count, grid, work_stride);
-  if (a.max_M <= kMaxModesSmem) return plan_sym_t<4>(a, sm_count, grid, work_stride);
+  if (a.max_M <= 16)
+    return prop_warps<1>(a, sm_count) ? plan_sym_t<1, true>(a, sm_count, grid, work_stride)
+                                      : plan_sym_t<1, false>(a, sm_count, grid, work_stride);
+  if (a.max_M <= 32)
+    return prop_warps<2>(a, sm_count) ? plan_sym_t<2, true>(a, sm_count, grid, work_stride)
+                                      : plan_sym_t<2, false>(a, sm_count, grid, work_stride);
+  if (a.max_M <= 48) return plan_sym_t<3, false>(a, sm_count, grid, work_stride);
+  if (a.max_M <= kMaxModesSmem) return plan_sym_t<4, false>(a, sm_count, grid, work_stride);
   return fail(RG_ERR_INVALID_ARG, "symmetric sweep kernel: too many modes");
 }
 
 int launch_sweep_sym(const SweepArgs& a, cudaStream_t stream, int grid) {
   if (a.nreal <= 0) return RG_OK;
-  if (a.max_M <= 16) return launch_sym_t<1>(a, stream, grid);
-  if (a.max_M <= 32) return launch_sym_t<2>(a, stream, grid);
-  if (a.max_M <= 48) return launch_sym_t<3>(a, stream, grid);
-  return launch_sym_t<4>(a, stream, grid);
+  if (a.max_M <= 16) return a.prop_warps ? launch_sym_t<1, true>(a, stream, grid) : launch_sym_t<1, false>(a, stream, grid);
+  if (a.max_M <= 32) return a.prop_warps ? launch_sym_t<2, true>(a, stream, grid) : launch_sym_t<2, false>(a, stream, grid);
+  if (a.max_M <= 48) return launch_sym_t<3, false>(a, stream, grid);
+  return launch_sym_t<4, false>(a, stream, grid);
 }
 
 }  // namespace rg
