@@ -415,16 +415,17 @@ __device__ __forceinline__ void put_words(const uint32_t* w, uint4* d, int s, in
 // np..np+n-1, `plane` uint4 apart.  The values are signed fixed point of BITS
 // bits after a right shift by sh (a left shift when negative).  The words of
 // a digit that gets no plane (n = D - 1) go to `last`, when given.
-template <int BITS, int NE>
+// With NP = 2 the lane has only the NE values of part `part0` (0 re, 1 im).
+template <int BITS, int NE, int NP = 1>
 __device__ __forceinline__ void put_planes(const long long* x, int n, uint4* dst, int plane, int np, int half,
-                                           int sh = 0, uint32_t* last = nullptr) {
+                                           int sh = 0, uint32_t* last = nullptr, int part0 = 0) {
   constexpr int D = (BITS - 8) / kDigitBits + 1;  // digits of the format
   const int s = (threadIdx.x >> 3) & 1;           // odd octet: pairs swapped
   long long bias = 0;
 #pragma unroll
   for (int p = 0; p < D; ++p) bias += 256LL << (kDigitBits * p);
 #pragma unroll
-  for (int part = 0; part < 2; ++part) {
+  for (int part = 0; part < 2 / NP; ++part) {
     unsigned long long y[NE];
 #pragma unroll
     for (int k = 0; k < NE; ++k) {
@@ -442,7 +443,7 @@ __device__ __forceinline__ void put_planes(const long long* x, int n, uint4* dst
                             (uint32_t)(y[2 * k + 1] >> (kDigitBits * (D - 1 - p))) & mask);
         }
         if (p < n) {
-          put_words<NE>(w, dst + (part * np + p) * plane, s, half);
+          put_words<NE>(w, dst + ((NP == 2 ? part0 : part) * np + p) * plane, s, half);
         } else {
 #pragma unroll
           for (int k = 0; k < NE / 2; ++k) last[part * (NE / 2) + k] = w[k];
@@ -497,11 +498,14 @@ __device__ __forceinline__ double fold_to_double(long long hi, long long lo, int
 // the sums of two k tiles stay within 2^24, and are folded together.
 // A seventh digit of B (NB = 7) has its real plane at b6 and its imaginary
 // plane after it.
-template <int T, int NA, int NB, int LMAX>
+template <int T, int NA, int NB, int LMAX, int NP = 1>
 __device__ __forceinline__ void half_product(const char* a0, const char* a1, int SA, const char* b, int SB, int plane,
-                                             long long* hi, long long* lo, const char* b6 = nullptr) {
+                                             long long* hi, long long* lo, const char* b6 = nullptr, int part = 0) {
+  constexpr int NV = 8 / NP;  // sums of a lane
+  // NP = 2, by part: A_re meets B_re or B_im, A_im meets -B_im or B_re
+  const uint32_t neg = NP == 2 && part ? 0u : 0x80008000u;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) hi[k] = lo[k] = 0;
+  for (int k = 0; k < NV; ++k) hi[k] = lo[k] = 0;
 #pragma unroll
   for (int L = 0; L <= LMAX; L += 3) {
     const int top = L + 2 < LMAX ? L + 2 : LMAX;
@@ -517,11 +521,11 @@ __device__ __forceinline__ void half_product(const char* a0, const char* a1, int
     const int KF = np <= 4 && T > 1 ? 2 : 1;  // k tiles per fold
 #pragma unroll 1
     for (int tk0 = 0; tk0 < T; tk0 += KF) {
-      float acc[3][8];
+      float acc[3][NV];
 #pragma unroll
       for (int v = 0; v < 3; ++v)
 #pragma unroll
-        for (int w = 0; w < 8; ++w) acc[v][w] = 0.0f;
+        for (int w = 0; w < NV; ++w) acc[v][w] = 0.0f;
 #pragma unroll 1
       for (int tk = tk0; tk < tk0 + KF && tk < T; ++tk) {
         const char* pa0 = a0 + tk * 512;
@@ -532,14 +536,15 @@ __device__ __forceinline__ void half_product(const char* a0, const char* a1, int
         for (int q = 0; q < NB; ++q)  // the digits the first A digit meets
           if (q >= L && q <= top) {
             const char* pq = q == 6 ? b6 + tk * 512 : pb + q * plane;
-            br[q % 3] = *reinterpret_cast<const uint2*>(pq);
-            bi[q % 3] = *reinterpret_cast<const uint2*>(pq + (q == 6 ? plane : SB));
+            const int im = q == 6 ? plane : SB;
+            br[q % 3] = *reinterpret_cast<const uint2*>(pq + (NP == 2 && part ? im : 0));
+            bi[q % 3] = *reinterpret_cast<const uint2*>(pq + (NP == 2 && part ? 0 : im));
           }
 #pragma unroll
         for (int p = 0; p < NA; ++p) {
           if (p > 0 && L - p >= 0 && L - p < NB) {
-            br[(L - p) % 3] = *reinterpret_cast<const uint2*>(pb + (L - p) * plane);
-            bi[(L - p) % 3] = *reinterpret_cast<const uint2*>(pb + SB + (L - p) * plane);
+            br[(L - p) % 3] = *reinterpret_cast<const uint2*>(pb + (NP == 2 && part ? SB : 0) + (L - p) * plane);
+            bi[(L - p) % 3] = *reinterpret_cast<const uint2*>(pb + (NP == 2 && part ? 0 : SB) + (L - p) * plane);
           }
           if (top - p >= 0 && L - p < NB) {
             const uint2 r0 = *reinterpret_cast<const uint2*>(pa0 + p * plane);
@@ -552,15 +557,15 @@ __device__ __forceinline__ void half_product(const char* a0, const char* a1, int
               const int q = L + v - p;
               if (q >= 0 && q < NB && L + v <= LMAX) {
                 mma16816(acc[v], ar, br[q % 3].x, br[q % 3].y);
-                mma16816(acc[v] + 4, ar, bi[q % 3].x, bi[q % 3].y);
+                if (NP == 1) mma16816(acc[v] + 4 % NV, ar, bi[q % 3].x, bi[q % 3].y);
               }
             }
 #pragma unroll
             for (int v = 0; v < 3; ++v) {
               const int q = L + v - p;
               if (q >= 0 && q < NB && L + v <= LMAX) {
-                mma16816(acc[v], ai, bi[q % 3].x ^ 0x80008000u, bi[q % 3].y ^ 0x80008000u);
-                mma16816(acc[v] + 4, ai, br[q % 3].x, br[q % 3].y);
+                mma16816(acc[v], ai, bi[q % 3].x ^ neg, bi[q % 3].y ^ neg);
+                if (NP == 1) mma16816(acc[v] + 4 % NV, ai, br[q % 3].x, br[q % 3].y);
               }
             }
           }
@@ -570,7 +575,7 @@ __device__ __forceinline__ void half_product(const char* a0, const char* a1, int
       for (int v = 0; v < 3; ++v)
         if (L + v <= LMAX) {
 #pragma unroll
-          for (int w = 0; w < 8; ++w) {
+          for (int w = 0; w < NV; ++w) {
             const int x = __float2int_rn(acc[v][w]);
             if (L + v < kHiLevels) hi[w] += (long long)x * (1LL << (kDigitBits * (kHiLevels - 1 - L - v)));
             else lo[w] += (long long)x * (1LL << (kDigitBits * (kLmax - L - v)));

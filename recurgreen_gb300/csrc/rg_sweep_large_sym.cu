@@ -430,11 +430,13 @@ __device__ __noinline__ bool leaf_inverse(double2* P, const int n, const float t
   ts.exX = reinterpret_cast<int*>(ts.red + 32);
   ts.exY = ts.exX + NCW * MP;
   __shared__ int s_flag;
-  double2 x[NE], gd[NE];
+  double x[2 * NE], gd[2 * NE];
 #pragma unroll
   for (int k = 0; k < NE; ++k) {
     const int i = r0 + erow(k), j = c0 + ecol(k);
-    x[k] = i < n && j < n ? __ldcg(P + (i <= j ? i * n + j : j * n + i)) : make_double2(0.0, 0.0);
+    const double2 v = i < n && j < n ? __ldcg(P + (i <= j ? i * n + j : j * n + i)) : make_double2(0.0, 0.0);
+    x[k] = v.x;
+    x[NE + k] = v.y;
   }
   if (tid == 0) s_flag = RG_OK;
   __syncthreads();  // the staging area's previous contents have been used
@@ -445,7 +447,7 @@ __device__ __noinline__ bool leaf_inverse(double2* P, const int n, const float t
 #pragma unroll
     for (int k = 0; k < NE; ++k) {
       const int i = r0 + erow(k), j = c0 + ecol(k);
-      if (i <= j && j < n) P[i * n + j] = gd[k];
+      if (i <= j && j < n) P[i * n + j] = make_double2(gd[k], gd[NE + k]);
     }
   }
   if (cluster.num_blocks() > 1) cluster.sync();

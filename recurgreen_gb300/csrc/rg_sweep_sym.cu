@@ -30,7 +30,7 @@
 // within 0.95 to 1.3 (7 to 64 modes, 40 to 300 slices; geometric mean 1.08).
 // Measured, with the eigenvalues: 304 guides of 64 modes and 600 slices 607 ms
 // before, 184 now; 500 of 37 modes and 150 slices 110 ms before, 41 now; one
-// guide of 10 modes and 200 slices 8.2 ms before, 3.4 now.
+// guide of 10 modes and 200 slices 8.2 ms before, 2.1 now.
 //
 // Layout: T = ceil(M/16) tiles a side, one warp per tile or two, as in
 // rg_tile_inverse.cuh.  (Q is kept transposed so that it is only ever an A
@@ -96,29 +96,33 @@ __device__ __forceinline__ double2 from_real_modes(const double2* F, int ld, int
   return cscale(0.70710678118654752440, make_double2(c.x - f * s.y, c.y + f * s.x));
 }
 
-// PROP: Q has warps of its own, as many as the main ones, one slice behind
-// them.  Q_n does not feed the recursion of G', so a slice's chain is then the
-// inverse alone.  They cost registers and shared memory, so the CTAs per SM
-// fall from 4 to 2 (up to 16 modes) and from 2 to 1 (up to 32): taken while
-// every realization has its CTA at once (prop_warps).
+// PROP: Q has warps of its own, as many as hold the matrix, one slice behind
+// the main ones.  Q_n does not feed the recursion of G', so a slice's chain is
+// then the inverse alone.  They cost registers and shared memory: at 17 to 32
+// modes an SM takes one such CTA instead of two (prop_warps).
 template <int T, bool PROP>
 struct SymCfg {
   static constexpr int MP = 16 * T;                // padded modes
   static constexpr int NE = T == 4 ? 8 : 4;        // complex entries per lane: a whole tile, or its column half
   static constexpr int NHALF = 8 / NE;             // warps per tile
-  static constexpr int NCW = T * NHALF;            // warps that share a row
-  static constexpr int NMAIN = 32 * T * T * NHALF;
+  // 2: a main warp has one part, re or im, of its entries.  Up to 16 modes, where
+  // the instructions of two warps made a slice's latency: one guide of 10 modes
+  // and 200 slices 4.85 ms, 3.43 with PROP, 2.07 with both; 600 guides 5.7 ms in
+  // any of the forms.
+  static constexpr int NP = T == 1 && PROP ? 2 : 1;
+  static constexpr int NCW = T * NHALF;            // warps that share a row (main: NP times as many)
+  static constexpr int NPROP = 32 * T * T * NHALF;  // threads that hold Q; without PROP the main ones
+  static constexpr int NMAIN = NP * NPROP;
   // Producer threads.  Registers are handed out to four warps at a time.
   static constexpr int PROD = T == 4 ? 128 : 64;
-  static constexpr int NPROP = PROP ? NMAIN : 0;
-  static constexpr int NT = NMAIN + PROD + NPROP;
-  static constexpr int MINB = T == 1 ? (PROP ? 2 : 4) : T == 2 && !PROP ? 2 : 1;  // CTAs per SM
+  static constexpr int NT = NMAIN + PROD + (PROP ? NPROP : 0);
+  static constexpr int MINB = T == 1 || (T == 2 && !PROP) ? 2 : 1;  // CTAs per SM
   static constexpr int PL = T * T * 32;            // uint4 of one digit plane
   static constexpr int LDW = MP + 1;
   static constexpr size_t bytes() {
     return sizeof(uint4) * 24 * PL + sizeof(double) * (2 * (2 * MP + 2) + PROD) + sizeof(unsigned long long) * 2 +
-           sizeof(unsigned) * 32 + sizeof(int) * 3 * NCW * MP +
-           (PROP ? sizeof(uint4) * 24 * PL + sizeof(double2) * 2 * NMAIN * NE + sizeof(int) * 2 * MP : 0);
+           sizeof(unsigned) * 32 + sizeof(int) * (2 * NP + 1) * NCW * MP +
+           (PROP ? sizeof(uint4) * 24 * PL + sizeof(double2) * 2 * NPROP * NE + sizeof(int) * 2 * MP : 0);
   }
 };
 
@@ -132,28 +136,30 @@ template <int T, bool PROP>
 __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sweep_sym_kernel(SweepArgs a) {
   using Cf = SymCfg<T, PROP>;
   constexpr int MP = Cf::MP, NMAIN = Cf::NMAIN, NT = Cf::NT, PL = Cf::PL, LDW = Cf::LDW, kProd = Cf::PROD;
-  constexpr int NE = Cf::NE, NV = 2 * NE, NHALF = Cf::NHALF, NCW = Cf::NCW;
+  constexpr int NE = Cf::NE, NHALF = Cf::NHALF, NCW = Cf::NCW, NP = Cf::NP, NPROP = Cf::NPROP, NV = 2 * NE / NP;
   extern __shared__ uint4 smem[];
   uint4* regA = smem;                          // 12 planes
   uint4* regB = smem + 12 * PL;                // 12 planes
   double* cc = (double*)(smem + 24 * PL);      // [2][2 MP + 2] projection coefficients
-  double* part = cc + 2 * (2 * MP + 2);        // [kProd] partial projections
-  unsigned long long* rsum = (unsigned long long*)(part + kProd);  // [2] sum of squares of the residual
+  double* psum = cc + 2 * (2 * MP + 2);        // [kProd] partial projections
+  unsigned long long* rsum = (unsigned long long*)(psum + kProd);  // [2] sum of squares of the residual
   unsigned* red = (unsigned*)(rsum + 2);       // [32] maxima of a slice
   int* exX = (int*)(red + 32);                 // [NCW][MP] row exponents by warp column: X',
-  int* exY = exX + NCW * MP;                   // Y0,
-  int* exQ = exY + NCW * MP;                   // Q
-  // of the propagator's warps: [24] planes (G', Q), [2][NMAIN NE] G', [2][MP] its row exponents
+  int* exY = exX + NP * NCW * MP;              // Y0,
+  int* exQ = exY + NP * NCW * MP;              // Q
+  // of the propagator's warps: [24] planes (G', Q), [2][NPROP NE] G', [2][MP] its row exponents
   uint4* regC = (uint4*)(((size_t)(exQ + NCW * MP) + 15) & ~(size_t)15);
   double2* gbuf = (double2*)(regC + 24 * PL);
-  int* eybuf = (int*)(gbuf + 2 * NMAIN * NE);
+  int* eybuf = (int*)(gbuf + 2 * NPROP * NE);
   __shared__ int s_r;
   __shared__ volatile int s_status, s_abort[2], s_gabort[2];
   __shared__ WgDesc wd;
 
   const int tid = threadIdx.x, lane = tid & 31;
   const bool main_thread = tid < NMAIN, prop_thread = PROP && tid >= NMAIN + kProd;
-  const int warp = (prop_thread ? tid - NMAIN - kProd : tid) >> 5;  // of a propagator warp: the main one it follows
+  const bool out_thread = PROP ? prop_thread : main_thread;  // has whole elements of the results
+  const int part = NP == 2 && main_thread ? (tid >> 5) & 1 : 0;
+  const int warp = prop_thread ? (tid - NMAIN - kProd) >> 5 : (tid >> 5) / NP;
   const int g = lane >> 2, t4 = lane & 3;
   const int tile = warp / NHALF, half = NHALF == 2 ? warp & 1 : 0;
   const int ti = tile / T, tj = tile % T;
@@ -208,20 +214,20 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
       double2 q[NE];
       const char* bC = (const char*)regC;
       const char* bD = (const char*)(regC + 12 * PL);
-      auto pbar = [&]() { bar_sync(kBarProp, NMAIN); };
+      auto pbar = [&]() { bar_sync(kBarProp, NPROP); };
       for (int n = 0; n < nx && !refl; ++n) {
         const int b = n & 1;
-        bar_sync(kBarGFull + b, 2 * NMAIN);
+        bar_sync(kBarGFull + b, NMAIN + NPROP);
         const bool skip = s_gabort[b] != 0;
         double2 gd[NE];
         int ec[NE];  // by column of an element
         const int ey0 = eybuf[b * MP + r0], ey1 = eybuf[b * MP + r0 + 8];
 #pragma unroll
         for (int k = 0; k < NE; ++k) {
-          gd[k] = gbuf[(b * (NMAIN / 32) + warp) * 32 * NE + 32 * k + lane];
+          gd[k] = gbuf[(b * (NPROP / 32) + warp) * 32 * NE + 32 * k + lane];
           ec[k] = eybuf[b * MP + c0 + ecol(k)];
         }
-        if (n <= nx - 3) bar_arrive(kBarGFree + b, 2 * NMAIN);
+        if (n <= nx - 3) bar_arrive(kBarGFree + b, NMAIN + NPROP);
         if (skip) continue;
         if (n > a.inject_at) {
           int eq0 = oz::kNoExp, eq1 = oz::kNoExp;
@@ -232,7 +238,7 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
           }
           pbar();  // the last slice's planes and exponents have been read
           oz::put_row_exps(exQ + (tj * NHALF + half) * MP, ti, lane, eq0, eq1);
-          long long acc[NV];
+          long long acc[2 * NE];
 #pragma unroll
           for (int k = 0; k < NE; ++k) {
             acc[k] = oz::sfixed53(gd[k].x, erow(k) ? ey1 : ey0);
@@ -267,11 +273,16 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
           for (int k = 0; k < NE; ++k) q[k] = n == a.inject_at ? gd[k] : make_double2(0.0, 0.0);
         }
         if (a.state_dump) {
-          double2* d1 = a.state_dump + ((int64_t)r * nx + n) * 2 * M * M + (int64_t)M * M;
+          // as below: Gss = w G' w and Gs1 = w Q^T w
+          double2* d1 = a.state_dump + ((int64_t)r * nx + n) * 2 * M * M;
 #pragma unroll
           for (int k = 0; k < NE; ++k) {
             const int i = r0 + erow(k), j = c0 + ecol(k);
-            if (i < M && j < M) d1[(int64_t)j * M + i] = cmul(cmul(wd.wsc[i], wd.wsc[j]), q[k]);
+            if (i < M && j < M) {
+              const double2 w = cmul(wd.wsc[i], wd.wsc[j]);
+              d1[(int64_t)i * M + j] = cmul(w, gd[k]);
+              d1[(int64_t)M * M + (int64_t)j * M + i] = cmul(w, q[k]);
+            }
           }
         }
       }
@@ -342,11 +353,11 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
           };
           if (kProd > 32 && 2 * nd <= kProd) {  // several threads share a coefficient
             const int nseg = kProd / nd, seg = pt / nd, d = pt % nd;
-            if (seg < nseg) part[pt] = dot(d, seg * h / nseg, (seg + 1) * h / nseg, seg == nseg - 1);
+            if (seg < nseg) psum[pt] = dot(d, seg * h / nseg, (seg + 1) * h / nseg, seg == nseg - 1);
             bar_sync(kBarProd, kProd);
             if (pt < nd) {
-              double s = part[pt];
-              for (int k = 1; k < nseg; ++k) s += part[k * nd + pt];
+              double s = psum[pt];
+              for (int k = 1; k < nseg; ++k) s += psum[k * nd + pt];
               co[pt] = s;
             }
           } else {
@@ -380,45 +391,41 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
         const int i = r0 + erow(k), j = c0 + ecol(k);
         double2 v = make_double2(0.0, 0.0);
         if (i < M && j < M) v = cmul(wd.wsc[i], wd.wsc[j]);
-        Ww[32 * k] = v;
+        if (part == 0) Ww[32 * k] = v;
         real_w = real_w && v.y == 0.0;
       }
       real_w = __all_sync(0xffffffffu, real_w);
+      double* gp = reinterpret_cast<double*>(Gs) + part;  // value q of this lane: part of element q mod NE
+      const double* wp = reinterpret_cast<const double*>(Ww) + part;
+      mbar();  // Ww is complete
       bool aborted = false;
       for (int n = 0; n < nx; ++n) {
         const int b = n & 1;
         bar_sync(kBarFull + b, NMAIN + kProd);
-        double2 x[NE];
+        double x[NV];
         if (!aborted) {
           // 1. X' = A/B - w V w - G' (zero outside M x M).
           const int id = (refl ? nx - 1 - n : n) - wd.nxfree;
           const bool dis = (id >= 0 && id < wd.nxdiso), edge = (n == 0 || n == nx - 1);
           const double* co = cc + b * (2 * MP + 2);
+          const double* aw = (const double*)(edge ? wd.aw_edge : wd.aw_bulk);
 #pragma unroll
           for (int k = 0; k < NE; ++k) {
             const int i = r0 + erow(k), j = c0 + ecol(k);
-            double2 v = make_double2(0.0, 0.0);
-            if (i < M && j < M) {
-              if (n > 0) {
-                v = Gs[32 * k];
-                v = make_double2(-v.x, -v.y);
+            const bool on = i < M && j < M;
+            const double vij = on && dis ? potential_element(co, i, j, M, per) : 0.0;
+#pragma unroll
+            for (int q = k; q < NV; q += NE) {
+              const int p = q < NE ? part : 1;  // this value's part
+              double v = 0.0;
+              if (on) {
+                if (n > 0) v = -gp[64 * k + (q < NE ? 0 : 1)];
+                if (i == j) v += aw[2 * i + p];
+                if (dis && (p == 0 || !real_w)) v = fma(-wp[64 * k + (q < NE ? 0 : 1)], vij, v);
+                if (i == j) v += aw[2 * (M + i) + p];  // the rest of A/B beyond FP64
               }
-              if (i == j) {
-                const double2 d = edge ? wd.aw_edge[i] : wd.aw_bulk[i];
-                v = make_double2(v.x + d.x, v.y + d.y);
-              }
-              if (dis) {
-                const double vij = potential_element(co, i, j, M, per);
-                const double2 w = Ww[32 * k];
-                v.x = fma(-w.x, vij, v.x);
-                if (!real_w) v.y = fma(-w.y, vij, v.y);
-              }
-              if (i == j) {  // the rest of A/B beyond FP64
-                const double2 d = edge ? wd.aw_edge[M + i] : wd.aw_bulk[M + i];
-                v = make_double2(v.x + d.x, v.y + d.y);
-              }
+              x[q] = v;
             }
-            x[k] = v;
           }
         }
         if (n <= nx - 3) {
@@ -428,16 +435,17 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
         const bool hand_on = PROP && !refl;
         if (aborted) {
           if (hand_on) {
-            if (n >= 2) bar_sync(kBarGFree + b, 2 * NMAIN);
+            if (n >= 2) bar_sync(kBarGFree + b, NMAIN + NPROP);
             if (tid == 0) s_gabort[b] = 1;
-            bar_arrive(kBarGFull + b, 2 * NMAIN);
+            bar_arrive(kBarGFull + b, NMAIN + NPROP);
           }
           continue;
         }
 
         // 2. G' = X'^-1 (rg_tile_inverse.cuh).
         const bool prod = !PROP && !refl && n > a.inject_at;
-        double2 q[NE], gd[NE];
+        double2 q[NE];
+        double gd[NV];
         int ey0, ey1;
         auto q_exps = [&]() {  // Q, and its row exponents for the others
           if (!prod) return;
@@ -450,36 +458,35 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
           }
           oz::put_row_exps(exQ + (tj * NHALF + half) * MP, ti, lane, eq0, eq1);
         };
-        if (!tile_inverse<T, NE>(x, M, tau, ts, &s_status, mbar, q_exps, gd, ey0, ey1)) {
+        if (!tile_inverse<T, NE, NP>(x, M, tau, ts, &s_status, mbar, q_exps, gd, ey0, ey1)) {
           aborted = true;
           if (hand_on) {
-            if (n >= 2) bar_sync(kBarGFree + b, 2 * NMAIN);
+            if (n >= 2) bar_sync(kBarGFree + b, NMAIN + NPROP);
             if (tid == 0) s_gabort[b] = 1;
-            bar_arrive(kBarGFull + b, 2 * NMAIN);
+            bar_arrive(kBarGFull + b, NMAIN + NPROP);
           }
           continue;
         }
         if (hand_on) {
-          if (n >= 2) bar_sync(kBarGFree + b, 2 * NMAIN);
+          if (n >= 2) bar_sync(kBarGFree + b, NMAIN + NPROP);
 #pragma unroll
-          for (int k = 0; k < NE; ++k) gbuf[(b * (NMAIN / 32) + warp) * 32 * NE + 32 * k + lane] = gd[k];
-          if (tj == 0 && half == 0 && t4 == 0) {
+          for (int k = 0; k < NV; ++k)
+            reinterpret_cast<double*>(gbuf + (b * (NPROP / 32) + warp) * 32 * NE + 32 * (k % NE) + lane)[k < NE ? part : 1] =
+                gd[k];
+          if (tj == 0 && half == 0 && part == 0 && t4 == 0) {
             eybuf[b * MP + r0] = ey0;
             eybuf[b * MP + r0 + 8] = ey1;
           }
           if (tid == 0) s_gabort[b] = 0;
-          bar_arrive(kBarGFull + b, 2 * NMAIN);
+          bar_arrive(kBarGFull + b, NMAIN + NPROP);
         }
 
         // 3. Q <- -Q G' on the tensor cores.
-        long long acc[NV];
+        long long acc[2 * NE];
 #pragma unroll
-        for (int k = 0; k < NE; ++k) {
-          Gs[32 * k] = gd[k];
-          if (prod) {
-            acc[k] = oz::sfixed53(gd[k].x, erow(k) ? ey1 : ey0);
-            acc[NE + k] = oz::sfixed53(gd[k].y, erow(k) ? ey1 : ey0);
-          }
+        for (int k = 0; k < NV; ++k) {
+          gp[64 * (k % NE) + k / NE] = gd[k];
+          if (prod) acc[k] = oz::sfixed53(gd[k], erow(k % NE) ? ey1 : ey0);
         }
         if (prod) {
           oz::put_planes<53, NE>(acc, 6, regA + own, PL, 6, half);
@@ -512,7 +519,7 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
 #pragma unroll
           for (int k = 0; k < NE; ++k) Qs[32 * k] = n == a.inject_at ? Gs[32 * k] : make_double2(0.0, 0.0);
         }
-        if (a.state_dump) {
+        if (a.state_dump && !hand_on) {
           // The state after this slice, natural order: Gss = w G' w and
           // Gs1 = w Q^T w, the solve_block_tridiag pair (S_n, Z_n).
           double2* d1 = a.state_dump + ((int64_t)r * nx + n) * 2 * M * M;
@@ -521,7 +528,7 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
             const int i = r0 + erow(k), j = c0 + ecol(k);
             if (i < M && j < M) {
               d1[(int64_t)i * M + j] = cmul(Ww[32 * k], Gs[32 * k]);
-              if (!PROP) d1[(int64_t)M * M + (int64_t)j * M + i] = cmul(Ww[32 * k], Qs[32 * k]);
+              d1[(int64_t)M * M + (int64_t)j * M + i] = cmul(Ww[32 * k], Qs[32 * k]);
             }
           }
         }
@@ -544,13 +551,13 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
       double2* rout = a.tout + (int64_t)r * M * M;
       double2* F = (double2*)regB;  // [MP][LDW] periodic: G11 in the real modes
       if (per) {
-        if (main_thread) {
+        if (out_thread) {
 #pragma unroll
           for (int k = 0; k < NE; ++k) F[(r0 + erow(k)) * LDW + c0 + ecol(k)] = cmul(Ww[32 * k], Gs[32 * k]);
         }
         __syncthreads();
       }
-      if (main_thread) {
+      if (out_thread) {
 #pragma unroll
         for (int k = 0; k < NE; ++k) {
           const int i = r0 + erow(k), j = c0 + ecol(k);
@@ -575,13 +582,13 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
     double2* tout = a.tout ? a.tout + (int64_t)r * nrow * ncol : nullptr;
     double2* F = (double2*)regB;  // [MP][LDW] periodic: Gs1 in the real modes
     if (per) {
-      if (main_thread) {
+      if (out_thread) {
 #pragma unroll
         for (int k = 0; k < NE; ++k) F[(c0 + ecol(k)) * LDW + r0 + erow(k)] = cmul(Ww[32 * k], Qs[32 * k]);
       }
       __syncthreads();
     }
-    if (main_thread) {
+    if (out_thread) {
 #pragma unroll
       for (int k = 0; k < NE; ++k) {
         const int gj = r0 + erow(k), gi = c0 + ecol(k);  // Q[j][i]
@@ -606,14 +613,10 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
   }
 }
 
-// Whether Q gets warps of its own: while all realizations run at once with
-// them.  10 modes and 200 slices, batches of 1, 152, 200 and 304: 3.4, 3.9, 4.0
-// and 4.0 ms with, 4.9, 4.9, 5.0 and 5.0 without; 400 would need two waves for
-// 5.2 ms.  32 modes and 150 slices, 1 and 152: 5.1 and 5.2 against 6.6 ms.
-template <int T>
-bool prop_warps(const SweepArgs& a, int sm_count) {
-  return T == 1 ? a.nreal <= 2 * sm_count : T == 2 && a.nreal <= sm_count;
-}
+// Whether Q gets warps of its own at 17 to 32 modes: while all realizations run
+// at once with them.  32 modes and 150 slices, batches of 1 and 152: 5.1 and 5.2
+// ms with, 6.6 without; 200 would need two waves for 7.9 ms.
+bool prop_warps(const SweepArgs& a, int sm_count) { return a.nreal <= sm_count; }
 
 template <int T, bool PROP>
 int plan_sym_t(SweepArgs& a, int sm_count, int* grid, int64_t* stride) {
@@ -643,12 +646,10 @@ int launch_sym_t(const SweepArgs& a, cudaStream_t stream, int grid) {
 }  // namespace
 
 int sweep_sym_plan(SweepArgs& a, int sm_count, int* grid, int64_t* work_stride) {
-  if (a.max_M <= 16)
-    return prop_warps<1>(a, sm_count) ? plan_sym_t<1, true>(a, sm_count, grid, work_stride)
-                                      : plan_sym_t<1, false>(a, sm_count, grid, work_stride);
+  if (a.max_M <= 16) return plan_sym_t<1, true>(a, sm_count, grid, work_stride);
   if (a.max_M <= 32)
-    return prop_warps<2>(a, sm_count) ? plan_sym_t<2, true>(a, sm_count, grid, work_stride)
-                                      : plan_sym_t<2, false>(a, sm_count, grid, work_stride);
+    return prop_warps(a, sm_count) ? plan_sym_t<2, true>(a, sm_count, grid, work_stride)
+                                   : plan_sym_t<2, false>(a, sm_count, grid, work_stride);
   if (a.max_M <= 48) return plan_sym_t<3, false>(a, sm_count, grid, work_stride);
   if (a.max_M <= kMaxModesSmem) return plan_sym_t<4, false>(a, sm_count, grid, work_stride);
   return fail(RG_ERR_INVALID_ARG, "symmetric sweep kernel: too many modes");
@@ -656,7 +657,7 @@ int sweep_sym_plan(SweepArgs& a, int sm_count, int* grid, int64_t* work_stride) 
 
 int launch_sweep_sym(const SweepArgs& a, cudaStream_t stream, int grid) {
   if (a.nreal <= 0) return RG_OK;
-  if (a.max_M <= 16) return a.prop_warps ? launch_sym_t<1, true>(a, stream, grid) : launch_sym_t<1, false>(a, stream, grid);
+  if (a.max_M <= 16) return launch_sym_t<1, true>(a, stream, grid);
   if (a.max_M <= 32) return a.prop_warps ? launch_sym_t<2, true>(a, stream, grid) : launch_sym_t<2, false>(a, stream, grid);
   if (a.max_M <= 48) return launch_sym_t<3, false>(a, stream, grid);
   return launch_sym_t<4, false>(a, stream, grid);

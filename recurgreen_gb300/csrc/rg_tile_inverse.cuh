@@ -187,18 +187,22 @@ struct TileSmem {
 };
 
 // x: this lane's entries of X (zero outside M x M), NE = 8 of a whole tile or
-// 4 of its column half; gd: its entries of X^-1, exactly symmetric; ey0, ey1:
-// the exponents of rows g and g + 8 (|gd| < 2^(ey+1)).  Called by the T^2 8/NE
-// warps 0, 1, ... of the CTA; bar() is a barrier of theirs, and pre() is run
+// 4 of its column half, real parts, then imaginary parts; gd: its entries of
+// X^-1, exactly symmetric; ey0, ey1: the exponents of rows g and g + 8 (|gd| <
+// 2^(ey+1)).  With NP = 2 (T = 1) a lane has one part of its entries, real in
+// even warps and imaginary in odd ones: half the instructions in each of twice
+// the warps.  Called by the T^2 8/NE NP warps 0, 1, ... of the CTA; bar() is a barrier of theirs, and pre() is run
 // before the last but one.  Returns false, in every thread, when a pivot falls
 // below tau times the largest unswept entry of its row (in its tile) or the
 // residual is not small; *flag (shared, zero before, kStatusNeedPivot after)
 // says so too.
-template <int T, int NE, class Bar, class Pre>
-__device__ __forceinline__ bool tile_inverse(const double2* x, const int M, const float tau, const TileSmem& s,
-                                             volatile int* flag, Bar bar, Pre pre, double2* gd, int& ey0, int& ey1) {
-  constexpr int MP = 16 * T, NV = 2 * NE, NHALF = 8 / NE, NCW = T * NHALF, PL = T * T * 32, LDW = MP + 1;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+template <int T, int NE, int NP = 1, class Bar, class Pre>
+__device__ __forceinline__ bool tile_inverse(const double* x, const int M, const float tau, const TileSmem& s,
+                                             volatile int* flag, Bar bar, Pre pre, double* gd, int& ey0, int& ey1) {
+  static_assert(NP == 1 || T == 1, "a part each only for one tile");
+  constexpr int MP = 16 * T, NV = 2 * NE / NP, NHALF = 8 / NE, NCW = T * NHALF * NP, PL = T * T * 32, LDW = MP + 1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) / NP, part = NP == 2 ? (tid >> 5) & 1 : 0;
+  const int cw = (warp % (T * NHALF)) * NP + part;  // this warp among those of its rows
   const int g = lane >> 2, t4 = lane & 3;
   const int tile = warp / NHALF, half = NHALF == 2 ? warp & 1 : 0;
   const int ti = tile / T, tj = tile % T;
@@ -218,16 +222,17 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
   const char* bB = (const char*)regB;
 
   // Row exponents over the warps of a row, then the planes of X.
-  float2 m[NE];
-  uint32_t x7[NE];  // the seventh digit of X
+  float2 m[NE];  // (NP = 2: the other part is not used)
+  uint32_t x7[NE / NP];  // the seventh digit of X
   {
     int e0 = oz::kNoExp, e1 = oz::kNoExp;
 #pragma unroll
     for (int k = 0; k < NE; ++k) {
-      if (erow(k)) e1 = max(e1, oz::fexp2(x[k]));
-      else e0 = max(e0, oz::fexp2(x[k]));
+      const int e = oz::fexp2(make_double2(x[k], NP == 1 ? x[NE + k] : 0.0));
+      if (erow(k)) e1 = max(e1, e);
+      else e0 = max(e0, e);
     }
-    oz::put_row_exps(exX + (tj * NHALF + half) * MP, ti, lane, e0, e1);
+    oz::put_row_exps(exX + cw * MP, ti, lane, e0, e1);
     bar();
     if (tid < 32) red[tid] = 0;
     if (tid == 0) rsum[0] = 0;
@@ -237,11 +242,14 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
 #pragma unroll
     for (int k = 0; k < NE; ++k) {
       const int e = erow(k) ? e1 : e0;
-      fx[k] = oz::sfixed62(x[k].x, e);
-      fx[NE + k] = oz::sfixed62(x[k].y, e);
-      m[k] = make_float2(to_f32(x[k].x), to_f32(x[k].y));
+      fx[k] = oz::sfixed62(x[k], e);
+      m[k].x = to_f32(x[k]);
+      if (NP == 1) {
+        fx[NV - NE + k] = oz::sfixed62(x[NV - NE + k], e);
+        m[k].y = to_f32(x[NV - NE + k]);
+      }
     }
-    oz::put_planes<62, NE>(fx, 6, regA + own, PL, 6, half, 0, x7);
+    oz::put_planes<62, NE, NP>(fx, 6, regA + own, PL, 6, half, 0, x7, part);
   }
 
   // 2. Y0: block Gauss-Jordan in FP32 on the tiles in registers, pivot
@@ -262,9 +270,15 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
   const int lc = 2 * t4 + 8 * half;           // this lane's first column inside the tile
   auto put_tile = [&](float2* dst) {
 #pragma unroll
-    for (int q = 0; q < NE; q += 2)
-      *reinterpret_cast<float4*>(dst + (g + erow(q)) * kTileLd + lc + (q & 4 ? 8 : 0)) =
-          make_float4(m[q].x, m[q].y, m[q + 1].x, m[q + 1].y);
+    for (int q = 0; q < NE; q += 2) {
+      float2* d = dst + (g + erow(q)) * kTileLd + lc + (q & 4 ? 8 : 0);
+      if (NP == 2) {
+        reinterpret_cast<float*>(d)[part] = m[q].x;
+        reinterpret_cast<float*>(d)[2 + part] = m[q + 1].x;
+      } else {
+        *reinterpret_cast<float4*>(d) = make_float4(m[q].x, m[q].y, m[q + 1].x, m[q + 1].y);
+      }
+    }
   };
   bool small_pivot = false;
 #pragma unroll 1
@@ -276,11 +290,14 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
       if (ti == t && tj != t) put_tile(Rt + tj * kTileF2);
     }
     bar();
-    if (ti == t && tj == t && half == 0) small_pivot |= invert_tile(Pt, min(16, M - 16 * t), tau, lane);
+    if (ti == t && tj == t && half == 0 && part == 0) small_pivot |= invert_tile(Pt, min(16, M - 16 * t), tau, lane);
     bar();
     if (ti == t && tj == t) {
 #pragma unroll
-      for (int q = 0; q < NE; ++q) m[q] = Pt[(g + erow(q)) * kTileLd + lc + ecol(q)];
+      for (int q = 0; q < NE; ++q) {
+        m[q] = Pt[(g + erow(q)) * kTileLd + lc + ecol(q)];
+        if (NP == 2 && part) m[q].x = m[q].y;
+      }
     } else if (T > 1 && (ti == t || tj == t)) {
 #pragma unroll
       for (int q = 0; q < NE; ++q) m[q] = make_float2(0.0f, 0.0f);
@@ -303,13 +320,21 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
   // above it), so that its planes serve as both operands.
   float2* sy = (float2*)(regB + 6 * PL);  // [MP][LDW]
 #pragma unroll
-  for (int k = 0; k < NE; ++k) sy[(r0 + erow(k)) * LDW + c0 + ecol(k)] = m[k];
+  for (int k = 0; k < NE; ++k) {
+    float2* d = sy + (r0 + erow(k)) * LDW + c0 + ecol(k);
+    if (NP == 2) reinterpret_cast<float*>(d)[part] = m[k].x;
+    else *d = m[k];
+  }
   bar();
   if (*flag == kStatusNeedPivot) return false;
 #pragma unroll
   for (int k = 0; k < NE; ++k) {
     const int i = r0 + erow(k), j = c0 + ecol(k);
-    if (i > j) m[k] = sy[j * LDW + i];
+    if (i > j) {
+      m[k] = sy[j * LDW + i];
+      if (NP == 2 && part) m[k].x = m[k].y;
+    }
+    if (NP == 2) m[k].y = 0.0f;
   }
   long long acc[NV];  // the sum of the series, kAccBits of the row's power of two
   {
@@ -319,7 +344,7 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
       if (erow(k)) k1 = max(k1, fkey(m[k]));
       else k0 = max(k0, fkey(m[k]));
     }
-    oz::put_row_exps(exY + (tj * NHALF + half) * MP, ti, lane, k0 ? (int)(k0 >> 23) - 126 : oz::kNoExp,
+    oz::put_row_exps(exY + cw * MP, ti, lane, k0 ? (int)(k0 >> 23) - 126 : oz::kNoExp,
                      k1 ? (int)(k1 >> 23) - 126 : oz::kNoExp);
     bar();
     ey0 = oz::row_exp<NCW>(exY, MP, r0);
@@ -331,11 +356,11 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
     for (int k = 0; k < NE; ++k) {
       const float f = erow(k) ? s1 : s0;
       acc[k] = __float2int_rn(m[k].x * f);
-      acc[NE + k] = __float2int_rn(m[k].y * f);
+      if (NP == 1) acc[NV - NE + k] = __float2int_rn(m[k].y * f);
     }
-    oz::put_planes<kY0Bits, NE>(acc, 3, regB + own, PL, 3, half);
-    oz::put_words<NE>(x7, regB + 6 * PL + own, odd, half);
-    oz::put_words<NE>(x7 + NE / 2, regB + 7 * PL + own, odd, half);
+    oz::put_planes<kY0Bits, NE, NP>(acc, 3, regB + own, PL, 3, half, 0, nullptr, part);
+    oz::put_words<NE>(x7, regB + (6 + part) * PL + own, odd, half);
+    if (NP == 1) oz::put_words<NE>(x7 + (NE / 2) % (NE / NP), regB + 7 * PL + own, odd, half);
 #pragma unroll
     for (int k = 0; k < NV; ++k) acc[k] *= 1LL << (kAccBits - kY0Bits);
   }
@@ -348,11 +373,11 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
 #pragma unroll
   for (int h = 0; h < NE / 4; ++h) {
     long long hi[8], lo[8];
-    oz::half_product<T, 3, 7, oz::kLmax>(bB + offA0, bB + offA1, 3 * kPlane, bA + offB + 8 * (odd ^ (half | h)),
+    oz::half_product<T, 3, 7, oz::kLmax, NP>(bB + offA0, bB + offA1, 3 * kPlane, bA + offB + 8 * (odd ^ (half | h)),
                                          6 * kPlane, kPlane, hi, lo,
-                                         bB + 6 * kPlane + offB + 8 * (odd ^ (half | h)));
+                                         bB + 6 * kPlane + offB + 8 * (odd ^ (half | h)), part);
 #pragma unroll
-    for (int w = 0; w < 8; ++w) {
+    for (int w = 0; w < 8 / NP; ++w) {
       const int k = 4 * h + (w & 3);
       const int i = r0 + erow(k), j = c0 + ecol(k);
       const int e = (erow(k) ? ey1 : ey0) + oz::row_exp<NCW>(exX, MP, j);
@@ -361,7 +386,7 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
         const int up = 35 - e;  // |Y0 X| < 2, or the inverse is useless
         const long long top = hi[w] + (lo[w] >> 36);
         const bool fits = up >= 62 || (up >= 0 ? (top >> up) == 0 || (top >> up) == -1 : top == 0);
-        y = (w < 4 && i == j ? 1LL << 62 : 0) - oz::fix_shift(hi[w], lo[w], 28 + e);
+        y = (w < 4 && part == 0 && i == j ? 1LL << 62 : 0) - oz::fix_shift(hi[w], lo[w], 28 + e);
         const unsigned long long av = (unsigned long long)(y < 0 ? -y : y);
         mx = max(mx, fits ? (unsigned)(av >> 32) : ~0u);
         const unsigned long long q = min(av >> 36, 1ULL << 26);
@@ -389,7 +414,7 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
   auto levels = [&](int s) { return max(0, min(oz::kLmax, (62 + er + s + 8) / 9 - 1)); };
   // E_1 = R Y0, E_k+1 = R E_k; the sum starts from Y0.
   int lm = levels(0);
-  oz::put_planes<53, NE>(v, 6, regA + own, PL, 6, half, 9 + er);
+  oz::put_planes<53, NE, NP>(v, 6, regA + own, PL, 6, half, 9 + er, nullptr, part);
   bar();
   float rk = rn;  // ||R||^k of the term just formed
   int sk = 0;     // the B operand's entries are below 2^(e_i + sk)
@@ -400,17 +425,17 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
       long long hi[8], lo[8];
       const char* b = bB + offB + 8 * (odd ^ (half | h));
       if (term == 1) {
-        if (lm <= 4) oz::half_product<T, 5, 3, 4>(bA + offA0, bA + offA1, 6 * kPlane, b, 3 * kPlane, kPlane, hi, lo);
-        else oz::half_product<T, 6, 3, 6>(bA + offA0, bA + offA1, 6 * kPlane, b, 3 * kPlane, kPlane, hi, lo);
+        if (lm <= 4) oz::half_product<T, 5, 3, 4, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 3 * kPlane, kPlane, hi, lo, nullptr, part);
+        else oz::half_product<T, 6, 3, 6, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 3 * kPlane, kPlane, hi, lo, nullptr, part);
       } else if (lm == 0) {
-        oz::half_product<T, 1, 1, 0>(bA + offA0, bA + offA1, 6 * kPlane, b, 6 * kPlane, kPlane, hi, lo);
+        oz::half_product<T, 1, 1, 0, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 6 * kPlane, kPlane, hi, lo, nullptr, part);
       } else if (lm <= 2) {
-        oz::half_product<T, 3, 3, 2>(bA + offA0, bA + offA1, 6 * kPlane, b, 6 * kPlane, kPlane, hi, lo);
+        oz::half_product<T, 3, 3, 2, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 6 * kPlane, kPlane, hi, lo, nullptr, part);
       } else {
-        oz::half_product<T, 6, 6, 6>(bA + offA0, bA + offA1, 6 * kPlane, b, 6 * kPlane, kPlane, hi, lo);
+        oz::half_product<T, 6, 6, 6, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 6 * kPlane, kPlane, hi, lo, nullptr, part);
       }
 #pragma unroll
-      for (int w = 0; w < 8; ++w) {
+      for (int w = 0; w < 8 / NP; ++w) {
         const int k = 4 * h + (w & 3);
         const int e = oz::row_exp<NCW>(exY, MP, c0 + ecol(k)) - (erow(k) ? ey1 : ey0);
         // rounded: truncating, a bias of 2^-57 in every entry, is an
@@ -430,7 +455,8 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
     const int bits = 56 - __clz((int)red[term]);  // |E| < 2^bits
     sk = bits - kAccBits;
     lm = levels(sk);
-    oz::put_planes<53, NE>(v, lm == 0 ? 1 : lm <= 2 ? 3 : 6, regB + own, PL, 6, half, bits - 53);
+    oz::put_planes<53, NE, NP>(v, lm == 0 ? 1 : lm <= 2 ? 3 : 6, regB + own, PL, 6, half,
+                                  bits - 53, nullptr, part);
     bar();
   }
 
@@ -439,19 +465,24 @@ __device__ __forceinline__ bool tile_inverse(const double2* x, const int M, cons
   // G made exactly symmetric (below the diagonal from above it): left
   // to the rounding of the two halves, its asymmetry grew along the
   // guide and tripled the error of t.
-  double2* gb = (double2*)regB;  // [MP][LDW]
+  double* gb = (double*)regB;  // [MP][LDW] complex
 #pragma unroll
   for (int k = 0; k < NE; ++k) {
     const int e = (erow(k) ? ey1 : ey0) - kAccBits;
     const int i = r0 + erow(k), j = c0 + ecol(k);
-    gd[k] = make_double2(oz::fix_to_double(acc[k], e), oz::fix_to_double(acc[NE + k], e));
-    if (i < j) gb[i * LDW + j] = gd[k];
+#pragma unroll
+    for (int q = k; q < NV; q += NE) {
+      gd[q] = oz::fix_to_double(acc[q], e);
+      if (i < j) gb[2 * (i * LDW + j) + (q < NE ? part : 1)] = gd[q];
+    }
   }
   bar();
 #pragma unroll
   for (int k = 0; k < NE; ++k) {
     const int i = r0 + erow(k), j = c0 + ecol(k);
-    if (i > j) gd[k] = gb[j * LDW + i];
+#pragma unroll
+    for (int q = k; q < NV; q += NE)
+      if (i > j) gd[q] = gb[2 * (j * LDW + i) + (q < NE ? part : 1)];
   }
   return true;
 }
