@@ -174,11 +174,6 @@ __device__ __forceinline__ float2 reduce2(float2 x, float2 mp, float2 inv) {  //
   return fma2(q, mp, x);
 }
 
-__device__ __forceinline__ float reduce(float x, float p, float inv) {
-  const float q = fmaf(x, inv, kMagic) - kMagic;
-  return fmaf(-q, p, x);
-}
-
 __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);
   uint32_t r;
@@ -276,15 +271,17 @@ __device__ __forceinline__ void split(int M, Get get, const int* ex, uint4* dig,
 }
 
 // A CTA of 8 warps computes a 64 x 64 block: warps 0..3 the u products of its
-// four 32 x 32 quadrants, warps 4..7 the v products.  The planes of 32 k (16
+// four 32 x 32 quadrants, warps 4..7 the v products.  The planes of 64 k (32
 // KB: 4 row and 4 column tiles, u and v) are staged in shared memory with
-// cp.async, kStages deep (stg: kStageUint4), the moduli in sequence; with two
-// stages of 64 k instead the copies' latency left a step at 2,800 clocks for
-// 550 of mma.sync.
+// cp.async, kStages deep (stg: kStageUint4), the moduli in sequence; the sums
+// of a stage stay exact, and are reduced modulo p at its end.  (Four stages of
+// 32 k: 126 for 116 ms of 512 modes, t of 16 realizations and 16 slices; 217 for
+// 212 ms of 152 at 256 modes.)
 constexpr int kBlkTiles = 4;
-constexpr int kStageK = 2;                                   // k tiles of a stage
-constexpr int kOneUint4 = 2 * 2 * kBlkTiles * kStageK * 32;  // [A, B][u, v][tile][k tile][lane]
-constexpr int kStages = 4;
+constexpr int kStageK = 4;                                        // k tiles of a stage
+constexpr int kHalfUint4 = 2 * kBlkTiles * kStageK * 32;          // [u, v][tile][k tile][lane]
+constexpr int kOneUint4 = 2 * kHalfUint4;                         // of A, then of B
+constexpr int kStages = 3;
 constexpr int kStageUint4 = kStages * kOneUint4;
 
 // Stores C_ij by out(i, j, 0, re) and out(i, j, 1, im) for i, j < M in the
@@ -298,29 +295,29 @@ __device__ void gemm_block(int M, int ti0, int tj0, const uint4* adig, const uin
   const int64_t plane = (int64_t)T * T * 32;
   const int nch = (T + kStageK - 1) / kStageK;  // stages of a modulus
   const int nsteps = kMod * nch;
-  // The 4 copies of a thread and step: element e of the stage is lane e & 31
-  // of k tile (e >> 5) & 1 of tile (e >> 6) & 3 of plane (e >> 8) & 1 of A
-  // (e < 512) or B; the addresses advance by stage and modulus.
-  const uint4* src[4];
-  bool on[4];
-  const int kt0 = (tid >> 5) & 1;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int e = tid + 256 * q;
-    const int tile = (e >> 6) & 3, pl = (e >> 8) & 1;
-    const int t = (q >= 2 ? tj0 : ti0) + tile;
-    on[q] = t < T;
-    src[q] = (q >= 2 ? bdig : adig) + pl * plane + ((int64_t)t * T + kt0) * 32 + (e & 31);
-  }
+  // The 8 copies of a thread and step: element e = tid + 256 q of the stage is
+  // lane e & 31 of k tile (e >> 5) & 3 of tile (e >> 7) & 3 of plane (e >> 9) &
+  // 1 of A (e < 1024) or B.
+  const int kt0 = (tid >> 5) & 3, tl0 = tid >> 7;  // tiles tl0 and tl0 + 2
+  const int64_t at = ((int64_t)tl0 * T + kt0) * 32 + lane;
+  const uint4* asrc = adig + (int64_t)ti0 * T * 32 + at;
+  const uint4* bsrc = bdig + (int64_t)tj0 * T * 32 + at;
+  const int two = 2 * T * 32;  // two tiles on
+  const bool a0 = ti0 + tl0 < T, a1 = ti0 + tl0 + 2 < T, b0 = tj0 + tl0 < T, b1 = tj0 + tl0 + 2 < T;
   int fm = 0, fch = 0;  // modulus and stage of the next fetch
   auto fetch = [&](int step) {
     if (step < nsteps) {
-      uint4* dst = stg + (step % kStages) * kOneUint4;
-      const int64_t off = 2 * fm * plane + fch * (kStageK * 32);
-      const bool kin = fch * kStageK + kt0 < T;
+      uint4* dst = stg + (step % kStages) * kOneUint4 + tid;
+      if (fch * kStageK + kt0 < T) {
+        const int64_t off = 2 * fm * plane + fch * (kStageK * 32);
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (on[q] && kin) oz::cp_async16(dst + tid + 256 * q, src[q] + off);
+        for (int pl = 0; pl < 2; ++pl) {
+          if (a0) oz::cp_async16(dst + 512 * pl, asrc + off + pl * plane);
+          if (a1) oz::cp_async16(dst + 512 * pl + 256, asrc + off + pl * plane + two);
+          if (b0) oz::cp_async16(dst + kHalfUint4 + 512 * pl, bsrc + off + pl * plane);
+          if (b1) oz::cp_async16(dst + kHalfUint4 + 512 * pl + 256, bsrc + off + pl * plane + two);
+        }
+      }
       if (++fch == nch) {
         fch = 0;
         ++fm;
@@ -333,6 +330,7 @@ __device__ void gemm_block(int M, int ti0, int tj0, const uint4* adig, const uin
   for (int k = 0; k < kStages - 1; ++k) fetch(k);
   int m = 0, ch = 0;
   for (int step = 0; step < nsteps; ++step) {
+    const float2 mp = both(-kT.p[m]), inv = both(kT.inv[m]);
     asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
     __syncthreads();  // this stage is here, and the one before it has been used
     fetch(step + kStages - 1);
@@ -346,7 +344,7 @@ __device__ void gemm_block(int M, int ti0, int tj0, const uint4* adig, const uin
     }
     const uint4* cur = stg + (step % kStages) * kOneUint4;
     const uint4* As = cur + (uv * 4 + 2 * qr) * (kStageK * 32) + lane;
-    const uint4* Bs = cur + 512 + (uv * 4 + 2 * qc) * (kStageK * 32) + lane;
+    const uint4* Bs = cur + kHalfUint4 + (uv * 4 + 2 * qc) * (kStageK * 32) + lane;
     const int nk = min(kStageK, T - kStageK * ch);
 #pragma unroll
     for (int kt = 0; kt < kStageK; ++kt) {
@@ -367,15 +365,16 @@ __device__ void gemm_block(int M, int ti0, int tj0, const uint4* adig, const uin
       }
     }
     const bool last = ch == nch - 1;
-    if (last || (ch & 1)) {  // 64 k at most since the last reduction
-      const float p = kT.p[m], inv = kT.inv[m];
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int w = 0; w < 8; ++w) acc[i][j][w] = reduce(acc[i][j][w], p, inv);
-    }
+        for (int w = 0; w < 8; w += 2) {
+          const float2 r = reduce2(make_float2(acc[i][j][w], acc[i][j][w + 1]), mp, inv);
+          acc[i][j][w] = r.x;
+          acc[i][j][w + 1] = r.y;
+        }
     if (last) {
 #pragma unroll
       for (int i = 0; i < 2; ++i)
