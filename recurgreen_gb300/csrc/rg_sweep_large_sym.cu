@@ -284,38 +284,49 @@ struct ZgemmCtx {
 // read only in the first two phases, so out may overwrite them.  Called by
 // every thread of the cluster; ends with a cluster barrier.  Not inlined: the
 // products of a slice share one copy.
+// Two of the four products of a node take over planes (512 modes 116 -> 112 ms,
+// 152 realizations of 256 modes 212 -> 203): the planes and exponents of an
+// operand that the last product, of the same
+// Mb, has left are taken over: with have = 1 those of its B, which is this A's
+// transpose, with have = 2 those of its A, which is this B's transpose.
 __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const Opnd A, const Opnd B,
-                                           const TileOut out) {
+                                           const TileOut out, const int have) {
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int tid = threadIdx.x, ctid = rank * kSymNT + tid, CNT = C * kSymNT;
   const int T = oz::tiles(Mb);
+  uint4 *const adig = have ? c.bdig : c.adig, *const bdig = have ? c.adig : c.bdig;
+  int *const ea = have ? c.eb_s : c.ea_s, *const eb = have ? c.ea_s : c.eb_s;
   for (int i = tid; i < 16 * T; i += kSymNT) {
-    c.ea_s[i] = oz::kNoExp;
-    c.eb_s[i] = oz::kNoExp;
+    if (have != 1) ea[i] = oz::kNoExp;
+    if (have != 2) eb[i] = oz::kNoExp;
   }
   __syncthreads();
-  operand_exps(A, true, c.ea_s, ctid >> 5, CNT >> 5);
-  operand_exps(B, false, c.eb_s, ctid >> 5, CNT >> 5);
+  if (have != 1) operand_exps(A, true, ea, ctid >> 5, CNT >> 5);
+  if (have != 2) operand_exps(B, false, eb, ctid >> 5, CNT >> 5);
   __syncthreads();
-  int* mine = c.expart + rank * 32 * T;
-  for (int i = tid; i < 16 * T; i += kSymNT) {
-    mine[i] = c.ea_s[i];
-    mine[16 * T + i] = c.eb_s[i];
-  }
-  cluster.sync();
-  for (int i = tid; i < 16 * T; i += kSymNT) {
-    int x = oz::kNoExp, y = oz::kNoExp;
-    for (int r = 0; r < C; ++r) {
-      x = max(x, __ldcg(c.expart + r * 32 * T + i));
-      y = max(y, __ldcg(c.expart + r * 32 * T + 16 * T + i));
+  if (C > 1) {
+    int* mine = c.expart + rank * 32 * T;
+    for (int i = tid; i < 16 * T; i += kSymNT) {
+      mine[i] = ea[i];
+      mine[16 * T + i] = eb[i];
     }
-    c.ea_s[i] = x;
-    c.eb_s[i] = y;
+    cluster.sync();
+    for (int i = tid; i < 16 * T; i += kSymNT) {
+      int x = oz::kNoExp, y = oz::kNoExp;
+      for (int r = 0; r < C; ++r) {
+        x = max(x, __ldcg(c.expart + r * 32 * T + i));
+        y = max(y, __ldcg(c.expart + r * 32 * T + 16 * T + i));
+      }
+      ea[i] = x;
+      eb[i] = y;
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  crt::split(Mb, [&](int i, int k) { return opnd_at(A, i, k); }, c.ea_s, c.adig, c.stage, ctid >> 5, CNT >> 5);
-  crt::split(Mb, [&](int j, int k) { return opnd_at(B, k, j); }, c.eb_s, c.bdig, c.stage, ctid >> 5, CNT >> 5);
+  if (have != 1)
+    crt::split(Mb, [&](int i, int k) { return opnd_at(A, i, k); }, ea, adig, c.stage, ctid >> 5, CNT >> 5);
+  if (have != 2)
+    crt::split(Mb, [&](int j, int k) { return opnd_at(B, k, j); }, eb, bdig, c.stage, ctid >> 5, CNT >> 5);
   __shared__ TileOut s_out;
   if (tid == 0) s_out = out;
   cluster.sync();  // every residue is written before any CTA reads them (and s_out is set)
@@ -324,8 +335,7 @@ __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const
   for (int bi = 0; bi < nb; ++bi)
     for (int bj = out.upper ? bi : 0; bj < nb; ++bj)
       if (k++ % C == rank)
-        block_product(Mb, bi * crt::kBlkTiles, bj * crt::kBlkTiles, c.adig, c.bdig, c.ea_s, c.eb_s, c.stage, c.res,
-                      &s_out);
+        block_product(Mb, bi * crt::kBlkTiles, bj * crt::kBlkTiles, adig, bdig, ea, eb, c.stage, c.res, &s_out);
   cluster.sync();
 }
 
@@ -1096,6 +1106,7 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
               for (int j = i + lane; j < h2; j += 32) P[(int64_t)(h1 + i) * nP + h1 + j] = __ldcg(Hs + i * h2 + j);
             cluster.sync();
           } else {
+            int have = 0;
             Opnd A, B;
             TileOut o{P, nP, h1, -1.0, nullptr, 0, 0, 0, 0, h1, h2};
             if (op == kInvT) {
@@ -1103,6 +1114,7 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
               B = Opnd{P, nP, h1, 0, 0, h1, h2};
               o.dst = Hb, o.ld = h1, o.off = 0, o.sign = 1.0;
             } else if (op == kInvS) {
+              have = 1;  // B^T, after kInvT's B
               A = Opnd{P, nP, h1, 0, 1, h2, h1};
               B = Opnd{Hb, h1, 0, 0, 0, h1, h2};
               o = TileOut{Hs, h2, 0, -1.0, P, nP, (int64_t)h1 * nP + h1, 0, 1, h2, h2};
@@ -1110,12 +1122,13 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
               A = Opnd{Hb, h1, 0, 0, 0, h1, h2};
               B = Opnd{Hs, h2, 0, 1, 0, h2, h2};
             } else {  // kInvY11
+              have = 2;  // T^T, after kInvY12's T
               A = Opnd{P, nP, h1, 0, 0, h1, h2};
               B = Opnd{Hb, h1, 0, 0, 1, h2, h1};
               o = TileOut{P, nP, 0, -1.0, Ha, h1, 0, 1, 1, h1, h1};
             }
             if (h1 <= kTinyModes) tiny_zgemm(stage, A, B, o);
-            else cluster_zgemm(zc, h1, A, B, o);
+            else cluster_zgemm(zc, h1, A, B, o, have);
           }
         }
       }
@@ -1134,7 +1147,7 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
         } else {
           // the result overwrites B Gs1 in place (its residues are already taken)
           cluster_zgemm(zc, M, Opnd{W, M, 0, 1, 0, M, M}, Opnd{Rg, M, 0, 0, 0, M, M},
-                        TileOut{Rg, M, 0, 1.0, nullptr, 0, 0, 0, 0, M, M});
+                        TileOut{Rg, M, 0, 1.0, nullptr, 0, 0, 0, 0, M, M}, 0);
         }
       }
       if (a.state_dump && *status0 != kStatusNeedPivot) {
