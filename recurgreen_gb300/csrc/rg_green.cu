@@ -17,6 +17,7 @@
 #include <algorithm>
 
 #include "rg_device.cuh"
+#include "rg_ozaki.cuh"
 
 namespace rg {
 namespace {
@@ -542,6 +543,192 @@ __global__ void __launch_bounds__(kNT) back_kernel(BackArgs a) {
   }
 }
 
+// The same for up to 64 modes on the FP16 tensor cores: eight vectors are the n8
+// side of mma.m16n8k16.  Per slice the 16 warps turn S and Z into six 9-bit
+// digits a part (rg_ozaki.cuh; a warp per tile), then each has one row tile, one
+// part and one of the two products; the vectors' digits, W in one word pair and B
+// Y_{n+1} in the other, follow those of S and Z in every plane.  The FP64 form
+// takes 32 M^2 multiply-adds a slice and vector at 1.7 lanes per clock: 25 ms of
+// 152 items, 300 slices and some eight vectors at 64 modes, 6.4 here
+// (profiles 90 -> 71 ms).
+constexpr int kBackNT = 512;
+template <int T>
+struct BackTile {
+  static constexpr int MP = 16 * T, TILES = 2 * T * T + T;  // tiles of a plane: S, Z, vectors
+  static constexpr int kPlane = TILES * 512;                // bytes
+  static constexpr size_t bytes() {
+    return 12 * (size_t)kPlane + sizeof(double2) * MP * kKC + sizeof(double) * 2 * kKC +
+           sizeof(int) * (2 * T * MP + 3 * kKC);
+  }
+};
+template <int T>
+__global__ void __launch_bounds__(kBackNT, 1) back_tile_kernel(BackArgs a) {
+  using Cf = BackTile<T>;
+  constexpr int MP = Cf::MP, TILES = Cf::TILES, kPlane = Cf::kPlane, NW = kBackNT / 32, QT = (2 * T * T + NW - 1) / NW;
+  static_assert(kKC == 8 && 4 * T <= NW && 2 * kKC == NW, "warps' tasks");
+  extern __shared__ uint4 shp[];
+  char* P = reinterpret_cast<char*>(shp);
+  double2* R = reinterpret_cast<double2*>(P + 12 * kPlane);   // [MP][kKC] vectors
+  double* psum = reinterpret_cast<double*>(R + MP * kKC);     // [2 kKC] |Y|^2 by vector and half of the rows
+  int* ex = reinterpret_cast<int*>(psum + 2 * kKC);           // [2][T][MP] row exponents of S, Z by tile column
+  int* exw = ex + 2 * T * MP;                                 // [kKC] exponents of W,
+  int* exy = exw + kKC;                                       // [2 kKC] of B Y by half of the rows
+  const int M = a.M, r = blockIdx.y, kr = a.kcount ? a.kcount[r] : a.kmax, s0 = blockIdx.x * kKC;
+  if (s0 >= kr) return;  // uniform over the block
+  const int nv = min(kKC, kr - s0);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3, odd = (lane >> 3) & 1;
+  const int vv = warp >> 1, vm = (warp & 1) * 32 + lane;  // element steps: vector and row of a thread
+  // Digits of the vectors in R with exponents e(v), to word pair `slot`: warps
+  // (k tile, part); the vectors are the rows of the operand's transpose.
+  auto put_vectors = [&](int slot, auto e) {
+    if (warp >= 2 * T) return;
+    const int tk = warp >> 1, part = warp & 1;
+    const double* Rd = reinterpret_cast<const double*>(R);
+    const int ev = e(g);
+    long long bias = 0;
+#pragma unroll
+    for (int p = 0; p < 6; ++p) bias += 256LL << (oz::kDigitBits * p);
+    unsigned long long y[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int m = tk * 16 + 2 * t4 + (k & 1) + 8 * (k >> 1);
+      y[k] = (unsigned long long)(oz::sfixed53(Rd[2 * (m * kKC + g) + part], ev) + bias);
+    }
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+      const uint32_t mask = p ? 511u : 1023u;
+      uint32_t w[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        w[k] = oz::field_pair((uint32_t)(y[2 * k] >> (oz::kDigitBits * (5 - p))) & mask,
+                              (uint32_t)(y[2 * k + 1] >> (oz::kDigitBits * (5 - p))) & mask);
+      *reinterpret_cast<uint2*>(P + (6 * part + p) * kPlane + (2 * T * T + tk) * 512 + lane * 16 + 8 * (odd ^ slot)) =
+          make_uint2(w[0], w[1]);
+    }
+  };
+  double2 w0 = make_double2(0.0, 0.0);
+  if (vm < M && vv < nv) w0 = a.src[(int64_t)r * a.src_stride + (int64_t)(s0 + vv) * M + vm];
+  const double2 bm = vm < M ? a.bmat[vm] : w0;
+  if (vm < MP) R[vm * kKC + vv] = w0;
+  int ew = __reduce_max_sync(0xffffffffu, oz::fexp2(w0));
+  if (lane == 0) exy[warp] = ew;
+  __syncthreads();
+  if (tid < kKC) exw[tid] = max(exy[2 * tid], exy[2 * tid + 1]);
+  put_vectors(0, [&](int v) { return max(exy[2 * v], exy[2 * v + 1]); });
+  __syncthreads();
+  const int64_t mm = (int64_t)M * M;
+  const int nslices = a.only_lo ? 1 : a.nx - a.i_lo;
+  for (int n = a.nx - 1; n >= a.i_lo; --n) {
+    const double2* S = a.dump + ((int64_t)r * a.nx + n) * 2 * mm;  // Z follows
+    const bool first = n == a.nx - 1;
+    double2 x[QT][8];
+#pragma unroll
+    for (int q = 0; q < QT; ++q) {
+      const int task = warp + NW * q, mat = task / (T * T), tile = task % (T * T);
+      if (task < 2 * T * T) {
+        const int ti = tile / T, tj = tile % T;
+        int e0 = oz::kNoExp, e1 = oz::kNoExp;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int i = ti * 16 + g + 8 * ((k >> 1) & 1), j = tj * 16 + 2 * t4 + (k & 1) + 8 * (k >> 2);
+          x[q][k] = i < M && j < M ? __ldg(S + mat * mm + (int64_t)i * M + j) : make_double2(0.0, 0.0);
+          if ((k >> 1) & 1) e1 = max(e1, oz::fexp2(x[q][k]));
+          else e0 = max(e0, oz::fexp2(x[q][k]));
+        }
+        oz::put_row_exps(ex + (mat * T + tj) * MP, ti, lane, e0, e1);
+      }
+    }
+    __syncthreads();  // the exponents, and B Y's digits
+#pragma unroll
+    for (int q = 0; q < QT; ++q) {
+      const int task = warp + NW * q, mat = task / (T * T), tile = task % (T * T);
+      if (task < 2 * T * T) {
+        const int row = (tile / T) * 16 + g;
+        const int e0 = oz::row_exp<T>(ex + mat * T * MP, MP, row), e1 = oz::row_exp<T>(ex + mat * T * MP, MP, row + 8);
+        long long f[16];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          f[k] = oz::sfixed53(x[q][k].x, (k >> 1) & 1 ? e1 : e0);
+          f[8 + k] = oz::sfixed53(x[q][k].y, (k >> 1) & 1 ? e1 : e0);
+        }
+        oz::put_planes<53, 8>(f, 6, reinterpret_cast<uint4*>(P) + (mat * T * T + tile) * 32 + lane, TILES * 32, 6, 0);
+      }
+    }
+    __syncthreads();
+    // warps 0 .. 2 T - 1: S (B Y), the next 2 T: Z W; the difference meets in R
+    const int mat = warp / (2 * T), rt = (warp >> 1) % T, part = warp & 1;
+    double val[4];
+    if (warp < 4 * T && !(first && mat == 0)) {
+      const char* pa = P + (mat * T * T + rt * T) * 512 + lane * 16;
+      long long hi[4], lo[4];
+      oz::half_product<T, 6, 6, oz::kLmax, 2>(pa + 8 * odd, pa + 8 * (1 - odd), 6 * kPlane,
+                                              P + 2 * T * T * 512 + lane * 16 + 8 * (odd ^ (1 - mat)), 6 * kPlane, kPlane,
+                                              hi, lo, nullptr, part);
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const int v = 2 * t4 + (w & 1);
+        const int e = oz::row_exp<T>(ex + mat * T * MP, MP, rt * 16 + g + 8 * (w >> 1));
+        val[w] = oz::fold_to_double(hi[w], lo[w], e + (mat ? exw[v] : max(exy[2 * v], exy[2 * v + 1])));
+      }
+    } else {
+#pragma unroll
+      for (int w = 0; w < 4; ++w) val[w] = 0.0;
+    }
+    double* Rd = reinterpret_cast<double*>(R) + 2 * ((rt * 16 + g) * kKC + 2 * t4) + part;
+    if (mat == 0) {
+#pragma unroll
+      for (int w = 0; w < 4; ++w) Rd[2 * (8 * (w >> 1) * kKC + (w & 1))] = val[w];
+    }
+    __syncthreads();
+    if (mat == 1) {
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        double* d = Rd + 2 * (8 * (w >> 1) * kKC + (w & 1));
+        *d = val[w] - *d;
+      }
+    }
+    __syncthreads();
+    double2 by = make_double2(0.0, 0.0);
+    double p = 0.0;
+    if (vm < M && vv < nv) {
+      const double2 y = R[vm * kKC + vv];
+      by = cmul(bm, y);
+      p = fma(y.x, y.x, y.y * y.y);
+      if (a.out_mode == kBackColumns && (!a.only_lo || n == a.i_lo)) {
+        const int64_t sl = a.only_lo ? 0 : n - a.i_lo;
+        double2 o = y;
+        if (a.left) {
+          const double2 q = cmul(a.left[vm], y);
+          o = make_double2(-2.0 * q.y, 2.0 * q.x);
+        }
+        a.cols[(((int64_t)r * nslices + sl) * a.kmax + s0 + vv) * M + vm] = o;
+      }
+    }
+    if (vm < MP) R[vm * kKC + vv] = by;
+    ew = __reduce_max_sync(0xffffffffu, oz::fexp2(by));
+    if (a.out_mode == kBackProfile) {
+#pragma unroll
+      for (int off = 16; off; off >>= 1) p += __shfl_xor_sync(0xffffffffu, p, off);
+    }
+    if (lane == 0) {
+      exy[warp] = ew;
+      psum[warp] = p;
+    }
+    __syncthreads();
+    if (a.out_mode == kBackProfile && tid < nv)
+      a.prof[((int64_t)r * a.kmax + s0 + tid) * a.nx + n] = psum[2 * tid] + psum[2 * tid + 1];
+    put_vectors(1, [&](int v) { return max(exy[2 * v], exy[2 * v + 1]); });
+  }
+}
+
+template <int T>
+int launch_back_tile(const BackArgs& a, cudaStream_t s) {
+  RG_CUDA(allow_smem((const void*)back_tile_kernel<T>, BackTile<T>::bytes()));
+  back_tile_kernel<T><<<dim3((a.kmax + kKC - 1) / kKC, a.nreal), kBackNT, BackTile<T>::bytes(), s>>>(a);
+  RG_CUDA(cudaGetLastError());
+  return RG_OK;
+}
+
 __global__ void windows_kernel(WindowArgs a) {
   const int64_t total = (int64_t)a.nreal * a.nprof * a.nx;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
@@ -624,10 +811,13 @@ int launch_eigvec(const EigvecArgs& a, cudaStream_t s) {
 int launch_back(const BackArgs& a, cudaStream_t s) {
   if (a.nreal <= 0 || a.kmax <= 0) return RG_OK;
   if (a.i_lo < 0 || a.i_lo >= a.nx) return fail(RG_ERR_INVALID_ARG, "back-substitution: slice out of range");
+  if (a.M <= 16) return launch_back_tile<1>(a, s);
+  if (a.M <= 32) return launch_back_tile<2>(a, s);
+  if (a.M <= 48) return launch_back_tile<3>(a, s);
+  if (a.M <= 64) return launch_back_tile<4>(a, s);
   const int J = (a.M * kKC + kNT - 1) / kNT;
   if ((2 * sizeof(double2) + sizeof(double)) * (size_t)a.M * kKC > 200 * 1024)
     return fail(RG_ERR_INVALID_ARG, "back-substitution: too many modes");
-  if (J <= 2) return launch_back_t<2>(a, s);
   if (J <= 4) return launch_back_t<4>(a, s);
   if (J <= 8) return launch_back_t<8>(a, s);
   if (J <= 16) return launch_back_t<16>(a, s);
