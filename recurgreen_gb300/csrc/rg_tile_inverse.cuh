@@ -77,6 +77,11 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
   return o;
 }
 
+__device__ __forceinline__ void fms(float2& m, float2 f, float2 s) {  // m -= f s
+  m.x = fmaf(f.y, s.y, fmaf(-f.x, s.x, m.x));
+  m.y = fmaf(-f.y, s.x, fmaf(-f.x, s.y, m.y));
+}
+
 // Entry k of a lane: row g + erow(k), column 2 t + ecol(k) (plus 8 in the
 // second half of a split tile), with g = lane / 4, t = lane % 4.
 __device__ __forceinline__ constexpr int erow(int k) { return 8 * ((k >> 1) & 1); }
@@ -87,24 +92,20 @@ __device__ __forceinline__ constexpr int ecol(int k) { return (k & 1) + 8 * (k >
 constexpr int kTileLd = 18, kTileF2 = 16 * kTileLd;
 
 // m -= A B over the 16 columns of A, for a lane's entries (rows g, g + 8;
-// columns lc, lc + 1 and, for a whole tile, 8 further on).  A product f s is
-// (-f.x, -f.x) (s.x, s.y) + (f.y, -f.y) (s.y, s.x): two packed FMAs.
+// columns lc, lc + 1 and, for a whole tile, 8 further on).  (Packed FMAs, two to
+// an instruction, need as many moves for their swapped and negated pairs.)
 template <int NE>
 __device__ __forceinline__ void tile_fms(float2* m, const float2* A, const float2* B, int g, int lc) {
-#pragma unroll 4
+#pragma unroll 2
   for (int k = 0; k < 16; ++k) {
     const float2 f0 = A[g * kTileLd + k], f1 = A[(g + 8) * kTileLd + k];
-    const float2 f0r = make_float2(-f0.x, -f0.x), f0i = make_float2(f0.y, -f0.y);
-    const float2 f1r = make_float2(-f1.x, -f1.x), f1i = make_float2(f1.y, -f1.y);
 #pragma unroll
     for (int q = 0; q < NE; q += 4) {
       const float4 u = *reinterpret_cast<const float4*>(B + k * kTileLd + lc + 2 * q);
-      const float2 s0 = make_float2(u.x, u.y), s1 = make_float2(u.z, u.w);
-      const float2 t0 = make_float2(s0.y, s0.x), t1 = make_float2(s1.y, s1.x);
-      m[q] = ffma2(f0i, t0, ffma2(f0r, s0, m[q]));
-      m[q + 1] = ffma2(f0i, t1, ffma2(f0r, s1, m[q + 1]));
-      m[q + 2] = ffma2(f1i, t0, ffma2(f1r, s0, m[q + 2]));
-      m[q + 3] = ffma2(f1i, t1, ffma2(f1r, s1, m[q + 3]));
+      fms(m[q], f0, make_float2(u.x, u.y));
+      fms(m[q + 1], f0, make_float2(u.z, u.w));
+      fms(m[q + 2], f1, make_float2(u.x, u.y));
+      fms(m[q + 3], f1, make_float2(u.z, u.w));
     }
   }
 }
@@ -301,8 +302,7 @@ __device__ __forceinline__ bool tile_inverse(const double* x, const int M, const
     } else if (T > 1 && (ti == t || tj == t)) {
 #pragma unroll
       for (int q = 0; q < NE; ++q) m[q] = make_float2(0.0f, 0.0f);
-      if (ti == t) tile_fms<NE>(m, Pt, Rt + tj * kTileF2, g, lc);
-      else tile_fms<NE>(m, Ct + ti * kTileF2, Pt, g, lc);
+      tile_fms<NE>(m, ti == t ? Pt : Ct + ti * kTileF2, ti == t ? Rt + tj * kTileF2 : Pt, g, lc);
       if (ti == t) {
 #pragma unroll
         for (int q = 0; q < NE; ++q) m[q] = make_float2(-m[q].x, -m[q].y);
