@@ -106,25 +106,31 @@ def flops_per_realization(M: int, nx: int) -> float:
 
 
 def executed_flops(M: int, nx: int, kernel: str) -> tuple[float, float]:
-    """(FP64 flops, FP16 tensor flops) the sweep executes for one realization:
-      * shared-memory symmetric kernel (M <= 64): 12 M^3 + 4 M^2 FP64 per slice;
-      * blocked symmetric kernel with the tensor-core propagator product
-        (64 < M <= 512): the inverse in FP64 -- 4 M^3 for one Gauss-Jordan
-        sweep; each level of the 2 x 2 block form (even sizes >= 128, at most
-        two levels) replaces a size-m inverse by two of size m/2 and four
-        (m/2)^3 products -- and 26 digit pairs x 4 real products x 2 k^3 FP16
-        flops per k x k product: 208 M^3 for the propagator product plus
-        4 x 208 (m/2)^3 per block split;
+    """(FP64 flops, FP16 tensor flops) the sweep executes for one realization, O(M^2) terms left out:
+      * tensor-core symmetric kernel (M <= 64): per slice 26 digit pairs x 8 M^3 for the propagator and 37 pairs
+        (residual 18, series 12 + 6 + 1) for the inverse, whose FP32 part is not counted;
+      * blocked symmetric kernel (64 < M <= 512): per k x k product 12 moduli x 2 real products of 2 k^3; one of M
+        for the propagator and four of half the size per block of the 2 x 2 form, halved down to leaves of at most
+        32 modes, whose own products (26 pairs) and inverse (37 pairs) are digit products.  With RG_SPLIT_INVERSE
+        0, 1 or 2 that many levels over even sizes >= 128 and FP64 elimination of the blocks left, the products
+        counted at the 26 digit pairs of their digit form;
       * otherwise the pivoted reference count 16 M^3 in FP64.
-    RG_TENSOR_R=0 / RG_SPLIT_INVERSE=0 or 1 select the other variants."""
+    RG_TENSOR_R=0 selects the FP64-only symmetric elimination."""
     tensor = os.environ.get("RG_TENSOR_R", "1") != "0" and 64 < M <= 512
-    want = {"0": 0, "1": 1}.get(os.environ.get("RG_SPLIT_INVERSE", "2"), 2)
+    want = {"0": 0, "1": 1, "2": 2}.get(os.environ.get("RG_SPLIT_INVERSE", "3"), 3)
     if kernel == "symmetric":
-        return flops_symmetric(M, nx), 0.0
+        return 0.0, (26 + 37) * 8.0 * M ** 3 * nx
     if kernel != "blocked_symmetric":
         return flops_per_realization(M, nx), 0.0
     if not tensor:
         return flops_symmetric(M, nx), 0.0
+    if want == 3:
+        fp16, m, blocks = 48.0 * M ** 3, float(M), 1
+        while m > 32:
+            m /= 2
+            fp16 += blocks * 4 * (48.0 if m > 32 else 26 * 8.0) * m ** 3
+            blocks *= 2
+        return 0.0, (fp16 + blocks * 37 * 8.0 * m ** 3) * nx
     fp16 = 208.0 * M ** 3
     m, blocks = M, 1
     while want > 0 and m >= 128 and m % 2 == 0:
@@ -142,7 +148,7 @@ def flops_symmetric(M: int, nx: int) -> float:
     return (12.0 * M ** 3 + 4.0 * M ** 2) * nx
 
 
-KERNEL_NAMES = {"symmetric": "sweep_sym_kernel<64,256,2>", "pivoted": "sweep_kernel<64,256,2>",
+KERNEL_NAMES = {"symmetric": "sweep_sym_kernel", "pivoted": "sweep_kernel<64,256,2>",
                 "blocked": "sweep_large_kernel", "blocked_symmetric": "sweep_large_sym_kernel"}
 
 
@@ -400,10 +406,10 @@ def run_main(args, spec: dict) -> None:
                                "fp16_tensor_flops_per_launch": fl16 * n, "fp16_tensor_tflops": t16,
                                "fp16_mma_sync_peak_tflops": mma_peak,
                                "fp16_tensor_frac_of_mma_sync": t16 / mma_peak if mma_peak == mma_peak else None,
-                               "note": "the FP64 inverse runs on the FP64 pipe; the propagator product (and, in "
-                                       "the 2x2 block form, the block products) on the FP16 tensor cores with "
-                                       "FP64 accuracy (exact digit products), so achieved above the FP64 peak "
-                                       "is work moved off the FP64 pipe"},
+                               "note": "inverse and products run on the FP16 tensor cores with FP64 accuracy "
+                                       "(exact modular and digit products, an FP32 inverse with its exact "
+                                       "residual series), so achieved above the FP64 peak is work moved off "
+                                       "the FP64 pipe"},
                            "kernel": KERNEL_NAMES.get(info["kernel"], info["kernel"]), "launch": info,
                            "kernel_ms_per_launch": 1e3 * per_launch,
                            "kernel_timing": "CUDA events around each batch's graph (sweep + pivoted re-run)"}

@@ -7,8 +7,8 @@
 // The reference solves the block tridiagonal system for every slice with
 // solve_block_tridiag (src/base_utils.f90:296-335): a forward loop S_n =
 // inv(A_n - B S_{n-1} B), Z_n = S_n (I_n - B Z_{n-1}) and a backward loop
-// X_n = Z_n - S_n B X_{n+1}, each block M x M.  Here the forward loop is the
-// pivoted blocked sweep kernel (its state after slice n is (Gss, Gs1) =
+// X_n = Z_n - S_n B X_{n+1}, each block M x M.  Here the forward loop is a
+// sweep kernel, symmetric or pivoted (its state after slice n is (Gss, Gs1) =
 // (S_n, Z_n), kept for every slice), and the backward loop runs only on the
 // few source vectors W the caller needs: X_n W for the eigenvectors of t^H t
 // inside a window of T, or one column for the deposition and the
@@ -29,8 +29,8 @@ constexpr int kKC = 8;  // source vectors per CTA of the back-substitution (one 
 // rotations accumulated in V (nv x nv): at convergence A_0 V = A has
 // orthogonal columns, so A_0^H A_0 = V diag(|a_v|^2) V^H.  Both matrices are
 // column-major in per-item global memory owned by this CTA (written and read
-// by its threads only, ordered by __syncthreads).  Same rotation and
-// convergence rule as tt_eigenvalues.  Returns false after 60 sweeps.
+// by its threads only, ordered by __syncthreads).  A pair is rotated while its
+// columns' product exceeds tol of their norms.  Returns false after 60 sweeps.
 __device__ bool jacobi_with_vectors(double2* A, int lda, int L, int nv, double2* V, int* rot) {
   constexpr int NW = kNT / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -340,8 +340,6 @@ __device__ bool svd_with_vectors(double2* A, const int m, const int n, double2* 
   return s_bad == 0;
 }
 
-// One CTA per item: the block of t, Jacobi with vectors, eigenvalues in
-// descending order with their eigenvectors, then the window selection.
 __host__ __device__ inline size_t eigvec_head_bytes(int nc) {
   return (sizeof(double) * nc + sizeof(int) * 2 * nc + 15) & ~(size_t)15;
 }
@@ -353,6 +351,9 @@ __host__ __device__ inline bool eigvec_in_smem(int m, int nc) {
   return eigvec_head_bytes(nc) + eigvec_qr_bytes(m, nc) + sizeof(double2) * ((size_t)m * nc + (size_t)nc * nc) <= 200 * 1024;
 }
 
+// One CTA per item: the block of t, its singular values and right vectors (QR
+// iteration or Jacobi, see launch_eigvec), eigenvalues in descending order with
+// their eigenvectors, then the window selection.
 template <bool QR>
 __global__ void __launch_bounds__(kNT) eigvec_kernel(EigvecArgs a) {
   extern __shared__ double sh[];

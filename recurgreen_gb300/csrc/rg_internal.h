@@ -123,9 +123,10 @@ struct SweepArgs {
   double2* state_dump;        // [nreal][n_end-n_begin][2][M][M] (Gss, Gs1) after every slice, optional
   double2* state_out;         // [nreal][2][M][M] state after slice n_end-1, optional
   int force_large;            // 1: the pivoted blocked kernel even for max_M <= 64 (segment mode with states)
-  // Symmetric sweep (Dirichlet items, periodic ones up to 64 modes): the symmetric kernel (shared-memory
-  // or blocked, by max_M) runs every item and appends those it cannot pivot
-  // stably to flag_list; the pivoted kernel of the same class re-runs them.
+  // Symmetric sweep (Dirichlet items, periodic ones up to 64 modes): the
+  // symmetric kernel (rg_sweep_sym.cu or the blocked one, by max_M) runs every
+  // item and appends those it cannot pivot stably to flag_list; the pivoted
+  // kernel of the same class re-runs them.
   int symmetric;              // 1: symmetric kernel first (needs flag_list)
   int prop_warps;             // set by sweep_sym_plan: the propagator has warps of its own
   int32_t* flag_list;         // [nreal] flagged item indices
@@ -145,15 +146,15 @@ struct SweepArgs {
   // 0 is the usual sweep (source at slice 0, where Z_0 = Gss_0).
   int inject_at;
   // 1: the blocked symmetric kernel forms the propagator product Gss (B Gs1)
-  // on the tensor cores (rg_ozaki.cuh) after inverting X on its own, instead
+  // on the tensor cores (rg_crt.cuh) after inverting X on its own, instead
   // of carrying B Gs1 through the Gauss-Jordan sweep (up to 512 modes).
   // Set from RG_TENSOR_R (default on).
   int tensor_r;
   // With tensor_r, the levels of the 2 x 2 block inverse of X in the blocked
   // symmetric kernel: each halves a size into two half-size inverses and four
-  // half-size tensor-core products; the blocks left are inverted by FP64
-  // Gauss-Jordan sweeps.  3: as many as the kernel's rule takes; 0..2: at most
-  // that many, of even sizes of at least 128.  Set from RG_SPLIT_INVERSE
+  // half-size tensor-core products.  3: down to leaves of at most 32 modes
+  // (rg_tile_inverse.cuh); 0..2: at most that many, of even sizes of at least
+  // 128, the blocks left inverted by FP64 Gauss-Jordan sweeps.  Set from RG_SPLIT_INVERSE
   // (default 3).
   int split_inverse;
 };
@@ -187,8 +188,8 @@ int launch_potential(const PotArgs& a, cudaStream_t stream);
 int sweep_plan(SweepArgs& a, int sm_count, int* grid, int64_t* work_stride);
 int launch_sweep(const SweepArgs& a, cudaStream_t stream, int grid);
 // Symmetric sweep (rg_sweep_sym.cu): complex-symmetric slice matrices
-// (Dirichlet), M <= kMaxModesSmem, diagonal pivoting.  launch_sweep calls it
-// when a.symmetric is set and re-runs the flagged items itself.
+// (Dirichlet, and periodic in real modes), M <= kMaxModesSmem.  launch_sweep
+// calls it when a.symmetric is set and re-runs the flagged items itself.
 int sweep_sym_plan(SweepArgs& a, int sm_count, int* grid, int64_t* work_stride);
 int launch_sweep_sym(const SweepArgs& a, cudaStream_t stream, int grid);
 // The large-mode kernel behind sweep_plan/launch_sweep for max_M > kMaxModesSmem (rg_sweep_large.cu).

@@ -11,7 +11,7 @@
 //                        Gss = inv(A - B Gss B) and Gs1 = -Gss B Gs1
 //                        (src/waveguide.f90:426-440, src/base_utils.f90:235-274),
 //                        Fisher-Lee t (src/waveguide.f90:443-445, :510) and the
-//                        eigenvalues of t^H t by one-sided Jacobi
+//                        eigenvalues of t^H t by bidiagonalisation
 //                        (src/waveguide.f90:448-449, src/base_utils.f90:341-380).
 //   histogram_kernel  -- histogram with the exact edge semantics of
 //                        src/base_utils.f90:491-516.

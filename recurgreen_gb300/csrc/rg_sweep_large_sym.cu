@@ -2,9 +2,8 @@
 //
 // The slice matrix X_n = A_n - V_n - B Gss B of a Dirichlet guide is complex
 // symmetric, so its inverse is formed by a symmetric Gauss-Jordan sweep on
-// the upper triangle (the shared-memory version and its sign rule are in
-// rg_sweep_sym.cu), here blocked for matrices that live in global memory
-// (L2-resident when the batch allows):
+// the upper triangle (the sign rule is that of invert_tile in
+// rg_tile_inverse.cuh), here blocked for matrices that live in global memory:
 //
 //   for each panel of NB diagonal pivots
 //     for each step k of the panel (left-looking)
@@ -27,7 +26,8 @@
 // another ends the update.
 //
 // With tensor_r the sweep inverts X alone, by recursive 2 x 2 blocks
-// (kInvSteps), and then forms the new right-hand side B Gs1 <- X^-1 (B Gs1).
+// (kInvSteps) down to leaves that one CTA inverts in shared memory
+// (rg_tile_inverse.cuh), and then forms the right-hand side B Gs1 <- X^-1 (B Gs1).
 // The products of both run on the FP16 tensor cores with FP64 accuracy in
 // modular arithmetic (rg_crt.cuh, cluster_zgemm): the row exponents of A and
 // column exponents of B are reduced over the cluster, the cluster writes both
@@ -284,11 +284,11 @@ struct ZgemmCtx {
 // read only in the first two phases, so out may overwrite them.  Called by
 // every thread of the cluster; ends with a cluster barrier.  Not inlined: the
 // products of a slice share one copy.
-// Two of the four products of a node take over planes (512 modes 116 -> 112 ms,
-// 152 realizations of 256 modes 212 -> 203): the planes and exponents of an
-// operand that the last product, of the same
+// The planes and exponents of an operand that the last product, of the same
 // Mb, has left are taken over: with have = 1 those of its B, which is this A's
-// transpose, with have = 2 those of its A, which is this B's transpose.
+// transpose, with have = 2 those of its A, which is this B's transpose: two of
+// the eight operands of a node (512 modes 116 -> 112 ms, 152 realizations of
+// 256 modes 212 -> 203).
 __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const Opnd A, const Opnd B,
                                            const TileOut out, const int have) {
   cg::cluster_group cluster = cg::this_cluster();
@@ -1134,7 +1134,7 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
       }
 
       if (gemm_on) {
-        // 4. B Gs1 <- X^-1 (B Gs1) on the tensor cores (rg_ozaki.cuh).
+        // 4. B Gs1 <- X^-1 (B Gs1) on the tensor cores (rg_crt.cuh).
         if (n < a.inject_at) {
           // before the source slice the right-hand side is zero and stays zero
         } else if (n == a.inject_at) {
