@@ -174,6 +174,11 @@ __device__ __forceinline__ bool invert_tile(float2* P, int n, float tau, int lan
   return __any_sync(0xffffffffu, small_pivot);
 }
 
+template <int N>
+struct Int {
+  static constexpr int value = N;
+};
+
 // The shared memory of tile_inverse: the plane regions (12 planes of T^2 x 32
 // uint4 each), [32] maxima, one sum, and two [NCW][16 T] arrays of row
 // exponents by warp column (of X and of Y0; the latter also scale the
@@ -424,15 +429,27 @@ __device__ __forceinline__ bool tile_inverse(const double* x, const int M, const
     for (int h = 0; h < NE / 4; ++h) {
       long long hi[8], lo[8];
       const char* b = bB + offB + 8 * (odd ^ (half | h));
+      // the digits that the levels 0 .. lm take
       if (term == 1) {
-        if (lm <= 4) oz::half_product<T, 5, 3, 4, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 3 * kPlane, kPlane, hi, lo, nullptr, part);
-        else oz::half_product<T, 6, 3, 6, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 3 * kPlane, kPlane, hi, lo, nullptr, part);
-      } else if (lm == 0) {
-        oz::half_product<T, 1, 1, 0, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 6 * kPlane, kPlane, hi, lo, nullptr, part);
-      } else if (lm <= 2) {
-        oz::half_product<T, 3, 3, 2, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 6 * kPlane, kPlane, hi, lo, nullptr, part);
+        if (lm <= 4)
+          oz::half_product<T, 5, 3, 4, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 3 * kPlane, kPlane, hi, lo, nullptr,
+                                           part);
+        else if (lm == 5)
+          oz::half_product<T, 6, 3, 5, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 3 * kPlane, kPlane, hi, lo, nullptr,
+                                           part);
+        else
+          oz::half_product<T, 6, 3, 6, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 3 * kPlane, kPlane, hi, lo, nullptr,
+                                           part);
       } else {
-        oz::half_product<T, 6, 6, 6, NP>(bA + offA0, bA + offA1, 6 * kPlane, b, 6 * kPlane, kPlane, hi, lo, nullptr, part);
+        auto product = [&](auto n, auto lmax) {
+          oz::half_product<T, decltype(n)::value, decltype(n)::value, decltype(lmax)::value, NP>(
+              bA + offA0, bA + offA1, 6 * kPlane, b, 6 * kPlane, kPlane, hi, lo, nullptr, part);
+        };
+        if (lm == 0) product(Int<1>{}, Int<0>{});
+        else if (lm == 1) product(Int<2>{}, Int<1>{});
+        else if (lm == 2) product(Int<3>{}, Int<2>{});
+        else if (lm <= 4) product(Int<5>{}, Int<4>{});
+        else product(Int<6>{}, Int<6>{});
       }
 #pragma unroll
       for (int w = 0; w < 8 / NP; ++w) {
@@ -455,7 +472,7 @@ __device__ __forceinline__ bool tile_inverse(const double* x, const int M, const
     const int bits = 56 - __clz((int)red[term]);  // |E| < 2^bits
     sk = bits - kAccBits;
     lm = levels(sk);
-    oz::put_planes<53, NE, NP>(v, lm == 0 ? 1 : lm <= 2 ? 3 : 6, regB + own, PL, 6, half,
+    oz::put_planes<53, NE, NP>(v, lm <= 2 ? lm + 1 : lm <= 4 ? 5 : 6, regB + own, PL, 6, half,
                                   bits - 53, nullptr, part);
     bar();
   }
