@@ -348,7 +348,8 @@ __host__ __device__ inline size_t eigvec_qr_bytes(int m, int nc) {
   return (sizeof(double) * (size_t)((7 * nc + 1) & ~1) + sizeof(double2) * (size_t)(m + nc) + 15) & ~(size_t)15;
 }
 __host__ __device__ inline bool eigvec_in_smem(int m, int nc) {
-  return eigvec_head_bytes(nc) + eigvec_qr_bytes(m, nc) + sizeof(double2) * ((size_t)m * nc + (size_t)nc * nc) <= 200 * 1024;
+  return eigvec_head_bytes(nc) + eigvec_qr_bytes(m, nc) + sizeof(double2) * ((size_t)m * nc + (size_t)nc * nc) <=
+         200 * 1024;
 }
 
 // One CTA per item: the block of t, its singular values and right vectors (QR
@@ -663,8 +664,8 @@ __global__ void __launch_bounds__(kBackNT, 1) back_tile_kernel(BackArgs a) {
       const char* pa = P + (mat * T * T + rt * T) * 512 + lane * 16;
       long long hi[4], lo[4];
       oz::half_product<T, 6, 6, oz::kLmax, 2>(pa + 8 * odd, pa + 8 * (1 - odd), 6 * kPlane,
-                                              P + 2 * T * T * 512 + lane * 16 + 8 * (odd ^ (1 - mat)), 6 * kPlane, kPlane,
-                                              hi, lo, nullptr, part);
+                                              P + 2 * T * T * 512 + lane * 16 + 8 * (odd ^ (1 - mat)), 6 * kPlane,
+                                              kPlane, hi, lo, nullptr, part);
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         const int v = 2 * t4 + (w & 1);

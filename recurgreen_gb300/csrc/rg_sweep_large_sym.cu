@@ -398,8 +398,8 @@ __device__ __noinline__ void tiny_zgemm(uint4* stage, const Opnd A, const Opnd B
     const char* ca = reinterpret_cast<const char*>(pa) + ti * T * 512 + lane * 16;
     const char* cb = reinterpret_cast<const char*>(pb) + tj * T * 512 + lane * 16;
     long long hi[8], lo[8];
-    oz::half_product<T, 6, 6, oz::kLmax>(ca + 8 * odd, ca + 8 * (1 - odd), 6 * 16 * PL, cb + 8 * (odd ^ half), 6 * 16 * PL,
-                                         16 * PL, hi, lo);
+    oz::half_product<T, 6, 6, oz::kLmax>(ca + 8 * odd, ca + 8 * (1 - odd), 6 * 16 * PL, cb + 8 * (odd ^ half),
+                                         6 * 16 * PL, 16 * PL, hi, lo);
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       const int i = r0 + 8 * (w >> 1), j = c0 + (w & 1);

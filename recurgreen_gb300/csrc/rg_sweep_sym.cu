@@ -29,16 +29,16 @@
 // error of t against an extended-precision sweep is that of the elimination
 // within 0.95 to 1.3 (7 to 64 modes, 40 to 300 slices; geometric mean 1.08).
 // Measured, with the eigenvalues: 304 guides of 64 modes and 600 slices 607 ms
-// before, 184 now; 500 of 37 modes and 150 slices 110 ms before, 41 now; one
-// guide of 10 modes and 200 slices 8.2 ms before, 2.1 now.
+// before, 187 now; 500 of 37 modes and 150 slices 110 ms before, 44 now; one
+// guide of 10 modes and 200 slices 8.2 ms before, 2.0 now.
 //
 // Layout: T = ceil(M/16) tiles a side, one warp per tile or two, as in
 // rg_tile_inverse.cuh.  (Q is kept transposed so that it is only ever an A
 // operand.)  Its plane regions are reused through the slice:
 //   region A: X' -> R -> G';   region B: Y0 -> E_k -> Q.
 // Q, G' and the scaling products w_i w_j stay with their owner lanes, in the
-// CTA's workspace (L2).  At 33 to 48 modes two CTAs fit on an SM, at 49 to
-// 64 one.
+// CTA's workspace (L2).  Above 32 modes the registers of one CTA fill an SM (at 48
+// modes a warp per tile and two CTAs of 80 registers took the same time).
 //
 // If a pivot is too small against the unswept entries of its row (sym_tau),
 // or the residual is not small, the item is flagged (kStatusNeedPivot), its
@@ -49,7 +49,9 @@
 namespace rg {
 namespace {
 
-__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_sync(int id, int n) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
 __device__ __forceinline__ void bar_arrive(int id, int n) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
 }
@@ -167,7 +169,8 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
   double2* ws = a.work + (int64_t)blockIdx.x * a.work_stride;
   uint64_t* gen = (uint64_t*)ws;               // [max_ny][4]
   double* urow = (double*)(ws + 2 * (int64_t)a.max_ny);  // [max_ny] potential row
-  double2* Qs = ws + 2 * (int64_t)a.max_ny + (a.max_ny + 1) / 2 + (main_thread || prop_thread ? warp * 32 * NE + lane : 0);
+  double2* Qs = ws + 2 * (int64_t)a.max_ny + (a.max_ny + 1) / 2;
+  if (main_thread || prop_thread) Qs += warp * 32 * NE + lane;
   double2* Gs = Qs + T * T * 256;              // entry k of this lane at [32 k]
   double2* Ww = Gs + T * T * 256;
   // This lane's place in the planes: its tile, and the word pairs of its tile
@@ -470,9 +473,10 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
         if (hand_on) {
           if (n >= 2) bar_sync(kBarGFree + b, NMAIN + NPROP);
 #pragma unroll
-          for (int k = 0; k < NV; ++k)
-            reinterpret_cast<double*>(gbuf + (b * (NPROP / 32) + warp) * 32 * NE + 32 * (k % NE) + lane)[k < NE ? part : 1] =
-                gd[k];
+          for (int k = 0; k < NV; ++k) {
+            double2* d = gbuf + (b * (NPROP / 32) + warp) * 32 * NE + 32 * (k % NE) + lane;
+            reinterpret_cast<double*>(d)[k < NE ? part : 1] = gd[k];
+          }
           if (tj == 0 && half == 0 && part == 0 && t4 == 0) {
             eybuf[b * MP + r0] = ey0;
             eybuf[b * MP + r0 + 8] = ey1;
@@ -511,7 +515,8 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
             for (int w = 0; w < 4; ++w) {
               const int k = 4 * h + w;
               const int e = (erow(k) ? eq1 : eq0) + oz::row_exp<NCW>(exY, MP, c0 + ecol(k));
-              Qs[32 * k] = make_double2(-oz::fold_to_double(hi[w], lo[w], e), -oz::fold_to_double(hi[4 + w], lo[4 + w], e));
+              Qs[32 * k] =
+                  make_double2(-oz::fold_to_double(hi[w], lo[w], e), -oz::fold_to_double(hi[4 + w], lo[4 + w], e));
             }
           }
         } else if (!PROP && !refl) {
@@ -658,7 +663,8 @@ int sweep_sym_plan(SweepArgs& a, int sm_count, int* grid, int64_t* work_stride) 
 int launch_sweep_sym(const SweepArgs& a, cudaStream_t stream, int grid) {
   if (a.nreal <= 0) return RG_OK;
   if (a.max_M <= 16) return launch_sym_t<1, true>(a, stream, grid);
-  if (a.max_M <= 32) return a.prop_warps ? launch_sym_t<2, true>(a, stream, grid) : launch_sym_t<2, false>(a, stream, grid);
+  if (a.max_M <= 32)
+    return a.prop_warps ? launch_sym_t<2, true>(a, stream, grid) : launch_sym_t<2, false>(a, stream, grid);
   if (a.max_M <= 48) return launch_sym_t<3, false>(a, stream, grid);
   return launch_sym_t<4, false>(a, stream, grid);
 }
