@@ -103,7 +103,7 @@ __device__ bool jacobi_with_vectors(double2* A, int lda, int L, int nv, double2*
 // 4 doubles and 2 m double2 of shared memory.  Warp 0 runs the rotations of a
 // sweep, a serial chain, while the other warps apply those of the sweep before.
 // As accurate as the reference's zgesvd: absolutely, to the norm of A.
-// Returns false when the iteration does not end.
+// Returns false when the iteration does not end or A is not finite (then d is NaN).
 __device__ bool svd_with_vectors(double2* A, const int m, const int n, double2* V, double* sc) {
   constexpr int NW = kNT / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -199,7 +199,7 @@ __device__ bool svd_with_vectors(double2* A, const int m, const int n, double2* 
   if (!finite) {
     for (int i = tid; i < n; i += kNT) d[i] = NAN;
     __syncthreads();
-    return true;
+    return false;
   }
   const double eps = 0x1p-53, tiny = 0x1p-56 * norm;
   // (c, s) with [c s; -s c] (f, g) = (r, 0)
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kNT) eigvec_kernel(EigvecArgs a) {
   extern __shared__ double sh[];
   double* tv = sh;                        // [nc] |a_v|^2 by column
   int* order = (int*)(tv + a.nc);         // [nc] column of rank k
-  int* rankof = order + a.nc;             // [nc] rank of column v
+  int* selcol = order + a.nc;             // [nc] column of selected vector k
   __shared__ int s_rot, s_k;
   const int r = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -397,14 +397,12 @@ __global__ void __launch_bounds__(kNT) eigvec_kernel(EigvecArgs a) {
   }
   __syncthreads();
   for (int v = tid; v < nc; v += kNT) {
-    const double t = tv[v];
-    int k = 0;
-    for (int j = 0; j < nc; ++j) k += (tv[j] > t || (tv[j] == t && j < v)) ? 1 : 0;
+    const int k = descending_rank(tv, nc, v);
     order[k] = v;
-    rankof[v] = k;
-    a.tvals[(int64_t)r * nc + k] = t;
+    a.tvals[(int64_t)r * nc + k] = tv[v];
+    ok = ok && tv[v] < INFINITY;
   }
-  __syncthreads();
+  ok = __syncthreads_and(ok) != 0;  // no decomposition of a matrix that is not finite
   if (a.u) {
     double2* u = a.u + (int64_t)r * nc * nc;
     for (int64_t e = tid; e < (int64_t)nc * nc; e += kNT) {
@@ -431,7 +429,7 @@ __global__ void __launch_bounds__(kNT) eigvec_kernel(EigvecArgs a) {
         }
         if (bits) {
           a.member[(int64_t)r * nc + k] = bits;
-          rankof[k] = order[q];  // reused: column of selected vector k
+          selcol[k] = order[q];
           ++k;
         }
       }
@@ -445,7 +443,7 @@ __global__ void __launch_bounds__(kNT) eigvec_kernel(EigvecArgs a) {
     for (int64_t e = tid; e < (int64_t)k * a.M; e += kNT) {
       const int s = (int)(e / a.M), m = (int)(e % a.M);
       const int j = m - a.col0;
-      ws[e] = (j >= 0 && j < nc) ? cmul(a.sqmu[m], V[(int64_t)rankof[s] * nc + j]) : make_double2(0.0, 0.0);
+      ws[e] = (j >= 0 && j < nc) ? cmul(a.sqmu[m], V[(int64_t)selcol[s] * nc + j]) : make_double2(0.0, 0.0);
     }
   }
   if (tid == 0) a.status[r] = ok ? RG_OK : RG_ERR_NOCONV;

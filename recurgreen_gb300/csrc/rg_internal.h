@@ -36,6 +36,16 @@ inline cudaError_t allow_smem(const void* kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Position of value v among the n values t in descending order, ties by index
+// and NaN last: a permutation whatever the values, so that what is stored by
+// it leaves no slot unset.
+__host__ __device__ inline int descending_rank(const double* t, int n, int v) {
+  const double x = t[v];
+  int k = 0;
+  for (int j = 0; j < n; ++j) k += (x != x ? t[j] == t[j] || j < v : t[j] > x || (t[j] == x && j < v)) ? 1 : 0;
+  return k;
+}
+
 // Switches to a handle's device for the duration of a call.
 struct DeviceGuard {
   int prev = -1;

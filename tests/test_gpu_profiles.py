@@ -33,3 +33,11 @@ def test_profiles_at_kernel_edges(bt, m):
     po, nto = o.tprofile_upot(u, lo, hi)
     assert nt == nto
     assert np.linalg.norm(p - po) <= 1e-9 * max(np.linalg.norm(po), 1.0)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_a_matrix_that_is_not_finite_has_no_decomposition(bad):
+    a = np.ones((5, 4), complex)
+    a[2, 1] = bad
+    with pytest.raises(rg.RecurGreenError):
+        rg.diagonalize_ahca(a)
