@@ -77,6 +77,22 @@ __device__ __forceinline__ void cluster_tt_eigenvalues(int C, const int rank, do
     for (int i = tid; i < L; i += NT) x[i] = i == 0 ? make_double2(1.0, 0.0) : cmul(x[i], sc);
     __syncthreads();
   };
+  __shared__ int s_top;
+  if (tid == 0) s_top = 0;
+  __syncthreads();
+  int top = 0;
+#pragma unroll 4
+  for (int64_t q = tid; q < (int64_t)m * n; q += NT) top = max(top, biased_exp(__ldcg(A + q)));
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) atomicMax(&s_top, top);
+  __syncthreads();
+  double unscale;
+  const double scale = range_scale(s_top, &unscale);
+  if (scale != 1.0) {
+    sync();  // every CTA has read A
+    for (int64_t q = rank * NT + tid; q < (int64_t)m * n; q += C * NT) A[q] = cscale(scale, __ldcg(A + q));
+    sync();
+  }
   for (int i = tid; i < m; i += NT) z[i] = make_double2(0.0, 0.0);
   for (int j = tid; j < n; j += NT) u[j] = make_double2(0.0, 0.0);
   double2 tr = make_double2(0.0, 0.0);  // conj(tau') of the step before
@@ -181,7 +197,7 @@ __device__ __forceinline__ void cluster_tt_eigenvalues(int C, const int rank, do
     }
     sync();
   }
-  bidiag_values<NT>(d, e, n, neig, out, rank, C);
+  bidiag_values<NT>(d, e, n, neig, out, unscale, rank, C);
 }
 
 }  // namespace rg

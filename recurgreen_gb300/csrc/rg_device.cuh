@@ -105,6 +105,22 @@ __device__ __forceinline__ double fast_rcp(double x) {
   return fma(y, fma(-x, y, 1.0), y);
 }
 
+// The reductions below square entries, so a matrix is brought to order 1 when
+// its largest entry lies outside 2^-300 .. 2^300 (t of a strongly absorbing guide
+// comes down to 1e-300).  Powers of two: the singular values scale exactly.
+// Biased exponent of the larger part of x:
+__device__ __forceinline__ int biased_exp(double2 x) {
+  const int a = (__double2hiint(x.x) >> 20) & 0x7ff, b = (__double2hiint(x.y) >> 20) & 0x7ff;
+  return a > b ? a : b;
+}
+// The factor for a matrix whose entries have exponents up to e, and the one that
+// undoes it; 1 where no scaling is needed.
+__device__ __forceinline__ double range_scale(int e, double* undo) {
+  const bool on = e > 0 && (e < 1023 - 300 || e > 1023 + 300) && e < 2046;
+  *undo = on ? __longlong_as_double((long long)e << 52) : 1.0;
+  return on ? __longlong_as_double((long long)(2046 - e) << 52) : 1.0;
+}
+
 // Reflection of a complex vector x (first element a, squared norm xn2 of the
 // others): (I - tau v v^H) x = beta e_1 with v = (1, x[1:] * scale), beta real.
 struct Reflector {
@@ -113,12 +129,14 @@ struct Reflector {
 };
 __device__ __forceinline__ Reflector reflector(double2 a, double xn2) {
   Reflector r;
-  if (xn2 == 0.0 && a.y == 0.0) {
-    r.beta = a.x;
+  const double n2 = fma(a.x, a.x, fma(a.y, a.y, xn2));
+  // (below 1e-145 of a matrix of order 1: zero, whose square would underflow)
+  if ((xn2 == 0.0 && a.y == 0.0) || n2 < 1e-290) {
+    r.beta = n2 < 1e-290 ? 0.0 : a.x;
     r.tau = r.scale = make_double2(0.0, 0.0);
     return r;
   }
-  r.beta = -copysign(sqrt(fma(a.x, a.x, fma(a.y, a.y, xn2))), a.x);
+  r.beta = -copysign(sqrt(n2), a.x);
   const double rb = 1.0 / r.beta;
   r.tau = make_double2((r.beta - a.x) * rb, a.y * rb);
   const double dx = a.x - r.beta;  // no cancellation: beta has the sign opposite to a.x
@@ -146,10 +164,11 @@ __device__ __forceinline__ int bidiag_count(const double* dd, const double* ee, 
 // (shared memory; squared in place), descending, to out.  Bisection on sigma
 // down to 2^-54 of its bound, so every value has the absolute accuracy of the
 // reduction; a warp's lanes share out its values, S lanes cutting an interval
-// into S + 1 parts.  Called by NT threads of one CTA, or by CTA `rank` of
-// `parts` (then S = 1: the bits of a value do not depend on the sharing).
+// into S + 1 parts; `unscale` multiplies the singular values.  Called by NT threads of one CTA, or by CTA
+// `rank` of `parts` (then S = 1: the bits of a value do not depend on the sharing).
 template <int NT>
-__device__ void bidiag_values(double* d, double* e, int n, int neig, double* out, int rank = 0, int parts = 0) {
+__device__ void bidiag_values(double* d, double* e, int n, int neig, double* out, double unscale, int rank = 0,
+                              int parts = 0) {
   constexpr int NW = NT / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __syncthreads();
@@ -203,7 +222,7 @@ __device__ void bidiag_values(double* d, double* e, int n, int neig, double* out
       if (f > 0) lo = fma(w, f * rs, base);
     }
     if (on && s == 0) {
-      const double x = 0.5 * (lo + hi);
+      const double x = 0.5 * (lo + hi) * unscale;
       out[j0 + k] = x * x;
     }
   }
@@ -266,6 +285,23 @@ __device__ void tt_eigenvalues(double2* W, int LDW, int nrow, int ncol, int neig
       x[i * st] = make_double2(fma(-w.x, q.x, fma(sg * w.y, q.y, u.x)), fma(-w.x, sg * q.y, fma(-w.y, q.x, u.y)));
     }
   };
+  __shared__ int s_top;
+  if (threadIdx.x == 0) s_top = 0;
+  __syncthreads();
+  int top = 0;
+  for (int q = threadIdx.x; q < nrow * ncol; q += NT) top = max(top, biased_exp(W[(q / ncol) * LDW + q % ncol]));
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) atomicMax(&s_top, top);
+  __syncthreads();
+  double unscale;
+  const double scale = range_scale(s_top, &unscale);
+  if (scale != 1.0) {
+    for (int q = threadIdx.x; q < nrow * ncol; q += NT) {
+      double2* x = W + (q / ncol) * LDW + q % ncol;
+      *x = cscale(scale, *x);
+    }
+    __syncthreads();
+  }
   for (int k = 0; k < n; ++k) {
     if (warp == 0) reflect(W + k * rs + k * cs, rs, m - k, 1.0, d + k);
     __syncthreads();
@@ -278,7 +314,7 @@ __device__ void tt_eigenvalues(double2* W, int LDW, int nrow, int ncol, int neig
     for (int i = k + 1 + warp; i < m; i += NW) apply(W + i * rs + (k + 1) * cs, cs, n - k - 1, tc, -1.0);
     __syncthreads();
   }
-  bidiag_values<NT>(d, e, n, min(neigv, n), out);
+  bidiag_values<NT>(d, e, n, min(neigv, n), out, unscale);
 }
 
 }  // namespace rg

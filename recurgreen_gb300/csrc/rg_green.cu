@@ -155,7 +155,20 @@ __device__ bool svd_with_vectors(double2* A, const int m, const int n, double2* 
           make_double2(fma(-w.x, q.x, fma(sg * w.y, q.y, u.x)), fma(-w.x, sg * q.y, fma(-w.y, q.x, u.y)));
     }
   };
+  __shared__ int s_top;
+  if (tid == 0) s_top = 0;
   __syncthreads();
+  int top = 0;
+  for (int64_t q = tid; q < (int64_t)m * n; q += kNT) top = max(top, biased_exp(A[q]));
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) atomicMax(&s_top, top);
+  __syncthreads();
+  double unscale;
+  const double scale = range_scale(s_top, &unscale);
+  if (scale != 1.0) {
+    for (int64_t q = tid; q < (int64_t)m * n; q += kNT) A[q] = cscale(scale, A[q]);
+    __syncthreads();
+  }
   for (int k = 0; k < n; ++k) {
     double2* akk = A + (int64_t)k * m + k;
     if (warp == 0) reflect(akk, 1, m - k, 1.0, d + k);
@@ -337,6 +350,8 @@ __device__ bool svd_with_vectors(double2* A, const int m, const int n, double2* 
     __syncthreads();
     // (s_count[b] is zero after the last sweep, so the loop ends one pass later)
   }
+  for (int i = tid; i < n; i += kNT) d[i] *= unscale;
+  __syncthreads();
   return s_bad == 0;
 }
 
