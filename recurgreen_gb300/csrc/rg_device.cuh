@@ -161,9 +161,8 @@ __device__ __forceinline__ int bidiag_count(const double* dd, const double* ee, 
 }
 
 // The largest neig squared singular values of the bidiagonal d[n], e[n - 1]
-// (shared memory; squared in place), descending, to out.  Bisection on sigma
-// down to 2^-54 of its bound, so every value has the absolute accuracy of the
-// reduction; a warp's lanes share out its values, S lanes cutting an interval
+// (shared memory; squared in place), descending, to out.  Bisection on sigma,
+// down to 2^-52 of the value itself; a warp's lanes share out its values, S lanes cutting an interval
 // into S + 1 parts; `unscale` multiplies the singular values.  Called by NT threads of one CTA, or by CTA
 // `rank` of `parts` (then S = 1: the bits of a value do not depend on the sharing).
 template <int NT>
@@ -201,22 +200,39 @@ __device__ void bidiag_values(double* d, double* e, int n, int neig, double* out
   const int wn = min(NW, max(4, (cnt + 31) / 32));
   if (warp >= wn) return;
   const int per = (cnt + wn - 1) / wn;           // values of a warp
-  const double tiny = fmax(1e-40 * top, 1e-300);
+  const double tiny = fmax(1e-120 * top, 1e-300);  // (its reciprocal times two squares is finite)
   for (int v0 = 0; v0 < per; v0 += 32) {
     const int here = min(32, per - v0), S = parts ? 1 : 32 / here;
     const int grp = lane / S, s = lane % S;
     const int k = warp * per + v0 + grp;          // position among this sharer's values
     const bool on = grp < here && k < cnt;
     const int want = n - 1 - (j0 + k);            // the value has this many below it
-    double lo = 0.0, hi = bound;
+    const unsigned mask = S == 32 ? ~0u : (1u << S) - 1u;
+    // the first of a group's S cuts, falling or rising, that `hit`s
+    auto first = [&](bool hit) {
+      const unsigned b = (__ballot_sync(0xffffffffu, hit) >> (grp * S)) & mask;
+      return b ? __ffs(b) - 1 : S;
+    };
+    // Its octave first, bound 2^-p1 .. bound 2^-p0: the bidiagonal gives a small
+    // value to as many digits as a large one, and so does t where modes hardly
+    // mix (a clean absorbing guide).  (54 halvings of 0 .. bound took 1 % less of
+    // 256 modes and lost the small ones.)
+    int p0 = 0, p1 = 192;  // (zero below)
+    while (__any_sync(0xffffffffu, on && p1 - p0 > 1)) {
+      const bool go = on && p1 - p0 > 1;
+      const int p = p0 + (p1 - p0) * (s + 1) / (S + 1);
+      const double x = bound * __longlong_as_double((long long)(1023 - p) << 52);
+      const int f = first(go && bidiag_count(d, e, n, x * x, tiny) <= want), lo0 = p0, w = p1 - p0;
+      if (go && f < S) p1 = lo0 + w * (f + 1) / (S + 1);
+      if (go && f > 0) p0 = lo0 + w * f / (S + 1);
+    }
+    double hi = bound * __longlong_as_double((long long)(1023 - p0) << 52), lo = p1 == 192 ? 0.0 : 0.5 * hi;
     const double rs = 1.0 / (S + 1);
-    // 54 halvings, or as many cuts into S + 1 parts as shrink the interval alike
-    const int steps = (int)ceilf(54.0f / log2f((float)(S + 1)));
+    // 52 halvings, or as many cuts into S + 1 parts as shrink the interval alike
+    const int steps = (int)ceilf(52.0f / log2f((float)(S + 1)));
     for (int it = 0; it < steps; ++it) {
       const double x = fma(hi - lo, (s + 1) * rs, lo);
-      const bool above = on ? bidiag_count(d, e, n, x * x, tiny) > want : true;
-      const unsigned b = (__ballot_sync(0xffffffffu, above) >> (grp * S)) & (S == 32 ? ~0u : (1u << S) - 1u);
-      const int f = b ? __ffs(b) - 1 : S;         // the first cut above the value
+      const int f = first(on ? bidiag_count(d, e, n, x * x, tiny) > want : true);  // the first cut above the value
       const double w = hi - lo, base = lo;
       if (f < S) hi = fma(w, (f + 1) * rs, base);
       if (f > 0) lo = fma(w, f * rs, base);
@@ -235,7 +251,7 @@ __device__ void bidiag_values(double* d, double* e, int n, int neig, double* out
 //
 // Householder reflections from both sides make t real bidiagonal (8/3 n^3
 // complex multiply-adds) and bisection gives the values, as accurate as the
-// reference's zgesvd (absolutely, to the norm of t).  One-sided Jacobi took
+// reference's zgesvd (absolutely, to the norm of t, where modes mix).  One-sided Jacobi took
 // nine sweeps of 4 n^3 on the same FP64 pipe: 57 M clocks for 64 x 64.
 template <int NT>
 __device__ void tt_eigenvalues(double2* W, int LDW, int nrow, int ncol, int neigv, double* sc, double* out) {

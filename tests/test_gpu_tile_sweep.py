@@ -115,3 +115,17 @@ def test_transmission_of_strongly_absorbing_guides(m, nabs):
     assert np.all(np.abs(T - want) <= 1e-10 * want + 1e-300)
     p, nt = g.compute_tprofile(1, 0.0, 0.1)
     assert nt == m and np.all(np.isfinite(p))
+
+
+@pytest.mark.parametrize("m,dabso", [(40, 700.0), (70, 700.0), (100, 400.0), (33, 300.0)])
+def test_small_transmissions_of_clean_guides_keep_their_digits(m, dabso):
+    """Where modes do not mix, every T has the relative accuracy of its own mode, however much smaller than the
+    largest it is (here by up to 1e-63; nx slices of M-term sums: below 1e-10)."""
+    nx = 40
+    wol = (m + 0.5) / 2
+    kl = 2 * np.pi * wol
+    mu = np.sqrt(1 - (0.5 * np.arange(1, m + 1) / wol) ** 2 + 1j * dabso / kl)
+    want = np.sort(np.exp(-2 * mu.imag * kl * (nx - 1) / nx))[::-1]
+    T = np.asarray(rg.Waveguide(**dict(guide(m, m, nx, nxfree=0, dabso=dabso), dscat=0.0)).tdistrib_batch(
+        np.array([1], np.int32))).ravel()
+    assert np.all(np.abs(T - want) <= 1e-10 * want)
