@@ -181,12 +181,6 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
   return r;
 }
 
-// x 2^(53-e) rounded to nearest, with sign (|x| < 2^e).
-__device__ __forceinline__ long long fixed(double x, int e) {
-  const long long m = (long long)oz::fixed53(x, e);
-  return x < 0.0 ? -m : m;
-}
-
 __device__ __forceinline__ uint32_t sub_half2(uint32_t a, uint32_t b) {
   __half2 x, y;
   memcpy(&x, &a, 4);
@@ -237,7 +231,7 @@ __device__ __forceinline__ void split(int M, Get get, const int* ex, uint4* dig,
       const int r = r0 + 8 * ((k >> 1) & 1), c = k0 + (k & 1) + 8 * (k >> 2);
       const double2 v = r < M && c < M ? get(r, c) : make_double2(0.0, 0.0);
       const int e = r < M ? ex[r] : 0;
-      const long long x = fixed(v.x, e), y = fixed(v.y, e);
+      const long long x = oz::sfixed53(v.x, e), y = oz::sfixed53(v.y, e);
       st[lane * 10 + k] = make_uint4((uint32_t)x & 0x7ffffffu, (uint32_t)(x >> 27), (uint32_t)y & 0x7ffffffu,
                                      (uint32_t)(y >> 27));
     }

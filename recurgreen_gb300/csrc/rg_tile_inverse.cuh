@@ -397,7 +397,7 @@ __device__ __forceinline__ bool tile_inverse(const double* x, const int M, const
         const unsigned long long q = min(av >> 36, 1ULL << 26);
         sq += q * q;
       }
-      v[(w < 4 ? 0 : NE) + k] = y;
+      v[(w < 4 ? 0 : NE) + k] = i < M && j < M ? 2 * y - 1 : 0;  // (fix_shift truncates: half a unit taken back)
     }
   }
   mx = __reduce_max_sync(0xffffffffu, mx);
@@ -419,7 +419,7 @@ __device__ __forceinline__ bool tile_inverse(const double* x, const int M, const
   auto levels = [&](int s) { return max(0, min(oz::kLmax, (62 + er + s + 8) / 9 - 1)); };
   // E_1 = R Y0, E_k+1 = R E_k; the sum starts from Y0.
   int lm = levels(0);
-  oz::put_planes<53, NE, NP>(v, 6, regA + own, PL, 6, half, 9 + er, nullptr, part);
+  oz::put_planes<53, NE, NP>(v, 6, regA + own, PL, 6, half, 10 + er, nullptr, part);
   bar();
   float rk = rn;  // ||R||^k of the term just formed
   int sk = 0;     // the B operand's entries are below 2^(e_i + sk)
