@@ -451,8 +451,9 @@ __device__ __noinline__ bool leaf_inverse(double2* P, const int n, const float t
   if (tid == 0) s_flag = RG_OK;
   __syncthreads();  // the staging area's previous contents have been used
   int ey0, ey1;
-  const bool ok = tile_inverse<T, NE>(x, n, tau, ts, &s_flag, [] { __syncthreads(); }, [] {}, gd, ey0, ey1);
+  bool ok = tile_inverse<T, NE>(x, n, tau, ts, &s_flag, &s_flag, [] { __syncthreads(); }, [] {}, gd, ey0, ey1);
   if (cluster.num_blocks() > 1) cluster.sync();  // every CTA has read P
+  ok = ok && s_flag == RG_OK;
   if (ok && cluster.block_rank() == 0) {
 #pragma unroll
     for (int k = 0; k < NE; ++k) {

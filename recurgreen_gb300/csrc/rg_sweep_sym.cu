@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
           }
           oz::put_row_exps(exQ + (tj * NHALF + half) * MP, ti, lane, eq0, eq1);
         };
-        if (!tile_inverse<T, NE, NP>(x, M, tau, ts, &s_status, mbar, q_exps, gd, ey0, ey1)) {
+        if (!tile_inverse<T, NE, NP>(x, M, tau, ts, &s_status, &s_status, mbar, q_exps, gd, ey0, ey1)) {
           aborted = true;
           if (hand_on) {
             if (n >= 2) bar_sync(kBarGFree + b, NMAIN + NPROP);

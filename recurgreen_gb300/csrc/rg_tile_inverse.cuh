@@ -194,17 +194,20 @@ struct TileSmem {
 
 // x: this lane's entries of X (zero outside M x M), NE = 8 of a whole tile or
 // 4 of its column half, real parts, then imaginary parts; gd: its entries of
-// X^-1, exactly symmetric; ey0, ey1: the exponents of rows g and g + 8 (|gd| <
-// 2^(ey+1)).  With NP = 2 (T = 1) a lane has one part of its entries, real in
+// X^-1, exactly symmetric; ey0, ey1: the exponents of rows g and g + 8 (|gd| <=
+// 2^ey (1 + 2^-9)).  With NP = 2 (T = 1) a lane has one part of its entries, real in
 // even warps and imaginary in odd ones: half the instructions in each of twice
 // the warps.  Called by the T^2 8/NE NP warps 0, 1, ... of the CTA; bar() is a barrier of theirs, and pre() is run
 // before the last but one.  Returns false, in every thread, when a pivot falls
 // below tau times the largest unswept entry of its row (in its tile) or the
 // residual is not small; *flag (shared, zero before, kStatusNeedPivot after)
-// says so too.
+// says so too.  *late becomes kStatusNeedPivot before the last barrier when the
+// result is useless because an entry of a term or of the inverse does not fit the
+// fixed point that Y0 gave its row (the caller looks at it after the last slice: a
+// read here would lengthen every slice by a barrier's latency).
 template <int T, int NE, int NP = 1, class Bar, class Pre>
 __device__ __forceinline__ bool tile_inverse(const double* x, const int M, const float tau, const TileSmem& s,
-                                             volatile int* flag, Bar bar, Pre pre, double* gd, int& ey0, int& ey1) {
+                                             volatile int* flag, volatile int* late, Bar bar, Pre pre, double* gd, int& ey0, int& ey1) {
   static_assert(NP == 1 || T == 1, "a part each only for one tile");
   constexpr int MP = 16 * T, NV = 2 * NE / NP, NHALF = 8 / NE, NCW = T * NHALF * NP, PL = T * T * 32, LDW = MP + 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) / NP, part = NP == 2 ? (tid >> 5) & 1 : 0;
@@ -421,6 +424,9 @@ __device__ __forceinline__ bool tile_inverse(const double* x, const int M, const
   int lm = levels(0);
   oz::put_planes<53, NE, NP>(v, 6, regA + own, PL, 6, half, 10 + er, nullptr, part);
   bar();
+  bool bad = false;  // an entry does not fit its row's fixed point
+  // rows' exponents, those of the padding (where all is zero) out of the way
+  const int eu0 = r0 < M ? ey0 : 1 << 14, eu1 = r0 + 8 < M ? ey1 : 1 << 14;
   float rk = rn;  // ||R||^k of the term just formed
   int sk = 0;     // the B operand's entries are below 2^(e_i + sk)
   for (int term = 1;; ++term) {
@@ -451,14 +457,27 @@ __device__ __forceinline__ bool tile_inverse(const double* x, const int M, const
         else if (lm <= 4) product(Int<5>{}, Int<4>{});
         else product(Int<6>{}, Int<6>{});
       }
+      int e[4], top = oz::kNoExp;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        e[w] = er + sk + oz::row_exp<NCW>(exY, MP, c0 + ecol(4 * h + w)) - (erow(w) ? eu1 : eu0);
+        top = max(top, e[w]);
+      }
+      // However small ||R|| is, R Y0 brings entries of a large row of Y0 to a
+      // small one: |E| must stay below 2^4 of the row's power of two.  It does
+      // where e < -8, as |hi| < 2^46; else every entry is looked at (for one tile
+      // always: there the latency of a branch costs more than its instructions).
+      if (T == 1 || top >= -8) {
+#pragma unroll
+        for (int w = 0; w < 8 / NP; ++w)
+          bad |= (unsigned long long)(((hi[w] + (lo[w] >> 36)) >> min(max(94 - kAccBits - e[w & 3], 0), 63)) + 1) > 1;
+      }
 #pragma unroll
       for (int w = 0; w < 8 / NP; ++w) {
-        const int k = 4 * h + (w & 3);
-        const int e = oz::row_exp<NCW>(exY, MP, c0 + ecol(k)) - (erow(k) ? ey1 : ey0);
         // rounded: truncating, a bias of 2^-57 in every entry, is an
         // error of M 2^-57 in norm that adds up from slice to slice
-        const long long y = (oz::fix_shift(hi[w], lo[w], kAccBits - 33 + er + sk + e) + 1) >> 1;
-        const int q = (w < 4 ? 0 : NE) + k;
+        const long long y = (oz::fix_shift(hi[w], lo[w], kAccBits - 33 + e[w & 3]) + 1) >> 1;
+        const int q = (w < 4 ? 0 : NE) + 4 * h + (w & 3);
         acc[q] += y;
         v[q] = y;
         mx = max(mx, (unsigned)((unsigned long long)(y < 0 ? -y : y) >> 24));
@@ -483,6 +502,8 @@ __device__ __forceinline__ bool tile_inverse(const double* x, const int M, const
   // to the rounding of the two halves, its asymmetry grew along the
   // guide and tripled the error of t.
   double* gb = (double*)regB;  // [MP][LDW] complex
+  constexpr int kTop = (1 << (kAccBits - 32)) + (1 << (kAccBits - 41));
+  unsigned most = 0;
 #pragma unroll
   for (int k = 0; k < NE; ++k) {
     const int e = (erow(k) ? ey1 : ey0) - kAccBits;
@@ -490,9 +511,12 @@ __device__ __forceinline__ bool tile_inverse(const double* x, const int M, const
 #pragma unroll
     for (int q = k; q < NV; q += NE) {
       gd[q] = oz::fix_to_double(acc[q], e);
+      // the callers' digits hold entries of a row up to 2^ey (1 + 2^-8)
+      most = max(most, (unsigned)((int)(acc[q] >> 32) + kTop));
       if (i < j) gb[2 * (i * LDW + j) + (q < NE ? part : 1)] = gd[q];
     }
   }
+  if (bad || most > 2u * kTop) *late = kStatusNeedPivot;
   bar();
 #pragma unroll
   for (int k = 0; k < NE; ++k) {

@@ -129,3 +129,20 @@ def test_small_transmissions_of_clean_guides_keep_their_digits(m, dabso):
     T = np.asarray(rg.Waveguide(**dict(guide(m, m, nx, nxfree=0, dabso=dabso), dscat=0.0)).tdistrib_batch(
         np.array([1], np.int32))).ravel()
     assert np.all(np.abs(T - want) <= 1e-10 * want)
+
+
+@pytest.mark.parametrize("bt,m,nx,dscat,seeds", [
+    ("dirichlet", 20, 60, 20.0, (4035, 5037, 5194)), ("dirichlet", 20, 60, 30.0, (769, 1121, 1472)),
+    ("dirichlet", 20, 60, 100.0, (2643, 2666)), ("periodic", 19, 60, 30.0, (68, 1836, 4053)),
+    ("periodic", 19, 60, 50.0, (3880, 4274, 4640)), ("dirichlet", 32, 60, 30.0, (1908, 2396)),
+    ("periodic", 31, 60, 20.0, (630,)), ("dirichlet", 40, 40, 100.0, (1644, 2022)), ("periodic", 39, 40, 60.0, (550, 856)),
+    ("dirichlet", 64, 30, 100.0, (22, 1272, 1464)), ("periodic", 63, 30, 100.0, (593,))])
+def test_inverses_with_rows_of_very_different_size(bt, m, nx, dscat, seeds):
+    """Strong disorder: realizations in which some slice's inverse has entries beyond what the fixed point of their row
+    holds (found among thousands by comparison with the pivoted kernel; they gave T up to 7000)."""
+    kw = dict(boundtype=bt, nxdiso=nx, nxfree=0, wol=(m + 0.5) / 2 if bt == "dirichlet" else m // 2 + 0.45, exfac=1.0,
+              aratio=1.0, dscat=dscat, ny=m + 2)
+    o, g = O.Waveguide(**kw), rg.Waveguide(**kw)
+    T = g.tdistrib_batch(np.array(seeds, np.int32)).reshape(len(seeds), -1)
+    for k, s in enumerate(seeds):
+        assert np.max(np.abs(T[k] - o.tdistrib_upot(o.potential(s)))) <= 1e-9
