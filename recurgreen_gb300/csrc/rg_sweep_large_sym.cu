@@ -289,8 +289,11 @@ struct ZgemmCtx {
 // transpose, with have = 2 those of its A, which is this B's transpose: two of
 // the eight operands of a node (512 modes 116 -> 112 ms, 152 realizations of
 // 256 modes 212 -> 203).
-__device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const Opnd A, const Opnd B,
-                                           const TileOut out, const int have) {
+// With `bounded`, nothing is done, and false returned in every thread, when an
+// entry of B reaches kMaxGrowth.
+constexpr int kGrowthExp = 1;  // kMaxGrowth = 2^kGrowthExp
+__device__ __noinline__ bool cluster_zgemm(const ZgemmCtx c, const int Mb, const Opnd A, const Opnd B,
+                                           const TileOut out, const int have, const bool bounded) {
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int tid = threadIdx.x, ctid = rank * kSymNT + tid, CNT = C * kSymNT;
@@ -323,6 +326,11 @@ __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const
     }
     __syncthreads();
   }
+  if (bounded) {
+    int big = 0;
+    for (int i = tid; i < 16 * T; i += kSymNT) big |= eb[i] > kGrowthExp;
+    if (__syncthreads_or(big)) return false;
+  }
   if (have != 1)
     crt::split(Mb, [&](int i, int k) { return opnd_at(A, i, k); }, ea, adig, c.stage, ctid >> 5, CNT >> 5);
   if (have != 2)
@@ -337,6 +345,7 @@ __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const
       if (k++ % C == rank)
         block_product(Mb, bi * crt::kBlkTiles, bj * crt::kBlkTiles, adig, bdig, ea, eb, c.stage, c.res, &s_out);
   cluster.sync();
+  return true;
 }
 
 // A product of at most 32 x 32 by every CTA of the cluster on its own, in
@@ -345,9 +354,9 @@ __device__ __noinline__ void cluster_zgemm(const ZgemmCtx c, const int Mb, const
 // column half of the 2 x 2 tiles.  Serial latencies bound it: 35,000 clocks,
 // where the general path's passes through the workspace and its cluster
 // barriers took over 100,000 whatever the size.  Reads the operands before a cluster barrier, writes after it, and
-// ends with another.
+// ends with another.  `bounded` as in cluster_zgemm.
 constexpr int kTinyModes = 32;
-__device__ __noinline__ void tiny_zgemm(uint4* stage, const Opnd A, const Opnd B, const TileOut o) {
+__device__ __noinline__ bool tiny_zgemm(uint4* stage, const Opnd A, const Opnd B, const TileOut o, const bool bounded) {
   cg::cluster_group cluster = cg::this_cluster();
   constexpr int T = 2, PL = T * T * 32, MP = 16 * T, NE = 4;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -376,6 +385,7 @@ __device__ __noinline__ void tiny_zgemm(uint4* stage, const Opnd A, const Opnd B
     e[q] = oz::row_exp<4>(exa, MP, r0 + 8 * q);
     e[2 + q] = oz::row_exp<4>(exb, MP, r0 + 8 * q);
   }
+  if (bounded && __syncthreads_or(e[2] > kGrowthExp || e[3] > kGrowthExp)) return false;
   {
     long long x[2 * NE];
 #pragma unroll
@@ -419,6 +429,7 @@ __device__ __noinline__ void tiny_zgemm(uint4* stage, const Opnd A, const Opnd B
   }
   if (cluster.num_blocks() > 1) cluster.sync();
   else __syncthreads();
+  return true;
 }
 
 // The leaf blocks of the inverse, at most 32 modes: the symmetric n x n matrix
@@ -1092,6 +1103,14 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
       // down to the leaves (kInvSteps).  Every Gauss-Jordan block goes through
       // the one call below.  A small pivot in a block flags the realization
       // as the full elimination does.
+      // Pivots do not cross blocks, so an A that is nearly singular beside B
+      // loses digits: every level takes T's largest entry, squared.  Where that
+      // reaches kMaxGrowth the node is eliminated as one block.  (T stays below
+      // 2 up to a mean free path of one slice or so.  Without the bound T of 65
+      // modes, 20 slices and an optical depth of 300 was off by up to 1e-10, of
+      // 200 modes, 8 slices and 30000 by 8e-8.  Emulated at 65 to 200 modes,
+      // bounds of 2, 4 and 8 leave 1 to 20, 1 to 1e3 and 1e2 to 1e6 times the
+      // elimination's error at worst.)
       {
         const InvSteps& steps = kInvSteps[split_levels];
         for (int st = 0; st < steps.count; ++st) {
@@ -1108,12 +1127,10 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
           double2* Hb = Ha + (int64_t)h * h;
           double2* Hs = Hb + (int64_t)h * h;
           const int h1 = (nP + 1) >> 1, h2 = nP >> 1;  // A is h1 x h1, S is h2 x h2
+          bool eliminate = false;
           if (op == kInvGJ) {
             const float tau = (float)fmin(kNaturalTau * a.sym_tau, 3e38);
-            if (nP > kTinyModes || !leaf_inverse(P, nP, tau, stage)) {
-              if (nP <= kSmallGJ) gj_small(P, nP);
-              else gj(P, nP);
-            }
+            eliminate = nP > kTinyModes || !leaf_inverse(P, nP, tau, stage);
           } else if (op == kInvCopyA) {  // A into Ha (upper triangle)
             for (int i = ctid >> 5; i < h1; i += CNT >> 5)
               for (int j = i + lane; j < h1; j += 32) Ha[i * h1 + j] = __ldcg(P + (int64_t)i * nP + j);
@@ -1144,8 +1161,17 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
               B = Opnd{Hb, h1, 0, 0, 1, h2, h1};
               o = TileOut{P, nP, 0, -1.0, Ha, h1, 0, 1, 1, h1, h1};
             }
-            if (h1 <= kTinyModes) tiny_zgemm(stage, A, B, o);
-            else cluster_zgemm(zc, h1, A, B, o, have);
+            const bool bounded = op == kInvS;
+            const bool done =
+                h1 <= kTinyModes ? tiny_zgemm(stage, A, B, o, bounded) : cluster_zgemm(zc, h1, A, B, o, have, bounded);
+            if (!done) {  // P is as it was: eliminate it, past the node's other steps
+              eliminate = true;
+              while (steps.code[st] != kInvY22 * 32 + node) ++st;
+            }
+          }
+          if (eliminate) {
+            if (nP <= kSmallGJ) gj_small(P, nP);
+            else gj(P, nP);
           }
         }
       }
@@ -1164,7 +1190,7 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
         } else {
           // the result overwrites B Gs1 in place (its residues are already taken)
           cluster_zgemm(zc, M, Opnd{W, M, 0, 1, 0, M, M}, Opnd{Rg, M, 0, 0, 0, M, M},
-                        TileOut{Rg, M, 0, 1.0, nullptr, 0, 0, 0, 0, M, M}, 0);
+                        TileOut{Rg, M, 0, 1.0, nullptr, 0, 0, 0, 0, M, M}, 0, false);
         }
       }
       if (a.state_dump && *status0 != kStatusNeedPivot) {
