@@ -95,9 +95,10 @@ struct WgDesc {
   const double2* bmat;        // [M] B diagonal
   const double2* adiag_edge;  // [M] A diagonal on slices 1 and nx
   const double2* adiag_bulk;  // [M] A diagonal in the bulk
-  // The slice matrix scaled by B^(-1/2) on both sides (rg_sweep_sym.cu):
-  const double2* wsc;         // [M] B^(-1/2)
-  const double2* aw_edge;     // [2 M] A/B on slices 1 and nx: rounded to FP64, then the rest
+  // The slice matrix scaled by D^-1 on both sides, D^2 = B/c (rg_sweep_sym.cu):
+  const double* csc;          // [max(M, 64)] c, powers of two, or NULL: all 1
+  const double2* wsc;         // [M] D^-1
+  const double2* aw_edge;     // [2 M] A c/B on slices 1 and nx: rounded to FP64, then the rest
   const double2* aw_bulk;     // [2 M] the same in the bulk
   const double2* sqmu_c;      // [M] complex sqrt(mu) (tdistrib Fisher-Lee)
   const double2* sqmu_r;      // [M] sqrt(real(mu)) (v1 Fisher-Lee)

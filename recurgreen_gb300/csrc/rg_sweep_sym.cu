@@ -3,10 +3,15 @@
 // With Dirichlet modes the slice matrix X_n = A_n - V_n - B Gss B is complex
 // symmetric (A and B diagonal, V real symmetric, and Gss = inv(X_{n-1}) is
 // symmetric in turn).  The kernel keeps it in the variables scaled by
-// D = B^(1/2) (src/waveguide.f90:426-440 in them):
-//   X' = D^-1 X D^-1 = A/B - D^-1 V D^-1 - G',   G' = D Gss D = inv(X'),
-//   Q  = (D Gs1 D)^T:  Q_0 = G'_0,  Q_n = -Q_{n-1} G'_n,
-// so a slice needs no product with B, and every matrix entry is of order 1.
+// D = (B/c)^(1/2) (src/waveguide.f90:426-440 in them):
+//   X' = D^-1 X D^-1 = c A/B - D^-1 V D^-1 - c G' c,   G' = D Gss D = inv(X'),
+//   Q  = (D Gs1 D)^T:  Q_0 = G'_0,  Q_n = -Q_{n-1} c G'_n,
+// with c = 1 for open modes, so that a slice needs no product with B, and every
+// matrix entry is of order 1.  A closed mode's |A/B| is 2 cosh(kappa dx): on
+// coarse slices, where that passes 32, c is the power of two that takes it back
+// (the 26 bits of the FP32 inverse do not span cosh(6): whole items went to the
+// pivoted kernel: 304 guides of 63 modes, 14 of them closed, 200 slices,
+// kappa dx up to 6.4, 355 ms, 67 now).
 //
 // In the modes exp(2 pi i k y) of a periodic guide X is Hermitian but for its
 // diagonal, not symmetric; A and B depend on |k| alone, so in the real modes
@@ -204,6 +209,7 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
     const int M = wd.M, ny = wd.ny, nx = wd.nx;
     const bool per = wd.periodic != 0;
     const bool pass_on = per && a.state_dump;
+    const bool scaled = wd.csc != nullptr;
     if (tid == 0) {
       s_status = pass_on ? kStatusNeedPivot : RG_OK;
       s_abort[0] = s_abort[1] = 0;
@@ -233,6 +239,10 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
         if (n <= nx - 3) bar_arrive(kBarGFree + b, NMAIN + NPROP);
         if (skip) continue;
         if (n > a.inject_at) {
+          if (scaled) {  // Q c (the factors of the padding are 1)
+#pragma unroll
+            for (int k = 0; k < NE; ++k) q[k] = cscale(wd.csc[c0 + ecol(k)], q[k]);
+          }
           int eq0 = oz::kNoExp, eq1 = oz::kNoExp;
 #pragma unroll
           for (int k = 0; k < NE; ++k) {
@@ -407,7 +417,16 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
         bar_sync(kBarFull + b, NMAIN + kProd);
         double x[NV];
         if (!aborted) {
-          // 1. X' = A/B - w V w - G' (zero outside M x M).
+          if (scaled && n > 0) {  // c G' c and Q c in place (the factors of the padding are 1)
+#pragma unroll 1
+            for (int k = 0; k < NE; ++k) {
+              const double cj = wd.csc[c0 + ecol(k)], f = wd.csc[r0 + erow(k)] * cj;
+              gp[64 * k] *= f;
+              if (NP == 1) gp[64 * k + 1] *= f;
+              if (!PROP && !refl) Qs[32 * k] = cscale(cj, Qs[32 * k]);
+            }
+          }
+          // 1. X' = c A/B - w V w - c G' c (zero outside M x M).
           const int id = (refl ? nx - 1 - n : n) - wd.nxfree;
           const bool dis = (id >= 0 && id < wd.nxdiso), edge = (n == 0 || n == nx - 1);
           const double* co = cc + b * (2 * MP + 2);
@@ -425,7 +444,7 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
                 if (n > 0) v = -gp[64 * k + (q < NE ? 0 : 1)];
                 if (i == j) v += aw[2 * i + p];
                 if (dis && (p == 0 || !real_w)) v = fma(-wp[64 * k + (q < NE ? 0 : 1)], vij, v);
-                if (i == j) v += aw[2 * (M + i) + p];  // the rest of A/B beyond FP64
+                if (i == j) v += aw[2 * (M + i) + p];  // the rest of c A/B beyond FP64
               }
               x[q] = v;
             }

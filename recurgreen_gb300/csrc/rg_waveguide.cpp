@@ -184,7 +184,8 @@ struct rg_waveguide {
   double kl = 0, kdx = 0, dos = 0, stdu = 0;
   std::vector<double> xmesh, ymesh, kpmesh;
   std::vector<cplx> mumesh, bmat, aedge, abulk, sqmu_c, sqmu_r;
-  std::vector<cplx> wsc, aw;     // B^(-1/2); A/B on edge slices and in the bulk, [2][2][nmu] (rounded, rest)
+  std::vector<double> csc;       // c of D^2 = B/c, empty when all 1
+  std::vector<cplx> wsc, aw;     // D^-1; A c/B on edge slices and in the bulk, [2][2][nmu] (rounded, rest)
   std::vector<double> costab;    // [ny][2*nmu+1], Dirichlet
   std::vector<cplx> expfac;      // [ny][nmu], periodic
   std::vector<uint64_t> jump;    // [ny][4]
@@ -193,6 +194,7 @@ struct rg_waveguide {
   cudaStream_t stream = nullptr;
   double2 *d_bmat = nullptr, *d_aedge = nullptr, *d_abulk = nullptr, *d_sqmu_c = nullptr, *d_sqmu_r = nullptr;
   double2 *d_wsc = nullptr, *d_aw = nullptr;
+  double* d_csc = nullptr;
   double* d_costab = nullptr;
   double2* d_expfac = nullptr;
   uint64_t* d_jump = nullptr;
@@ -241,6 +243,7 @@ void free_device(rg_waveguide* w) {
   cudaFree(w->d_bmat);
   cudaFree(w->d_aedge);
   cudaFree(w->d_abulk);
+  cudaFree(w->d_csc);
   cudaFree(w->d_wsc);
   cudaFree(w->d_aw);
   cudaFree(w->d_sqmu_c);
@@ -273,6 +276,7 @@ void free_device(rg_waveguide* w) {
   w->sweep_timed = false;
   if (w->stream) cudaStreamDestroy(w->stream);
   w->d_bmat = w->d_aedge = w->d_abulk = w->d_sqmu_c = w->d_sqmu_r = w->d_wsc = w->d_aw = nullptr;
+  w->d_csc = nullptr;
   w->d_costab = nullptr;
   w->d_expfac = nullptr;
   w->d_jump = nullptr;
@@ -300,6 +304,28 @@ void divide_exactly(cplx a, cplx b, cplx* q, cplx* rest) {
   const cplx r(residual(a.real(), q->real(), b.real(), -q->imag(), b.imag()),
                residual(a.imag(), q->real(), b.imag(), q->imag(), b.real()));
   *rest = r / b;
+}
+
+// A mode's entries of the scaled slice matrix: c, D^-1 with D^2 = B/c, and A c/B
+// on edge slices (aw[0], aw[m]) and in the bulk (aw[2 m], aw[3 m]).  |A/B| is at
+// most 2 for an open mode and 2 cosh(kappa dx) for a closed one: from 32 on (3.4
+// e-foldings a slice), c brings it to 2 .. 8; at 2^900, where B is nothing beside
+// A, the matrix is left as it is (D = 1, c = 0).
+double scaled_mode(cplx edge, cplx bulk, cplx b, cplx* wsc, cplx* aw, int m) {
+  const double ratio = std::abs(bulk) / std::abs(b);
+  if (ratio >= 0x1p900) {
+    *wsc = 1.0;
+    aw[0] = edge, aw[2 * m] = bulk;
+    aw[m] = aw[3 * m] = 0.0;
+    return 0.0;
+  }
+  const int h = ratio < 32.0 ? 0 : (std::ilogb(ratio) - 1) / 2;  // c = 4^-h
+  const double c = std::ldexp(1.0, -2 * h);
+  *wsc = std::ldexp(1.0, -h) / std::sqrt(b);
+  divide_exactly(edge, b, aw, aw + m);
+  divide_exactly(bulk, b, aw + 2 * m, aw + 3 * m);
+  for (int k = 0; k < 4; ++k) aw[k * m] *= c;
+  return c;
 }
 
 // Host tables of init_waveguide, src/waveguide.f90:81-255.
@@ -371,6 +397,8 @@ int build_tables(rg_waveguide* w, const rg_params& p) {
   w->sqmu_r.resize(M);
   w->wsc.resize(M);
   w->aw.resize(4 * (size_t)M);
+  w->csc.assign(std::max(M, (int)rg::kMaxModesSmem), 1.0);
+  bool scaled = false;
   double dos = 0.0;
   for (int n = 0; n < M; ++n) {
     const double kp = w->kpmesh[n];
@@ -385,12 +413,12 @@ int build_tables(rg_waveguide* w, const rg_params& p) {
     const cplx cot = mu / std::tan(mu * w->kdx);
     w->aedge[n] = iu * mu - cot;
     w->abulk[n] = -2.0 * cot;
-    w->wsc[n] = 1.0 / std::sqrt(w->bmat[n]);
-    divide_exactly(w->aedge[n], w->bmat[n], &w->aw[n], &w->aw[M + n]);
-    divide_exactly(w->abulk[n], w->bmat[n], &w->aw[2 * M + n], &w->aw[3 * M + n]);
+    const double c = w->csc[n] = scaled_mode(w->aedge[n], w->abulk[n], w->bmat[n], &w->wsc[n], &w->aw[n], M);
+    scaled = scaled || c != 1.0;
     w->sqmu_c[n] = std::sqrt(mu);                              // src/waveguide.f90:443
     w->sqmu_r[n] = cplx(std::sqrt(std::real(mu)), 0.0);       // src/waveguide.f90:510
   }
+  if (!scaled) w->csc.clear();
   w->stdu = std::sqrt(p.dscat * ny / (2.0 * kPi * kPi * w->dos * p.wol * p.nxdiso));  // src/waveguide.f90:370
 
   // Projection tables.  Dirichlet modes chi_m(y) = sqrt(2/ny) sin(pi m y)
@@ -428,6 +456,7 @@ int upload_tables(rg_waveguide* w) {
   if ((rc = upload(&w->d_bmat, w->bmat.data(), cb))) return rc;
   if ((rc = upload(&w->d_aedge, w->aedge.data(), cb))) return rc;
   if ((rc = upload(&w->d_abulk, w->abulk.data(), cb))) return rc;
+  if (!w->csc.empty() && (rc = upload(&w->d_csc, w->csc.data(), sizeof(double) * w->csc.size()))) return rc;
   if ((rc = upload(&w->d_wsc, w->wsc.data(), cb))) return rc;
   if ((rc = upload(&w->d_aw, w->aw.data(), 4 * cb))) return rc;
   if ((rc = upload(&w->d_sqmu_c, w->sqmu_c.data(), cb))) return rc;
@@ -452,6 +481,7 @@ int upload_tables(rg_waveguide* w) {
   d.bmat = w->d_bmat;
   d.adiag_edge = w->d_aedge;
   d.adiag_bulk = w->d_abulk;
+  d.csc = w->d_csc;
   d.wsc = w->d_wsc;
   d.aw_edge = w->d_aw;
   d.aw_bulk = w->d_aw + 2 * w->nmu;

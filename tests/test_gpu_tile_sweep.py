@@ -146,3 +146,26 @@ def test_inverses_with_rows_of_very_different_size(bt, m, nx, dscat, seeds):
     T = g.tdistrib_batch(np.array(seeds, np.int32)).reshape(len(seeds), -1)
     for k, s in enumerate(seeds):
         assert np.max(np.abs(T[k] - o.tdistrib_upot(o.potential(s)))) <= 1e-9
+
+
+@pytest.mark.parametrize("bt", ["dirichlet", "periodic"])
+@pytest.mark.parametrize("m,nx,aratio,exfac,dabso", [(11, 3, 1.0, 1.3, 0.0), (21, 5, 1.0, 1.3, 0.0), (33, 5, 1.0, 2.0, 0.3),
+                                                     (47, 12, 2.0, 1.1, 0.0), (49, 4, 1.0, 1.3, 0.5), (63, 40, 3.0, 1.3, 0.0),
+                                                     (63, 2, 1.0, 2.0, 0.0)])
+def test_closed_channels_on_coarse_slices(bt, m, nx, aratio, exfac, dabso):
+    """Closed channels that decay by up to exp(60) over a slice: t, r, the filtered T and the deposition matrix from this
+    kernel, none passed on (but for small pivots in the guide of two slices, which share an optical depth of 3)."""
+    wol = ((m + 0.5) / 2 if bt == "dirichlet" else m // 2 + 0.45) / exfac
+    kw = dict(boundtype=bt, nxdiso=nx, nxfree=1, wol=wol, exfac=exfac, aratio=aratio, dscat=3.0, dabso=dabso, ny=m + 2)
+    o, g = O.Waveguide(**kw), rg.Waveguide(**kw)
+    assert g.nmu == m
+    u = o.potential(4)
+    ro, to = o.refl_trans_v1_upot(u)
+    r, t = g.refl_trans_v1_upot(u, want_r=True)
+    assert rel(t, to) <= 1e-10 and rel(r, ro) <= 1e-10
+    T = g.tdistrib_batch(np.arange(1, 201, dtype=np.int32)).reshape(200, -1)
+    info = g.last_batch_info()
+    assert info["kernel"] == "symmetric" and (info["rerun"] == 0 or (nx == 2 and info["rerun"] < 100))
+    assert np.max(np.abs(T[3] - o.tdistrib_upot(u))) <= 1e-9
+    np.testing.assert_array_equal(T[3], g.tdistrib_batch(np.array([4], np.int32)))
+    assert rel(g.compute_deposition(4, nx, 2), o.deposition_upot(u, nx, 2)) <= 1e-10
