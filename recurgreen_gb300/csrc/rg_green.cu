@@ -788,7 +788,7 @@ __global__ void wavefun_kernel(WavefunArgs a) {
 template <int JMAX>
 int launch_back_t(const BackArgs& a, cudaStream_t s) {
   const size_t smem = (2 * sizeof(double2) + sizeof(double)) * (size_t)a.M * kKC;
-  RG_CUDA(cudaFuncSetAttribute(back_kernel<JMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  RG_CUDA(allow_smem((const void*)back_kernel<JMAX>, smem));
   const dim3 grid((a.kmax + kKC - 1) / kKC, a.nreal);
   back_kernel<JMAX><<<grid, kNT, smem, s>>>(a);
   RG_CUDA(cudaGetLastError());

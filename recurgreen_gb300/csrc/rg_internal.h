@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <complex>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -28,8 +29,12 @@ int cuda_fail(cudaError_t e, const char* what);
   } while (0)
 
 // Lets a kernel take `bytes` of dynamic shared memory, and never less than it
-// may already take: one launch plan may cover several sizes of a kernel.
+// may already take: the limit is the kernel's, not the launch's, and between a
+// plan and its launch another handle, on another thread, may plan a smaller size.
+// Every kernel's limit is set here, one thread at a time.
 inline cudaError_t allow_smem(const void* kernel, size_t bytes) {
+  static std::mutex one_at_a_time;
+  std::lock_guard<std::mutex> lock(one_at_a_time);
   cudaFuncAttributes fa{};
   cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
   if (e != cudaSuccess || (size_t)fa.maxDynamicSharedSizeBytes >= bytes) return e;

@@ -137,7 +137,7 @@ int launch_zgemm(int M, int nbatch, const ZOp& A, const ZOp& B, const double2* r
   const int per = std::max(1, std::min(16, T * T * 32 / kOzThreads));
   zb_exps_kernel<<<nbatch * 2 * ((M + 31) / 32), kOzThreads, 0, s>>>(M, A, B, rowscale, ws);
   zb_split_kernel<<<nbatch * per, kOzThreads, 0, s>>>(M, A, B, rowscale, ws, per);
-  RG_CUDA(cudaFuncSetAttribute(zb_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZbGemmSmem));
+  RG_CUDA(allow_smem((const void*)zb_gemm_kernel, kZbGemmSmem));
   const int nblk = ((T + oz::kBlkRows - 1) / oz::kBlkRows) * ((T + oz::kBlkCols - 1) / oz::kBlkCols);
   zb_gemm_kernel<<<nbatch * nblk, kOzThreads, kZbGemmSmem, s>>>(M, ws, alpha, D, beta, C, strideC, colmajor);
   RG_CUDA(cudaGetLastError());

@@ -553,7 +553,7 @@ int launch_histogram(const double* d_samples, int64_t n, const double* d_bins, i
   const size_t smem = sizeof(unsigned long long) * (nbins + 1);
   if (smem > 200 * 1024) return fail(RG_ERR_INVALID_ARG, "too many histogram bins");
   if (smem > 48 * 1024)
-    RG_CUDA(cudaFuncSetAttribute(histogram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RG_CUDA(allow_smem((const void*)histogram_kernel, smem));
   int64_t blocks = (n + 255) / 256;
   if (blocks > 1024) blocks = 1024;
   if (blocks < 1) blocks = 1;

@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(kLargeNT, 2) sweep_large_kernel(SweepArgs a) {
 int sweep_large_plan(SweepArgs& a, int sm_count, int* grid, int64_t* work_stride) {
   const size_t smem = LargeSmem::bytes(a.max_M, a.max_ny);
   if (smem > 227 * 1024) return fail(RG_ERR_INVALID_ARG, "too many modes or transverse points for the large-mode kernel");
-  RG_CUDA(cudaFuncSetAttribute(sweep_large_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  RG_CUDA(allow_smem((const void*)sweep_large_kernel, smem));
   int per_sm = 0;
   RG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_large_kernel, kLargeNT, smem));
   if (per_sm < 1) return fail(RG_ERR_INVALID_ARG, "large-mode sweep kernel does not fit on an SM");

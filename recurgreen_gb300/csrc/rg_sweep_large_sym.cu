@@ -1279,7 +1279,7 @@ int sweep_large_sym_plan(SweepArgs& a, int sm_count, int* grid, int64_t* work_st
   const bool tensor = a.tensor_r != 0;
   const size_t smem = LargeSymSmem::bytes(a.max_M, tensor);
   if (smem > 227 * 1024) return fail(RG_ERR_INVALID_ARG, "too many modes for the symmetric large-mode kernel");
-  RG_CUDA(cudaFuncSetAttribute(sweep_large_sym_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  RG_CUDA(allow_smem((const void*)sweep_large_sym_kernel, smem));
   int per_sm = 0;
   RG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_large_sym_kernel, kSymNT, smem));
   if (per_sm < 1) return fail(RG_ERR_INVALID_ARG, "symmetric large-mode sweep kernel does not fit on an SM");
