@@ -175,6 +175,22 @@ struct SweepArgs {
   int split_inverse;
 };
 
+// Whether the blocked symmetric kernel spends its slices in the elimination
+// whose row split is tuned: without the tensor-core product, or with fewer
+// block levels asked for.  (With the block inverse down to its leaves only a
+// node that is nearly singular comes there.)
+inline bool row_split_matters(const SweepArgs& a, bool periodic) {
+  return a.symmetric && !periodic && a.max_M > kMaxModesSmem && (!a.tensor_r || a.max_M > 512 || a.split_inverse < 3);
+}
+
+// What a tuned launch configuration holds for besides the shape and the batch:
+// the kernel that runs, and the form of its inverse.
+inline int tuned_kernel(const SweepArgs& a, bool periodic) {
+  const bool symmetric = a.symmetric && (!periodic || a.max_M <= kMaxModesSmem);
+  return (symmetric ? 1 : 0) | (symmetric && a.max_M > kMaxModesSmem ? (a.tensor_r ? 2 : 0) | a.split_inverse << 2 : 0) |
+         (periodic ? 16 : 0);
+}
+
 // Status the symmetric kernel leaves on an item whose diagonal pivots were
 // too small; the pivoted kernel recomputes such items (never returned).
 constexpr int kStatusNeedPivot = 64;

@@ -586,7 +586,7 @@ int place_workspace(rg_waveguide* w, rg::SweepArgs& a, size_t off, int* grid) {
 }
 
 // ---------------------------------------------------------------------------
-// Autotuner.  For a waveguide shape (M, ny) and a batch size, candidate launch
+// Autotuner.  For a waveguide shape (M, ny), a kernel and a batch size, candidate launch
 // configurations are timed once on a short proxy guide (the same modes and
 // grid, 16 slices, the same number of realizations) and the fastest is
 // cached for the process.  RG_AUTOTUNE=0 disables it (the built-in
@@ -594,9 +594,10 @@ int place_workspace(rg_waveguide* w, rg::SweepArgs& a, size_t off, int* grid) {
 // bit for bit the same are tuned:
 //   * above 64 modes, the blocked kernel's cluster size (CTAs per
 //     realization; it changes which CTA computes an element, not its
-//     arithmetic), then, for the chosen cluster size, the threads per update
-//     unit of the symmetric kernel (1, 4 or 8; it changes which thread
-//     updates a row, not the row's operations);
+//     arithmetic), then, for the chosen cluster size and where the symmetric
+//     kernel eliminates whole slices (row_split_matters), the threads per
+//     update unit (1, 4 or 8; it changes which thread updates a row, not the
+//     row's operations);
 //   * up to 64 modes, the persistent CTAs per SM of the shared-memory
 //     kernels (each realization is one CTA's, whatever the grid).
 // The kernel itself (symmetric but for periodic guides above 64 modes, which
@@ -612,9 +613,9 @@ struct TuneChoice {
 };
 
 struct TuneKey {
-  int M, ny, bucket, sms;
+  int M, ny, bucket, sms, kernel;
   bool operator<(const TuneKey& o) const {
-    return std::tie(M, ny, bucket, sms) < std::tie(o.M, o.ny, o.bucket, o.sms);
+    return std::tie(M, ny, bucket, sms, kernel) < std::tie(o.M, o.ny, o.bucket, o.sms, o.kernel);
   }
 };
 
@@ -686,7 +687,9 @@ TuneChoice autotune(rg_waveguide* w, int n, cudaStream_t s) {
   TuneChoice def;
   if (!autotune_enabled() || n <= 0) return def;
   const bool blocked = w->nmu > rg::kMaxModesSmem;
-  const TuneKey key{w->nmu, w->ny, size_bucket(n), w->sm_count};
+  const rg::SweepArgs form = make_args(w, rg::kModeEig);
+  const bool periodic = w->p.boundtype == RG_BOUND_PERIODIC;
+  const TuneKey key{w->nmu, w->ny, size_bucket(n), w->sm_count, rg::tuned_kernel(form, periodic)};
   {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
     auto it = g_tune_cache.find(key);
@@ -729,7 +732,7 @@ TuneChoice autotune(rg_waveguide* w, int n, cudaStream_t s) {
   if (blocked) {
     for (int c = 1; c <= 8; c *= 2) consider(TuneChoice{c, 0, 0});
     const int cbest = best.force_cluster;
-    if (w->p.boundtype == RG_BOUND_DIRICHLET)  // the symmetric kernel's row split
+    if (rg::row_split_matters(form, periodic))
       for (int t : {1, 4, 8}) consider(TuneChoice{cbest, t, 0});
   } else {
     // CTAs per SM: the occupancy limit, then fewer (distinct grids only)
