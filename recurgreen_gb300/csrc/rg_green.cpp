@@ -70,6 +70,7 @@ class Arena {
     }
     return RG_OK;
   }
+  size_t size() const { return size_; }
   template <class T>
   T* at(size_t off) const {
     return reinterpret_cast<T*>(static_cast<char*>(base_) + off);
@@ -79,26 +80,6 @@ class Arena {
   void* base_ = nullptr;
   size_t size_ = 0;
 };
-
-// Realizations per launch: what fits in half the free device memory (at most
-// 96 GiB), rounded down to whole waves of two CTAs per SM when larger.
-// RG_GREEN_CHUNK=k caps it at k (tests use it to run several chunks).
-int chunk_size(const GreenView& v, int n, size_t per_item) {
-  const char* cap = std::getenv("RG_GREEN_CHUNK");
-  const long cap_n = (cap && *cap) ? std::strtol(cap, nullptr, 10) : 0;
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-    cudaGetLastError();
-    free_b = (size_t)8 << 30;
-  }
-  const size_t budget = std::min(free_b / 2, (size_t)96 << 30);
-  int64_t c = (int64_t)(budget / std::max<size_t>(per_item, 1));
-  c = std::max<int64_t>(1, std::min<int64_t>(c, n));
-  const int wave = 2 * v.sm_count;
-  if (c > wave && c < n) c -= c % wave;
-  if (cap_n > 0 && c > cap_n) c = cap_n;
-  return (int)c;
-}
 
 // The forward sweep of nk realizations with the state of every slice kept,
 // Fisher-Lee t (sqrt(real(mu)), full nmu x nmu) to d_t when given, source at
@@ -154,6 +135,32 @@ int plan_sweep(const GreenView& v, int nk, int source, Arena& ar, DumpSweep* ds,
   }
   ds->off_work = ar.add(work);
   return RG_OK;
+}
+
+// Realizations per launch: what fits in half the free device memory (at most
+// 96 GiB), rounded down to whole waves of two CTAs per SM when larger, and fewer
+// where the sweep's workspace does not fit beside them (above 64 modes 11 MB for
+// each at 256, 40 MB at 512).
+// RG_GREEN_CHUNK=k caps it at k (tests use it to run several chunks).
+int chunk_size(const GreenView& v, int n, size_t per_item) {
+  const char* cap = std::getenv("RG_GREEN_CHUNK");
+  const long cap_n = (cap && *cap) ? std::strtol(cap, nullptr, 10) : 0;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    free_b = (size_t)8 << 30;
+  }
+  const size_t budget = std::min(free_b / 2, (size_t)96 << 30);
+  int64_t c = (int64_t)(budget / std::max<size_t>(per_item, 1));
+  c = std::max<int64_t>(1, std::min<int64_t>(c, n));
+  const int wave = 2 * v.sm_count;
+  if (c > wave && c < n) c -= c % wave;
+  if (cap_n > 0 && c > cap_n) c = cap_n;
+  return rg::fitting_chunk((int)c, per_item, free_b, [&](int k) {
+    Arena plan;
+    DumpSweep ds;
+    return plan_sweep(v, k, 0, plan, &ds) == RG_OK ? plan.size() : 0;
+  });
 }
 
 int launch_dump_sweep(const GreenView& v, DumpSweep& ds, const Arena& ar, int nk, const int32_t* d_seeds,

@@ -51,6 +51,14 @@ __host__ __device__ inline int descending_rank(const double* t, int n, int v) {
   return k;
 }
 
+// The largest of c, 3/4 c, ... realizations per launch that fit 15/16 of the free
+// memory with the sweep's workspace, work(c) bytes, beside their own buffers.
+template <class Work>
+int fitting_chunk(int c, size_t per_item, size_t free_bytes, Work work) {
+  while (c > 1 && (size_t)c * per_item + work(c) > free_bytes - free_bytes / 16) c -= (c + 3) / 4;
+  return c;
+}
+
 // Switches to a handle's device for the duration of a call.
 struct DeviceGuard {
   int prev = -1;
