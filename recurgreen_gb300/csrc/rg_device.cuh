@@ -96,8 +96,9 @@ __device__ __forceinline__ double scaled_normal(double stdu, Xoshiro& st) {
 // Singular values: Householder bidiagonalisation, then bisection.
 // ---------------------------------------------------------------------------
 
-// 1/x to about one ulp for normal x: the hardware's approximation and two
-// Newton steps (a division instruction sequence is twice as long).
+// 1/x to one ulp where x and 1/x are normal (NaN elsewhere): the hardware's
+// approximation and two Newton steps (a division instruction sequence is twice as
+// long).  For bidiag_count, whose divisors lie in between.
 __device__ __forceinline__ double fast_rcp(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));

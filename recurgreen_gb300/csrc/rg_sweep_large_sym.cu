@@ -1035,7 +1035,7 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
             double2 d = make_double2(0.0, 0.0);
             if (!singular) {
               const double2 z = Sw[pk * ld + pk];
-              const double rden = fast_rcp(fma(z.x, z.x, z.y * z.y));
+              const double rden = 1.0 / fma(z.x, z.x, z.y * z.y);
               d = make_double2(z.x * rden, -z.y * rden);
             }
             unsigned long long offmax = 0ULL;
