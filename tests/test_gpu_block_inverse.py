@@ -61,3 +61,16 @@ def test_block_inverse_under_strong_disorder(monkeypatch, m, nx, dscat, n, bar):
     assert g.last_batch_info()["rerun"] < n // 2  # most T are this kernel's own
     monkeypatch.setenv("RG_SYMMETRIC", "0")
     assert np.max(np.abs(T - g.tdistrib_batch(seeds))) <= bar
+
+
+@pytest.mark.parametrize("levels", ["0", "1", "2"])
+@pytest.mark.parametrize("m", [67, 128, 130, 300])
+def test_fewer_block_levels(monkeypatch, levels, m):
+    """RG_SPLIT_INVERSE=0, 1, 2: the blocks left are eliminated, whole ones of more than 64 modes among them."""
+    monkeypatch.setenv("RG_SPLIT_INVERSE", levels)
+    kw = guide(m, m + 3, 3, dabso=0.2)
+    o, g = O.Waveguide(**kw), rg.Waveguide(**kw)
+    u = o.potential(4)
+    ro, to = o.refl_trans_v1_upot(u)
+    r, t = g.refl_trans_v1_upot(u, want_r=True)
+    assert rel(t, to) <= 1e-10 and rel(r, ro) <= 1e-10
