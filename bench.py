@@ -105,15 +105,19 @@ def flops_per_realization(M: int, nx: int) -> float:
     return 16.0 * M ** 3 * (nx - 1) + 8.0 * M ** 3
 
 
-def executed_flops(M: int, nx: int, kernel: str) -> tuple[float, float]:
+DIGIT_PRODUCT = 26 * 8.0  # FP16 flops of a complex k x k product over k^3: 26 digit pairs, or 12 moduli x 2 products
+MODULAR_PRODUCT = 48.0
+
+
+def executed_flops(M: int, nx: int, kernel: str, product: float = DIGIT_PRODUCT) -> tuple[float, float]:
     """(FP64 flops, FP16 tensor flops) the sweep executes for one realization, O(M^2) terms left out:
       * tensor-core symmetric kernel (M <= 64): per slice 26 digit pairs x 8 M^3 for the propagator and 37 pairs
         (residual 18, series 12 + 6 + 1) for the inverse, whose FP32 part is not counted;
       * blocked symmetric kernel (64 < M <= 512): per k x k product 12 moduli x 2 real products of 2 k^3; one of M
         for the propagator and four of half the size per block of the 2 x 2 form, halved down to leaves of at most
         32 modes, whose own products (26 pairs) and inverse (37 pairs) are digit products.  With RG_SPLIT_INVERSE
-        0, 1 or 2 that many levels over even sizes >= 128 and FP64 elimination of the blocks left, the products
-        counted at the 26 digit pairs of their digit form;
+        0, 1 or 2 that many levels over even sizes >= 128 and FP64 elimination of the blocks left, a product of k
+        counted as `product` k^3 (the kernel's are modular ones, MODULAR_PRODUCT);
       * otherwise the pivoted reference count 16 M^3 in FP64.
     RG_TENSOR_R=0 selects the FP64-only symmetric elimination."""
     tensor = os.environ.get("RG_TENSOR_R", "1") != "0" and 64 < M <= 512
@@ -125,20 +129,26 @@ def executed_flops(M: int, nx: int, kernel: str) -> tuple[float, float]:
     if not tensor:
         return flops_symmetric(M, nx), 0.0
     if want == 3:
-        fp16, m, blocks = 48.0 * M ** 3, float(M), 1
+        fp16, m, blocks = MODULAR_PRODUCT * M ** 3, float(M), 1
         while m > 32:
             m /= 2
-            fp16 += blocks * 4 * (48.0 if m > 32 else 26 * 8.0) * m ** 3
+            fp16 += blocks * 4 * (MODULAR_PRODUCT if m > 32 else DIGIT_PRODUCT) * m ** 3
             blocks *= 2
         return 0.0, (fp16 + blocks * 37 * 8.0 * m ** 3) * nx
-    fp16 = 208.0 * M ** 3
+    fp16 = product * M ** 3
     m, blocks = M, 1
     while want > 0 and m >= 128 and m % 2 == 0:
         want -= 1
-        fp16 += blocks * 4 * 208.0 * (m // 2) ** 3
+        fp16 += blocks * 4 * product * (m // 2) ** 3
         m, blocks = m // 2, blocks * 2
     fp64 = blocks * 4.0 * m ** 3
     return fp64 * nx, fp16 * nx
+
+
+def flops_eigenvalues(M: int) -> float:
+    """FP64 flops of the eigenvalue stage, once per realization: the bidiagonalisation's two passes over what is left
+    of t, four complex multiply-adds an entry and step, 4/3 M^3 of them."""
+    return 32.0 / 3.0 * M ** 3
 
 
 def flops_symmetric(M: int, nx: int) -> float:
@@ -372,7 +382,8 @@ def run_main(args, spec: dict) -> None:
     info = w.last_batch_info()
     M = w.nmu
     fl = flops_per_realization(M, w.nx)
-    fl64, fl16 = executed_flops(M, w.nx, info["kernel"])
+    fl64, fl16 = executed_flops(M, w.nx, info["kernel"], MODULAR_PRODUCT)
+    fl64 += flops_eigenvalues(M)
     if info["kernel"] in ("symmetric", "blocked_symmetric"):  # re-run items also cost a pivoted sweep
         fl64 += fl * info["rerun"] / n
     value = world * n * args.steps / dev
@@ -396,7 +407,8 @@ def run_main(args, spec: dict) -> None:
         per_launch = sum(sweep_s) / len(sweep_s)  # this rank's batches
         achieved = fl * n / per_launch / 1e12
         t64, t16 = fl64 * n / per_launch / 1e12, fl16 * n / per_launch / 1e12
-        out["roofline"] = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+        # no pipe bounds the tensor-core sweeps: their phases wait for one another, and above 64 modes for memory
+        out["roofline"] = {"bound": "latency" if fl16 else "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                            "frac": achieved / peak, "traffic": None, "peak_source": peak_src,
                            "algorithmic_flops_per_launch": fl * n,
                            "algorithmic_count": "16 M^3 per slice-solve (slices 2..Nx) + 8 M^3, per realization: "
