@@ -14,8 +14,8 @@
 // So an entry is read and written twice a step, 16 FP64 multiply-adds in all,
 // 16/3 n^3 for the matrix: the FP64 pipe bounds it (51 M clocks for 256 x
 // 256), where nine sweeps of one-sided Jacobi at 4 n^3 complex rotations took
-// 0.9 G.  Measured with the sweep: 152 guides of 256 modes and 40 slices 1,435
-// ms before, 287 now; one guide of 60 slices on 8 CTAs 316 ms before, 150 now.
+// 0.9 G.  By this stage alone: 152 guides of 256 modes and 40 slices 1,435 ->
+// 287 ms, one guide of 60 slices on 8 CTAs 316 -> 150.
 #pragma once
 
 #include <cooperative_groups.h>

@@ -250,7 +250,7 @@ __device__ void bidiag_values(double* d, double* e, int n, int neig, double* out
 // NT-thread block calls this; sc is shared scratch of 2 n + 2 max(nrow, ncol)
 // + 4 doubles, n the smaller dimension.
 //
-// Householder reflections from both sides make t real bidiagonal (8/3 n^3
+// Householder reflections from both sides make t real bidiagonal (4/3 n^3
 // complex multiply-adds) and bisection gives the values, as accurate as the
 // reference's zgesvd (absolutely, to the norm of t, where modes mix).  One-sided Jacobi took
 // nine sweeps of 4 n^3 on the same FP64 pipe: 57 M clocks for 64 x 64.

@@ -98,10 +98,12 @@ __device__ bool jacobi_with_vectors(double2* A, int lda, int L, int nv, double2*
 // Singular values and right singular vectors of the m x n matrix A (m >= n,
 // column-major, leading dimension m, overwritten) by one CTA: Householder
 // bidiagonalisation U^H A Q = B, V = Q, then the implicit-shift QR iteration of
-// Golub and Kahan on B, whose right rotations V takes.  d[n], e[n]: the singular
-// values end up in d, up to sign, in no order.  V: n x n column-major.  sc: 7 n +
-// 4 doubles and 2 m double2 of shared memory.  Warp 0 runs the rotations of a
-// sweep, a serial chain, while the other warps apply those of the sweep before.
+// Golub and Kahan on B, whose right rotations V takes (its sweeps start from
+// (|d| - sigma)(sign d + sigma/d), the form that LAPACK documents for xBDSQR).
+// d[n], e[n]: the singular values end up in d, up to sign, in no order.  V: n x n
+// column-major.  sc: 7 n + 4 doubles and 2 m double2 of shared memory.  Warp 0
+// runs the rotations of a sweep, a serial chain, while the other warps apply
+// those of the sweep before.
 // As accurate as the reference's zgesvd: absolutely, to the norm of A.
 // Returns false when the iteration does not end or A is not finite (then d is NaN).
 __device__ bool svd_with_vectors(double2* A, const int m, const int n, double2* V, double* sc) {
@@ -801,9 +803,12 @@ int64_t eigvec_work_stride(int nr, int nc) {
   return (((int64_t)(nr > nc ? nr : nc) * nc + (int64_t)nc * nc) + 15) & ~(int64_t)15;
 }
 
-// Vectors for a selection of open channels come from the QR iteration; an
-// eigenvector call by itself keeps one-sided Jacobi, whose small eigenvalues are
-// accurate relatively, not only to the norm of the matrix.  152 matrices of 64 x
+// Vectors for a selection by windows of T come from the QR iteration, whose
+// values are accurate to the norm of t.  So is t itself: profiles of localised
+// guides in windows down to T = 1e-18 are as far from an extended-precision
+// reference as with one-sided Jacobi (1e-12 .. 1e-9 there, 1e-14 above 1e-5).  An
+// eigenvector call by itself, whose matrix may be better than that, keeps Jacobi
+// and its relative accuracy.  152 matrices of 64 x
 // 64: 41 ms by Jacobi, 6.4 by QR (profiles of 152 guides of 64 modes and 300
 // slices 125 -> 90 ms).
 int launch_eigvec(const EigvecArgs& a, cudaStream_t s) {

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kOzThreads, 2) zb_gemm_kernel(int M, char* ws,
   const int ti0 = (rest / nbc) * oz::kBlkRows, tj0 = (rest % nbc) * oz::kBlkCols;
   const ItemWs w = item_ws(ws, M, item);
   double2* c = C + (int64_t)item * strideC;
-  oz::gemm_block(M, ti0, tj0, false, w.adig, w.bdig, w.ea, w.eb, stg, [&](int i, int j, double re, double im) {
+  oz::gemm_block(M, ti0, tj0, w.adig, w.bdig, w.ea, w.eb, stg, [&](int i, int j, double re, double im) {
     double2 v = make_double2(alpha.x * re - alpha.y * im, alpha.x * im + alpha.y * re);
     if (beta != 0.0) {
       const double2 d = zat(D, item, M, i, j);

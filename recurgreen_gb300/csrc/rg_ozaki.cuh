@@ -226,9 +226,7 @@ __device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wai
 // stages deep (stg: kBlkStageUint4 uint4 = 72 KB), so the copy of k tile
 // t + 1 runs while the tensor cores work on k tile t and the loop reads no
 // global memory; every staged A digit serves 4 tiles and every B digit 2.
-// The level sums of a k tile are folded after it.  With
-// `upper`, warps whose tile lies wholly below the diagonal (ti > tj) skip the
-// products (their outputs are not wanted).  out(i, j, re, im) stores C_ij
+// The level sums of a k tile are folded after it.  out(i, j, re, im) stores C_ij
 // (called for i, j < M only).
 // ---------------------------------------------------------------------------
 constexpr int kBlkRows = 2, kBlkCols = 4;
@@ -237,13 +235,13 @@ constexpr int kBlkOneUint4 = (kBlkRows + kBlkCols) * 2 * kSlices * 32;  // one s
 constexpr int kBlkStageUint4 = 2 * kBlkOneUint4;                       // two stages
 
 template <class Out>
-__device__ void gemm_block(int M, int ti0, int tj0, bool upper, const uint4* adig, const uint4* bdig, const int* ea,
-                           const int* eb, uint4* stg, Out out) {
+__device__ void gemm_block(int M, int ti0, int tj0, const uint4* adig, const uint4* bdig, const int* ea, const int* eb,
+                           uint4* stg, Out out) {
   const int T = tiles(M);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wr = warp / kBlkCols, wc = warp % kBlkCols;
   const int ti = ti0 + wr, tj = tj0 + wc;
-  const bool active = ti < T && tj < T && !(upper && ti > tj);
+  const bool active = ti < T && tj < T;
   const int64_t plane = (int64_t)T * T * 32;
   long long hi[16], lo[16];
 #pragma unroll

@@ -61,7 +61,7 @@ constexpr int kSymMaxRowSplit = 8;
 // (gj_small); two blocks of at most 32 on the tensor cores 58,000 each
 // (leaf_inverse), and the four products that join them 35,000 each
 // (tiny_zgemm).  Leaves of up to 32 against leaves of up to 64: t and r at 100
-// modes (25 or 50) 94 and 108 ms; 304 realizations of 256 modes 218 and 233;
+// modes (25 or 50) 94 and 108 ms; 152 realizations of 256 modes 218 and 233;
 // one of 256 111 and 145; gradients at 128 84 and 96.
 constexpr int kLeafModes = 32;
 constexpr int kMaxLevels = 4;  // 512 -> 32
@@ -73,7 +73,7 @@ constexpr int kSmallGJ = 64;
 // The pivot column (panel phase) and the chunk's z values (update phase)
 // share one region: they are never live at the same time.
 //
-// With tensor_r the products' stages (64 KB) and, between products, the
+// With tensor_r the products' stages (96 KB) and, between products, the
 // shared-memory Gauss-Jordan blocks overlay the start of this
 // area (dead during either), and two arrays of 16-padded exponents follow.
 constexpr size_t kSmallGJBytes = sizeof(double2) * (kSmallGJ * (kSmallGJ + 1) + 2 * kSmallGJ) +
@@ -1275,7 +1275,7 @@ __global__ void __launch_bounds__(kSymNT, 2) sweep_large_sym_kernel(SweepArgs a)
 
 // Same cluster-size policy as the pivoted blocked kernel (sweep_large_plan).
 int sweep_large_sym_plan(SweepArgs& a, int sm_count, int* grid, int64_t* work_stride) {
-  if (a.max_M > 512) a.tensor_r = 0;  // the product's int64 fold is sized for M <= 512
+  if (a.max_M > 512) a.tensor_r = 0;  // the products' integers are sized for M <= 512
   const bool tensor = a.tensor_r != 0;
   const size_t smem = LargeSymSmem::bytes(a.max_M, tensor);
   if (smem > 227 * 1024) return fail(RG_ERR_INVALID_ARG, "too many modes for the symmetric large-mode kernel");

@@ -9,16 +9,16 @@
 // with c = 1 for open modes, so that a slice needs no product with B, and every
 // matrix entry is of order 1.  A closed mode's |A/B| is 2 cosh(kappa dx): on
 // coarse slices, where that passes 32, c is the power of two that takes it back
-// (the 26 bits of the FP32 inverse do not span cosh(6): whole items went to the
-// pivoted kernel: 304 guides of 63 modes, 14 of them closed, 200 slices,
-// kappa dx up to 6.4, 355 ms, 67 now).
+// (the 26 bits of the FP32 inverse do not span cosh(6), and whole items went to
+// the pivoted kernel: 304 guides of 63 modes, 14 of them closed, 200 slices,
+// kappa dx up to 6.4, 355 ms; 67 now).
 //
 // In the modes exp(2 pi i k y) of a periodic guide X is Hermitian but for its
 // diagonal, not symmetric; A and B depend on |k| alone, so in the real modes
 // cos and sin of 2 pi |k| y, a unitary change within each pair k, -k, the same
 // recursion is symmetric with the same A and B.  Only V's elements, and t or r
 // at the end, differ.  200 guides of 51 modes and 100 slices, t and r: 161 ms
-// in the pivoted kernel, 68 here.
+// in the pivoted kernel, 58 to 62 here.
 // Periodic items whose states are kept go to the pivoted kernel.
 //
 // Why not FP64 elimination: FP64 is 1.7 FMA lanes per clock and SM here, so
@@ -30,11 +30,11 @@
 //   4. Q on the tensor cores, all 26 digit pairs, rounded once.
 // FP64 instructions are left in the potential's draw and projection, which
 // two producer warps run one slice ahead of the others, and in the assembly
-// of X'.  The residual makes the result as accurate as an FP64 inverse: the
-// error of t against an extended-precision sweep is that of the elimination
-// within 0.95 to 1.3 (7 to 64 modes, 40 to 300 slices; geometric mean 1.08).
+// of X'.  The residual makes the result as accurate as an FP64 inverse: against an
+// extended-precision sweep the error of t is 0.65 to 1.06 times the elimination's
+// (7 to 64 modes, 40 to 300 slices; geometric mean 0.9), that of T 0.4 to 0.95.
 // Measured, with the eigenvalues: 304 guides of 64 modes and 600 slices 607 ms
-// before, 187 now; 500 of 37 modes and 150 slices 110 ms before, 44 now; one
+// before, 185 now; 500 of 37 modes and 150 slices 110 ms before, 45 now; one
 // guide of 10 modes and 200 slices 8.2 ms before, 2.0 now.
 //
 // Layout: T = ceil(M/16) tiles a side, one warp per tile or two, as in
@@ -46,7 +46,8 @@
 // modes a warp per tile and two CTAs of 80 registers took the same time).
 //
 // If a pivot is too small against the unswept entries of its row (sym_tau),
-// or the residual is not small, the item is flagged (kStatusNeedPivot), its
+// the residual is not small, or something does not fit its row's fixed point
+// (strong disorder), the item is flagged (kStatusNeedPivot), its
 // index appended to a.flag_list, and it is recomputed by the pivoted kernel,
 // which launch_sweep starts on that list.
 #include "rg_tile_inverse.cuh"
@@ -193,10 +194,7 @@ __global__ void __launch_bounds__(SymCfg<T, PROP>::NT, SymCfg<T, PROP>::MINB) sw
   const float tau = (float)fmin(kNaturalTau * a.sym_tau, 3e38);
 
   const TileSmem ts{regA, regB, red, rsum, exX, exY};
-  auto mbar = [&]() {
-    if (NMAIN == 32) __syncwarp();
-    else bar_sync(kBarMain, NMAIN);
-  };
+  auto mbar = [&]() { bar_sync(kBarMain, NMAIN); };
 
   for (;;) {
     if (tid == 0) {
