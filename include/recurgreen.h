@@ -99,7 +99,9 @@ int rg_get_modes(const rg_waveguide* wg, double* mumesh, double* bmat);
  * `iseed`, runs the recursive Green sweep on the GPU, and writes the neigv
  * transmission eigenvalues (descending) into chunk iseed of the host array
  * tallvals[len].  Same checks as the reference: len must be a positive
- * multiple of neigv and 1 <= iseed <= len / neigv. */
+ * multiple of neigv and 1 <= iseed <= len / neigv.  As from the reference's
+ * zgesvd, a singular value of t is accurate to the norm of t, so T has that
+ * many digits less the smaller it is (all of them where modes do not mix). */
 int rg_compute_tdistrib(rg_waveguide* wg, int iseed, double* tallvals, int64_t len);
 
 /* compute_refl_trans_v1 (src/waveguide.f90:469-519): full nmu x nmu
@@ -146,8 +148,9 @@ int rg_refl_trans_v1_batch(rg_waveguide* wg, const int32_t* seeds, int n, double
  * tprofiledata(nx, nprofile, nseed) layout), nt[k*nprofile + w] eigenvalues
  * in the window and tavg[k] = sum(T)/ncol (the group's Tavg).  Host
  * pointers; nt, tavg and status may be NULL.  The window bounds are checked
- * as the reference checks them.  Returns the first non-OK status after all
- * realizations have run. */
+ * as the reference checks them.  T and eigenvectors are accurate to the norm
+ * of t, as zgesvd's.  Returns the first non-OK status after all realizations
+ * have run. */
 int rg_tprofile_batch(rg_waveguide* wg, const int32_t* seeds, int n, int kind, int nprofile, const double* a,
                       const double* b, double* profiles, int32_t* nt, double* tavg, int32_t* status);
 
@@ -186,7 +189,8 @@ int rg_compute_wavefunction(rg_waveguide* wg, int iseed, int ipos, int imode, do
  * T[n] (descending) and eigenvectors U (n x n, column-major, same order) of
  * A^H A for the m x n complex matrix a (column-major).  One-sided Jacobi with
  * accumulated rotations instead of zgesvd; eigenvectors are defined up to a
- * phase (and within degenerate eigenspaces). */
+ * phase (and within degenerate eigenspaces).  RG_ERR_NOCONV when a is not
+ * finite. */
 int rg_diagonalize_ahca(const double* a, int m, int n, double* T, double* U);
 
 /* As rg_compute_tdistrib / rg_compute_refl_trans_v1, but for a caller-given

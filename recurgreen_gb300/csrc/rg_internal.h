@@ -195,8 +195,8 @@ inline bool row_split_matters(const SweepArgs& a, bool periodic) {
 // the kernel that runs, and the form of its inverse.
 inline int tuned_kernel(const SweepArgs& a, bool periodic) {
   const bool symmetric = a.symmetric && (!periodic || a.max_M <= kMaxModesSmem);
-  return (symmetric ? 1 : 0) | (symmetric && a.max_M > kMaxModesSmem ? (a.tensor_r ? 2 : 0) | a.split_inverse << 2 : 0) |
-         (periodic ? 16 : 0);
+  const int inverse = symmetric && a.max_M > kMaxModesSmem ? (a.tensor_r ? 2 : 0) | a.split_inverse << 2 : 0;
+  return (symmetric ? 1 : 0) | inverse | (periodic ? 16 : 0);
 }
 
 // Status the symmetric kernel leaves on an item whose diagonal pivots were

@@ -209,7 +209,8 @@ struct TileSmem {
 // of 20 to 64 modes under strong disorder.
 template <int T, int NE, int NP = 1, class Bar, class Pre>
 __device__ __forceinline__ bool tile_inverse(const double* x, const int M, const float tau, const TileSmem& s,
-                                             volatile int* flag, volatile int* late, Bar bar, Pre pre, double* gd, int& ey0, int& ey1) {
+                                             volatile int* flag, volatile int* late, Bar bar, Pre pre, double* gd,
+                                             int& ey0, int& ey1) {
   static_assert(NP == 1 || T == 1, "a part each only for one tile");
   constexpr int MP = 16 * T, NV = 2 * NE / NP, NHALF = 8 / NE, NCW = T * NHALF * NP, PL = T * T * 32, LDW = MP + 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) / NP, part = NP == 2 ? (tid >> 5) & 1 : 0;
